@@ -128,7 +128,7 @@ def _options(case):
     if not case["mixed"]:
         return dict(precision=EQC_FP64, guess=EQC_GUESS_PREVIOUS, cg_tol=1e-10)
     opt = dict(precision=EQC_MIXED, guess=EQC_GUESS_EXTRAPOLATE, cg_tol=1e-10)
-    return dict(opt, mg_degree=4, mg_degree_coarse=1, apply_variant=8, reliable_delta=1e-4) if case["tuned"] else opt
+    return dict(opt, mg_degree=4, mg_degree_coarse=1, apply_variant=0, reliable_delta=1e-4) if case["tuned"] else opt
 
 
 def _vector(seed, ny, nx):
