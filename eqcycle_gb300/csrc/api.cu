@@ -93,6 +93,7 @@ static void load_element_data(Handle& h, const double* W) {
     h.W64p.upload(b.data(), b.size(), s);
     h.diag64.upload(dg.data(), dg.size(), s);
     h.diag32.upload(dg32.data(), dg32.size(), s);
+    classify_elements(h);
     EQC_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -171,7 +172,7 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
     h.Total_time = m.Total_time;
     h.yr2sec = (double)m.yr2sec;
     std::memcpy(h.H, m.H, sizeof(h.H));
-    set_H(h.H, s);
+    h.uni_ok = set_H(h.H, s);
     set_H_df(h.H, s);
     {   // the double-float apply uses the even-odd form: H must be centro-antisymmetric
         double hmax = 0.0, asym = 0.0;

@@ -102,8 +102,8 @@ struct Layout {
 // one for the padded element data, per precision.
 struct TmaCache {
     bool ok = false, walk_ok = false;
-    std::unordered_map<const void*, CUtensorMap> u32, u64, u32walk;
-    CUtensorMap w32, w64, w32walk;
+    std::unordered_map<const void*, CUtensorMap> u32, u64, u32walk, u64uni;
+    CUtensorMap w32, w64, w32walk, mu;
 };
 
 // W padded to a 16-byte multiple per element, so element tiles are TMA-addressable.

@@ -13,8 +13,10 @@
 //                  plus a halo warp (variants 0, 4-7; the FP32 default);
 //   k_apply_walk   the same arithmetic fed by TMA, one wave of CTAs each walking up a strip
 //                  (variant 8; the autotuner's usual choice);
-//   k_apply_pipe   persistent tiles with a TMA pipeline, node-line form (the FP64 default,
-//                  FP32 variant 3); k_apply_tma / k_apply_lines: one tile per CTA (1, 2);
+//   k_apply_uni64  FP64: persistent tiles with a TMA pipeline, node-line form, one contraction per
+//                  line where the elements have one rigidity (the FP64 default, variant 3);
+//   k_apply_pipe   FP32 variant 3: the same tiles and pipeline with both contractions of a line;
+//                  k_apply_tma / k_apply_lines: one tile per CTA (1, 2);
 //   k_apply        the strip modes 2 and 3 (first element row only).
 // The FP32 element kernels take an epilogue (epi.cuh) that finishes the V-cycle's residual or
 // Chebyshev step at each owned node.
@@ -193,6 +195,35 @@ struct EOCoef64 {   // the same coefficients for the FP64 kernels
 __constant__ EOCoef cEO[2];
 __constant__ EOCoef64 cEO64[2];
 __constant__ int cEO_ok;   // H is centro-antisymmetric (else the full contractions are used)
+
+// An element of one rigidity mu has W(p, j) = mu w_p w_j (w the GLL weights), so the two contractions
+// of a line and the multiplication between them are one 5 x 5 matrix: the line's share of K x is
+// c mu w_j S v with S = D^T diag(w) D.  S is symmetric and centrosymmetric and its rows sum to zero:
+// with o_m = v_m - v_(4-m) and e_m = v_m + v_(4-m) - 2 v_2,
+//   s_p, s_(4-p) = Q +- P,  Q = sum_m b_pm e_m,  P = sum_m a_pm o_m  (p = 0, 1),  s_2 = sum_m d_m e_m,
+// 20 operations where the two even-odd contractions and W take 45.  Every entry is taken as a
+// difference first (e_m = o_m + 2 (v_(4-m) - v_2)): on a smooth field the differences are exact or
+// nearly so, and the rounding left is of the size of the field's variation over the element (2e-16
+// of the result where the two contractions leave 3e-15).  Constants give exactly zero; through a
+// rounded D, whose rows sum to 2e-15 instead, they give 1e-15 of the entries of K.
+struct UniCoef {
+    double a[2][2], b[2][2], d[2];
+    double w[5];
+};
+__constant__ UniCoef cUni;
+
+__device__ __forceinline__ void uni_line(const double (&v)[5], double (&s)[5]) {
+    const double o0 = v[0] - v[4], o1 = v[1] - v[3];
+    const double e0 = fma(2.0, v[4] - v[2], o0), e1 = fma(2.0, v[3] - v[2], o1);
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const double P = fma(cUni.a[p][1], o1, cUni.a[p][0] * o0);
+        const double Q = fma(cUni.b[p][1], e1, cUni.b[p][0] * e0);
+        s[p] = Q + P;
+        s[4 - p] = Q - P;
+    }
+    s[2] = fma(cUni.d[1], e1, cUni.d[0] * e0);
+}
 
 __device__ __forceinline__ void eo5(const float (&v)[5], float (&s)[5], const EOCoef& c) {
     const float e0 = v[0] + v[4], e1 = v[1] + v[3], o0 = v[0] - v[4], o1 = v[1] - v[3];
@@ -542,6 +573,210 @@ __global__ void __launch_bounds__(NT) k_apply_pipe(const __grid_constant__ CUten
         if (threadIdx.x == 0) {
             const int tn = t + PSTAGES * gridDim.x;
             if (tn < ntiles) issue(tn, st);
+        }
+    }
+}
+
+// ---- FP64: persistent, pipelined, one contraction per line ---------------------------------
+// Rigidity of every element with one rigidity (k_classify), -1 for the others, on a grid shifted by
+// one column (column ex + 1; zero columns and rows outside the mesh).  An element outside the mesh
+// has rigidity 0.
+static int mu_pitch(int NelX) { return (NelX + 3) & ~1; }
+
+// Tolerance 2^-49: W is a rounded product of weights and rigidity (and of damage factors), a few
+// units in the last place from the product formed here.
+__global__ void k_classify(const double* __restrict__ W, double* __restrict__ mu, int NelX, int NelY, int pitch, int ok) {
+    EQC_GRID_WAIT();
+    const int64_t Nel = (int64_t)NelX * NelY;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < Nel; e += (int64_t)gridDim.x * blockDim.x) {
+        const double* w = W + 25 * e;
+        const double m = w[12] / (cUni.w[2] * cUni.w[2]);
+        bool uni = ok && m > 0 && isfinite(m);
+        for (int j = 0; j < 5; ++j)
+            for (int i = 0; i < 5; ++i)
+                uni = uni && fabs(w[i + 5 * j] - m * (cUni.w[i] * cUni.w[j])) <= 0x1p-49 * w[i + 5 * j];
+        mu[(e / NelX) * pitch + e % NelX + 1] = uni ? m : -1.0;
+    }
+}
+
+// Two contractions with W between them: a line that meets an element of several rigidities.
+__device__ __forceinline__ void generic_line(const double (&u)[5], const double (&w)[5], double (&o)[5]) {
+    double s[5];
+    if (cEO_ok) {
+        eo5(u, s, cEO64[0]);
+#pragma unroll
+        for (int p = 0; p < 5; ++p) s[p] *= w[p];
+        eo5(s, o, cEO64[1]);
+        return;
+    }
+#pragma unroll
+    for (int p = 0; p < 5; ++p) {
+        double acc = 0.0;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) acc += Hc<double>(k, p) * u[k];
+        s[p] = w[p] * acc;
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        double acc = 0.0;
+#pragma unroll
+        for (int p = 0; p < 5; ++p) acc += Hc<double>(i, p) * s[p];
+        o[i] = acc;
+    }
+}
+
+// Tile of 7 x 8 elements by 256 threads: 32 owned node rows times 8 element columns (the left halo
+// column first) are one x-line a thread, four whole rows to a warp, so that a line's 5th output
+// reaches its owner, the next lane, by a shuffle; 9 element rows (the halo row below first) times 28
+// owned node columns are one y-line a thread.
+constexpr int UEX = 7, UEY = 8, UNT = 256;
+struct UniTile {
+    static constexpr int UX = 4 * UEX + 8, UY = 4 * UEY + 5;   // node box (33 of 36 columns used)
+    static constexpr int OX = 4 * UEX, OY = 4 * UEY, EX = UEX + 1, EY = UEY + 1;
+    static constexpr int MX = 10;                             // rigidity box, from an even column
+    static constexpr int U_BYTES = UY * UX * 8, M_BYTES = EY * MX * 8;
+    static constexpr int M_OFF = (U_BYTES + 127) / 128 * 128;
+    static constexpr int STAGE = M_OFF + (M_BYTES + 127) / 128 * 128;
+    static constexpr int YS_OFF = PSTAGES * STAGE, CY_OFF = YS_OFF + OY * OX * 8, BAR_OFF = CY_OFF + EY * OX * 8;
+    static constexpr int BYTES = BAR_OFF + 8 * PSTAGES;
+};
+static_assert(UniTile::OY * UniTile::EX == UNT && UniTile::EY * UniTile::OX <= UNT, "one line of each kind per thread");
+
+// y = sign K x in FP64 (zero_row0: K_II), tiles and stages as k_apply_pipe's, in node lines: a line
+// whose one or two elements have one rigidity each takes uni_line, scaled by sign c w_j times their
+// summed rigidity (w_0 = w_4); any other line reads its W and takes both contractions.
+// Bound: GB300 issues two FP64 operations per SM and clock (every FP64 instruction of a warp holds
+// the pipe for 16 clocks, whatever its active lanes), so the lines, their scaling and the sums at
+// shared nodes are arranged in whole warps, the rigidities' signs are tested as integers, and a tile
+// takes about 430 warp instructions of the pipe: 7.7 per element, where both contractions took 15.
+// Back to back on the damage-zone models, before (both contractions, 8 x 7 tiles) and now: 61 x 95
+// elements 19.4 and 10.4 us, 120 x 240 37.1 and 21.9, 240 x 480 134.2 and 68.6 (122.8 and 60.8 where
+// one x and y stay in L2), 480 x 960 496 and 248: 48 us of the 60.8 are the pipe's.
+__global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUtensorMap umap,
+                                                     const __grid_constant__ CUtensorMap mmap, double* __restrict__ y,
+                                                     ApplyArgs<double> A, double sign, int zero_row0, int ntx, int ntiles) {
+    EQC_GRID_WAIT();
+    if (A.gate && *A.gate != A.gate_val) return;
+    using UT = UniTile;
+    const Layout& L = A.L;
+    extern __shared__ __align__(128) unsigned char smem[];
+    double* ys = reinterpret_cast<double*>(smem + UT::YS_OFF);
+    double* cy = reinterpret_cast<double*>(smem + UT::CY_OFF);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + UT::BAR_OFF);
+    auto issue = [&](int t, int st) {
+        const int ex0 = (t % ntx) * UEX, ey0 = (t / ntx) * UEY;
+        mbar_expect_tx(&bar[st], (uint32_t)(UT::U_BYTES + UT::M_BYTES));
+        tma_load_2d(smem + st * UT::STAGE, &umap, &bar[st], 4 * ex0 - 4, 4 * ey0 - 4);
+        tma_load_2d(smem + st * UT::STAGE + UT::M_OFF, &mmap, &bar[st], ex0 & ~1, ey0 - 1);   // 16-byte aligned
+    };
+    if (threadIdx.x == 0) {
+        for (int st = 0; st < PSTAGES; ++st) mbar_init(&bar[st], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int st = 0; st < PSTAGES; ++st) {
+            const int t = blockIdx.x + st * gridDim.x;
+            if (t < ntiles) issue(t, st);
+        }
+    // this thread's x-line (node row r, element column c) and y-line (element row er, node column q)
+    const int r = threadIdx.x >> 3, c = threadIdx.x & 7, jx = r & 3;
+    const int er = threadIdx.x / UT::OX, q = threadIdx.x - er * UT::OX, kq = q & 3, ec = (q >> 2) + 1;
+    const bool has_y = er < UT::EY;
+    const double kx = sign * A.c1 * cUni.w[jx], ky = sign * A.c2 * cUni.w[kq];
+    // W(p, j) of element (ex, ey), zero outside the mesh
+    auto Wat = [&](int ex, int ey, int n) {
+        const bool in = ex >= 0 && ex < L.NelX && ey >= 0 && ey < L.NelY;
+        return in ? __ldg(A.W + ((int64_t)ey * L.NelX + ex) * 25 + n) : 0.0;
+    };
+    int i = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++i) {
+        const int st = i % PSTAGES;
+        const uint32_t parity = (uint32_t)((i / PSTAGES) & 1);
+        bool done = false;
+        const int polls = i == 0 ? A.wait_polls : MBAR_SPIN_LIMIT;
+        for (int it = 0; it < polls && !done; ++it) done = mbar_try_wait(&bar[st], parity);
+        const int ex0 = (t % ntx) * UEX, ey0 = (t / ntx) * UEY;
+        const double* us = reinterpret_cast<const double*>(smem + st * UT::STAGE);
+        const double* ms = reinterpret_cast<const double*>(smem + st * UT::STAGE + UT::M_OFF) + (ex0 & 1);
+        if (done) {
+            const double* ul = us + (r + 4) * UT::UX + 4 * c;
+            const double2 a = reinterpret_cast<const double2*>(ul)[0], b = reinterpret_cast<const double2*>(ul)[1];
+            const double u[5] = {a.x, a.y, b.x, b.y, ul[4]};
+            double s[5], kap;
+            const double* m = ms + ((r >> 2) + 1) * UT::MX + c;
+            const double m1 = m[0], m0 = jx == 0 ? m[-UT::MX] : 0.0;
+            if ((__double2hiint(m1) | __double2hiint(m0)) >= 0) {
+                uni_line(u, s);
+                kap = kx * (m1 + m0);
+            } else {
+                double w[5];
+                const int ex = ex0 - 1 + c, ey = ey0 + (r >> 2);
+#pragma unroll
+                for (int p = 0; p < 5; ++p) {
+                    w[p] = Wat(ex, ey, p + 5 * jx);
+                    if (jx == 0) w[p] += Wat(ex, ey - 1, p + 20);
+                }
+                generic_line(u, w, s);
+                kap = sign * A.c1;
+            }
+            const double carry = __shfl_up_sync(0xffffffffu, kap * s[4], 1);   // of column c - 1
+            if (c > 0) {
+                double2* o = reinterpret_cast<double2*>(ys + r * UT::OX + 4 * (c - 1));
+                o[0] = make_double2(fma(kap, s[0], carry), kap * s[1]);
+                o[1] = make_double2(kap * s[2], kap * s[3]);
+            }
+        }
+        if (__syncthreads_or(!done)) {
+            // give up: flag it, wait (bounded) for every copy still targeting this CTA, leave
+            if (threadIdx.x == 0) {
+                if (A.err) atomicExch(A.err, 1);
+                int j = i;
+                for (int tt = t; tt < ntiles && j < i + PSTAGES; tt += gridDim.x, ++j)
+                    for (int it = 0; it < MBAR_SPIN_LIMIT; ++it)
+                        if (mbar_try_wait(&bar[j % PSTAGES], (uint32_t)((j / PSTAGES) & 1))) break;
+            }
+            return;
+        }
+        double v[4];
+        if (has_y) {
+            const double* ul = us + (4 * er) * UT::UX + q + 4;
+            double u[5], s[5], kap;
+#pragma unroll
+            for (int l = 0; l < 5; ++l) u[l] = ul[l * UT::UX];
+            const double* m = ms + er * UT::MX + ec;
+            const double m1 = m[0], m0 = kq == 0 ? m[-1] : 0.0;
+            if ((__double2hiint(m1) | __double2hiint(m0)) >= 0) {
+                uni_line(u, s);
+                kap = ky * (m1 + m0);
+            } else {
+                double w[5];
+                const int ex = ex0 - 1 + ec, ey = ey0 - 1 + er;
+#pragma unroll
+                for (int p = 0; p < 5; ++p) {
+                    w[p] = Wat(ex, ey, kq + 5 * p);
+                    if (kq == 0) w[p] += Wat(ex - 1, ey, 4 + 5 * p);
+                }
+                generic_line(u, w, s);
+                kap = sign * A.c2;
+            }
+            cy[er * UT::OX + q] = kap * s[4];
+            if (er > 0) {
+#pragma unroll
+                for (int l = 0; l < 4; ++l) v[l] = fma(kap, s[l], ys[(4 * (er - 1) + l) * UT::OX + q]);
+            }
+        }
+        __syncthreads();   // cy written; every read of this stage and of ys done
+        if (threadIdx.x == 0) {
+            const int tn = t + PSTAGES * gridDim.x;
+            if (tn < ntiles) issue(tn, st);
+        }
+        const int ix = 4 * ex0 + q, iy0 = 4 * (ey0 + er - 1);
+        if (has_y && er > 0 && ix < L.nx) {
+            v[0] += cy[(er - 1) * UT::OX + q];
+#pragma unroll
+            for (int l = 0; l < 4; ++l)
+                if (iy0 + l < L.ny) y[(int64_t)(iy0 + l) * L.ld + ix] = (zero_row0 && iy0 + l == 0) ? 0.0 : v[l];
         }
     }
 }
@@ -1001,6 +1236,18 @@ static const CUtensorMap* tma_umap(TmaCache& c, const T* x, const Layout& L) {
     return &(m[x] = tm);
 }
 
+// Node-vector map of k_apply_uni64 (cached by address).
+static const CUtensorMap* tma_umap_uni(TmaCache& c, const double* x, const Layout& L) {
+    if (!c.ok) return nullptr;
+    auto it = c.u64uni.find(x);
+    if (it != c.u64uni.end()) return &it->second;
+    if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return nullptr;
+    CUtensorMap tm;
+    if (!encode_2d(&tm, true, x, (uint64_t)L.nx, (uint64_t)L.ny, (uint64_t)L.ld * sizeof(double), UniTile::UX, UniTile::UY))
+        return nullptr;
+    return &(c.u64uni[x] = tm);
+}
+
 // Node-vector map of the walk apply (cached by address): box WK_UX x WK_UY.
 static const CUtensorMap* tma_umap_walk(TmaCache& c, const float* x, const Layout& L) {
     if (!c.walk_ok) return nullptr;
@@ -1015,49 +1262,75 @@ static const CUtensorMap* tma_umap_walk(TmaCache& c, const float* x, const Layou
 
 // Encodes the element-data maps of the padded W copies W32p / W64p; leaves the cache disabled
 // (plain loads) if TMA is unavailable.
-void tma_init_for(TmaCache& c, const Layout& L, const float* W32p, const double* W64p) {
+void tma_init_for(TmaCache& c, const Layout& L, const float* W32p, const double* W64p, const double* mu) {
     c.ok = false;
     c.walk_ok = false;
     c.u32.clear();
     c.u64.clear();
     c.u32walk.clear();
+    c.u64uni.clear();
     if (getenv("EQC_NO_TMA")) return;
     const int EX = LTEX + 1, EY = LTEY + 1;
     bool ok = encode_2d(&c.w32, false, W32p, (uint64_t)L.NelX * WPad<float>::v, (uint64_t)L.NelY,
                         (uint64_t)L.NelX * WPad<float>::v * sizeof(float), EX * WPad<float>::v, EY);
     ok = ok && encode_2d(&c.w64, true, W64p, (uint64_t)L.NelX * WPad<double>::v, (uint64_t)L.NelY,
                          (uint64_t)L.NelX * WPad<double>::v * sizeof(double), EX * WPad<double>::v, EY);
+    const int mp = mu_pitch(L.NelX);
+    ok = ok && encode_2d(&c.mu, true, mu, (uint64_t)mp, (uint64_t)L.NelY, (uint64_t)mp * sizeof(double), UniTile::MX,
+                         UniTile::EY);
     c.ok = ok;
     c.walk_ok = ok && encode_w_walk(&c.w32walk, W32p, L.NelX, L.NelY);
 }
-void tma_init(Handle& h) { tma_init_for(h.tma, h.L, h.W32p.p, h.W64p.p); }
+void tma_init(Handle& h) { tma_init_for(h.tma, h.L, h.W32p.p, h.W64p.p, h.mu64.p); }
+
+void classify_elements(Handle& h) {
+    const Layout& L = h.L;
+    const int mp = mu_pitch(L.NelX);
+    if (!h.mu64.p) h.mu64.alloc((size_t)mp * L.NelY);
+    const int64_t Nel = (int64_t)L.NelX * L.NelY;
+    k_classify<<<(int)std::min<int64_t>((Nel + 255) / 256, 4096), 256, 0, h.stream>>>(h.W64.p, h.mu64.p, L.NelX, L.NelY, mp,
+                                                                                      h.uni_ok ? 1 : 0);
+    EQC_CHECK_LAUNCH();
+    count_launch();
+}
 
 // CTAs of the pipelined apply: as many as fit on every SM at once.
-static int g_pipe_blocks[2] = {0, 0};
-template <class T>
-static int pipe_blocks() { return g_pipe_blocks[sizeof(T) == 8 ? 1 : 0]; }
+static int g_pipe_blocks = 0;
 
-template <class T>
-static void pipe_setup() {
-    const int bytes = PipeLayout<T, LTEX, LTEY>::BYTES;
-    EQC_CUDA(cudaFuncSetAttribute(k_apply_pipe<T, LTEX, LTEY, LNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+template <class K>
+static int resident_blocks(K kernel, int threads, int bytes) {
+    EQC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     int per_sm = 0, dev = 0, nsm = 0;
-    EQC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_apply_pipe<T, LTEX, LTEY, LNT>, LNT, bytes));
+    EQC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes));
     EQC_CUDA(cudaGetDevice(&dev));
     EQC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    g_pipe_blocks[sizeof(T) == 8 ? 1 : 0] = std::max(1, per_sm) * nsm;
+    return std::max(1, per_sm) * nsm;
+}
+
+// Launch shape of k_apply_uni64: g_uni_sms SMs, at most g_uni_per_sm CTAs on each.
+static int g_uni_sms = 0, g_uni_per_sm = 0, g_uni_smem = 0;
+static void uni_setup() {
+    int dev = 0;
+    EQC_CUDA(cudaGetDevice(&dev));
+    EQC_CUDA(cudaDeviceGetAttribute(&g_uni_sms, cudaDevAttrMultiProcessorCount, dev));
+    EQC_CUDA(cudaDeviceGetAttribute(&g_uni_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    g_uni_per_sm = resident_blocks(k_apply_uni64, UNT, UniTile::BYTES) / g_uni_sms;
+    EQC_CUDA(cudaFuncSetAttribute(k_apply_uni64, cudaFuncAttributeMaxDynamicSharedMemorySize, g_uni_smem));
+}
+// The FP64 pipe of each SM bounds the kernel, so its CTAs have to be spread evenly: per SM no more than
+// an even spread of the tiles needs, kept to that by the shared memory that a CTA asks for.  (A
+// programmatic launch otherwise fills the SMs that its predecessor leaves empty with several CTAs
+// each: 26 us instead of 16 back to back on 61 x 95 elements.)
+static void launch_uni64(const CUtensorMap& um, double* y, const ApplyArgs<double>& A, double sign, int zr,
+                         cudaStream_t s) {
+    const int ntx = A.L.NelX / UEX + 1, ntiles = ntx * (A.L.NelY / UEY + 1);
+    const int per_sm = std::min(g_uni_per_sm, (ntiles + g_uni_sms - 1) / g_uni_sms);
+    const int smem = std::max(UniTile::BYTES, std::min(g_uni_smem, 228 * 1024 / (per_sm + 1) / 128 * 128 + 128));
+    k_apply_uni64<<<std::min(ntiles, per_sm * g_uni_sms), UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles);
 }
 
 // CTAs of the walk apply that are resident at once (its grid never exceeds one wave).
 static int g_walk_slots = 0;
-static void walk_setup() {
-    EQC_CUDA(cudaFuncSetAttribute(k_apply_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, WK_BYTES));
-    int per_sm = 0, dev = 0, nsm = 0;
-    EQC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_apply_walk, 32 * WK_ROWS, WK_BYTES));
-    EQC_CUDA(cudaGetDevice(&dev));
-    EQC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    g_walk_slots = std::max(1, per_sm) * nsm;
-}
 
 // Walk length: the rows of every strip split evenly over the resident CTAs (one wave, every
 // SM holding the same number of rows to within one walk).
@@ -1083,8 +1356,9 @@ static bool launch_walk(const float* x, float* y, const ApplyArgs<float>& A, flo
     return true;
 }
 
-void set_H(const double* H, cudaStream_t s) {
+bool set_H(const double* H, cudaStream_t s) {
     float hf[25];
+    bool uni = false;
     for (int k = 0; k < 25; ++k) hf[k] = (float)H[k];
     EQC_CUDA(cudaMemcpyToSymbolAsync(cH64, H, sizeof(double) * 25, 0, cudaMemcpyHostToDevice, s));
     EQC_CUDA(cudaMemcpyToSymbolAsync(cH32, hf, sizeof(float) * 25, 0, cudaMemcpyHostToDevice, s));
@@ -1120,6 +1394,31 @@ void set_H(const double* H, cudaStream_t s) {
             }
         }
         const int ok = asym <= 1e-12 * hmax ? 1 : 0;
+        // S = D^T diag(w) D of the one-contraction lines, w the GLL weights of 5 points; its rows
+        // sum to zero when constants have no derivative (sum_k H(k, p) = 0)
+        const double gw[5] = {0.1, 49.0 / 90.0, 32.0 / 45.0, 49.0 / 90.0, 0.1};
+        double rows = 0.0;
+        for (int p = 0; p < 5; ++p) {
+            double t = 0.0;
+            for (int k = 0; k < 5; ++k) t += D1(p, k);
+            rows = std::max(rows, std::fabs(t));
+        }
+        uni = ok && rows <= 8 * 2.2e-16 * hmax;   // rounding of H only
+        UniCoef u;
+        auto S = [&](int i, int k) {
+            long double t = 0.0L;
+            for (int p = 0; p < 5; ++p) t += (long double)D2(i, p) * gw[p] * D1(p, k);
+            return t;
+        };
+        for (int p = 0; p < 2; ++p) {
+            for (int m = 0; m < 2; ++m) {
+                u.a[p][m] = (double)(0.5L * (S(p, m) - S(p, 4 - m)));
+                u.b[p][m] = (double)(0.5L * (S(p, m) + S(p, 4 - m)));
+            }
+            u.d[p] = (double)S(2, p);
+        }
+        for (int p = 0; p < 5; ++p) u.w[p] = gw[p];
+        EQC_CUDA(cudaMemcpyToSymbolAsync(cUni, &u, sizeof(u), 0, cudaMemcpyHostToDevice, s));
         EQC_CUDA(cudaMemcpyToSymbolAsync(cEO, c, sizeof(c), 0, cudaMemcpyHostToDevice, s));
         EQC_CUDA(cudaMemcpyToSymbolAsync(cEO64, c64, sizeof(c64), 0, cudaMemcpyHostToDevice, s));
         EQC_CUDA(cudaMemcpyToSymbolAsync(cEO_ok, &ok, sizeof(int), 0, cudaMemcpyHostToDevice, s));
@@ -1130,10 +1429,10 @@ void set_H(const double* H, cudaStream_t s) {
                                   (int)apply_smem<double>()));
     EQC_CUDA(cudaFuncSetAttribute(k_apply<float, TEX, TEY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)apply_smem<float>()));
-    pipe_setup<float>();
-    pipe_setup<double>();
-    walk_setup();
-
+    g_pipe_blocks = resident_blocks(k_apply_pipe<float, LTEX, LTEY, LNT>, LNT, PipeLayout<float, LTEX, LTEY>::BYTES);
+    uni_setup();
+    g_walk_slots = resident_blocks(k_apply_walk, 32 * WK_ROWS, WK_BYTES);
+    return uni;
 }
 
 // Element-per-lane apply: variant 0 -> 6 element rows per CTA (default), 4..7 -> 4, 6, 8, 12.
@@ -1170,14 +1469,23 @@ void apply_K(const T* x, T* y, const ApplyArgs<T>& A, T sign, int mode, cudaStre
                 return;
             }
         }
+        if constexpr (sizeof(T) == 8) {
+            const CUtensorMap* uu = (A.tma && A.variant != 1 && A.variant != 2) ? tma_umap_uni(*A.tma, x, A.L) : nullptr;
+            if (uu) {
+                launch_uni64(*uu, y, A, sign, mode == 1 ? 1 : 0, s);
+                EQC_CHECK_LAUNCH();
+                count_launch();
+                return;
+            }
+        }
         const CUtensorMap* um = (A.tma && A.variant != 2) ? tma_umap<T>(*A.tma, x, A.L) : nullptr;
         if (um && A.variant == 1) {
             k_apply_tma<T, LTEX, LTEY, LNT><<<grid, LNT, 0, s>>>(*um, tma_wmap<T>(*A.tma), y, A, sign, mode == 1 ? 1 : 0);
-        } else if (um) {
+        } else if (um && sizeof(T) == 4) {
             const int ntx = (int)grid.x, ntiles = (int)(grid.x * grid.y);
-            const int nblk = std::min(ntiles, pipe_blocks<T>());
-            k_apply_pipe<T, LTEX, LTEY, LNT><<<nblk, LNT, PipeLayout<T, LTEX, LTEY>::BYTES, s>>>(
-                *um, tma_wmap<T>(*A.tma), y, A, sign, mode == 1 ? 1 : 0, ntx, ntiles);
+            if constexpr (sizeof(T) == 4)
+                k_apply_pipe<T, LTEX, LTEY, LNT><<<std::min(ntiles, g_pipe_blocks), LNT, PipeLayout<T, LTEX, LTEY>::BYTES,
+                                                   s>>>(*um, tma_wmap<T>(*A.tma), y, A, sign, mode == 1 ? 1 : 0, ntx, ntiles);
         } else {
             k_apply_lines<T, LTEX, LTEY, LNT><<<grid, LNT, 0, s>>>(x, y, A, sign, mode == 1 ? 1 : 0);
         }

@@ -147,6 +147,8 @@ struct Handle {
     DBuf<double> ref_stage;      // the field in the reference numbering on its way in or out
     // element data
     DBuf<double> W64, W64p;
+    DBuf<double> mu64;   // rigidity per element, -1 where it varies within one (classify_elements)
+    bool uni_ok = false; // H admits the one-contraction lines of the FP64 apply
     DBuf<float> W32, W32p;
     DBuf<float> W32lo;   // W - W32p rounded to FP32 (padded like W32p): W as double-float
     bool df_ok = false;  // the double-float FP64-class apply is usable (EQC_NO_DF unset, H symmetric)
@@ -205,7 +207,10 @@ struct Handle {
 void materialize_dyn_state(Handle& h);
 
 // kapply.cu
-void set_H(const double* H, cudaStream_t s);
+// Uploads the derivative matrix; true when it admits one-contraction lines (Handle::uni_ok).
+bool set_H(const double* H, cudaStream_t s);
+// mu64 from W64 (after every change of W64)
+void classify_elements(Handle& h);
 template <class T>
 void apply_K(const T* x, T* y, const ApplyArgs<T>& A, T sign, int mode, cudaStream_t s);
 
@@ -221,7 +226,7 @@ void set_H_df(const double* H, cudaStream_t s);
 // y = sign K x (FP64 vectors, mode 0/1) in double-float arithmetic; false when unavailable.
 bool apply_K_df(Handle& h, const double* x, double* y, double sign, int mode, cudaStream_t s,
                 const int* gate = nullptr, int gate_val = 0);
-void tma_init_for(TmaCache& c, const Layout& L, const float* W32p, const double* W64p);
+void tma_init_for(TmaCache& c, const Layout& L, const float* W32p, const double* W64p, const double* mu);
 // FP32 apply y = K x (mode 0/1 as apply_K) whose owned nodes are finished by the epilogue E
 // (residual or Chebyshev step) instead of stored; false when the selected kernel has none.
 bool apply_K_epi(const float* x, const ApplyArgs<float>& A, int mode, const OpEpi<float>& E, cudaStream_t s);

@@ -157,6 +157,7 @@ void setup_element_data_device(Handle& h, const eqc_material& mat) {
     k_setup_W<<<blocks, 256, 0, h.stream>>>(a, h.W64.p, h.W32.p, h.W64p.p, h.W32p.p, h.W32lo.p);
     EQC_CHECK_LAUNCH();
     count_launch();
+    classify_elements(h);
 }
 
 void setup_node_data_device(Handle& h, const eqc_material& mat, const std::vector<int64_t>& lBcL, const double* BcLC,

@@ -106,7 +106,7 @@ extern "C" eqc_status eqc_time_apply_stream(eqc_handle* H, int32_t dtype, int32_
             EQC_CUDA(cudaMemcpyAsync(r.W32p, h.W32p.p, sizeof(float) * WPad<float>::v * Nel, cudaMemcpyDeviceToDevice, s));
             EQC_CUDA(cudaMemcpyAsync(r.W64p, h.W64p.p, sizeof(double) * WPad<double>::v * Nel, cudaMemcpyDeviceToDevice,
                                      s));
-            tma_init_for(r.tma, h.L, r.W32p, r.W64p);
+            tma_init_for(r.tma, h.L, r.W32p, r.W64p, h.mu64.p);
         }
         EQC_CUDA(cudaStreamSynchronize(s));
         auto launch = [&](Replica& r) {
