@@ -2,6 +2,7 @@
 // permutation, host-array entry points.
 #include "model.h"
 #include "learn.h"
+#include "sem.h"
 #include "host_par.h"
 #include <cmath>
 #include <cstring>
@@ -174,6 +175,7 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
     std::memcpy(h.H, m.H, sizeof(h.H));
     h.uni_ok = set_H(h.H, s);
     set_H_df(h.H, s);
+    set_H_sem(h.H, s);
     {   // the double-float apply uses the even-odd form: H must be centro-antisymmetric
         double hmax = 0.0, asym = 0.0;
         for (int k = 0; k < 25; ++k) hmax = std::max(hmax, std::fabs(h.H[k]));
@@ -233,7 +235,7 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
     for (DBuf<double>* b : {&h.M, &h.d, &h.v, &h.a, &h.dPre, &h.tmp64a, &h.tmp64b, &h.tmp64c, &h.r64, &h.z64, &h.p64,
                              &h.q64, &h.Kd})
         b->alloc(N);
-    for (DBuf<float>* b : {&h.r32, &h.z32, &h.p32, &h.q32, &h.x32, &h.g32}) b->alloc(N);
+    for (DBuf<float>* b : {&h.r32, &h.z32, &h.p32, &h.q32, &h.x32, &h.g32, &h.p32b}) b->alloc(N);
     if (h.opt.precision == EQC_MIXED && std::getenv("EQC_NO_DF_UPDATE") == nullptr) {
         h.dx64.alloc(N);    // the intermediate reliable updates' correction and its K dx
         h.kdx64.alloc(N);
@@ -407,7 +409,7 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
     tma_init(h);
     EQC_CUDA(cudaMallocHost(&h.h_ctrl, sizeof(Ctrl)));
     std::memset(h.h_ctrl, 0, sizeof(Ctrl));
-    h.red_part.alloc(4096);
+    h.red_part.alloc(2 * 4096);
     h.red_count.alloc(64);
     h.scal.alloc(16);
     EQC_CUDA(cudaMallocHost(&h.h_scal, sizeof(double) * 16));

@@ -12,14 +12,11 @@ namespace eqc {
 
 int64_t g_launches = 0;
 
-int vec_blocks() { return VEC_BLOCKS; }
-
 // x and y 16-byte aligned; 4-wide chunks on a fixed grid, the n % 4 tail in thread 0
 template <class T>
-__global__ void __launch_bounds__(VEC_THREADS) k_dot(const T* __restrict__ x, const T* __restrict__ y, int64_t n,
+__global__ void __launch_bounds__(VEC_THREADS, VEC_PER_SM<T>) k_dot(const T* __restrict__ x, const T* __restrict__ y, int64_t n,
                                                      double* part, unsigned* count, double* out) {
     EQC_GRID_WAIT();
-    __shared__ double sh[32];
     DotAcc<T> acc;
     const int64_t n4 = n & ~(int64_t)3;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -31,9 +28,7 @@ __global__ void __launch_bounds__(VEC_THREADS) k_dot(const T* __restrict__ x, co
 #pragma unroll
         for (int k = 0; k < 4; ++k) acc.add(a[k], b[k]);
     }
-    double s = acc.value();
-    s = block_sum(s, sh);
-    finish_reduction(s, part, count, sh, [&](double t) { *out = t; });
+    grid_sum(acc, part, count, [&](double t) { *out = t; });
 }
 
 static void check_vec(const void* x, const void* y, int64_t) {
@@ -42,13 +37,7 @@ static void check_vec(const void* x, const void* y, int64_t) {
 
 void dot64(Handle& h, const double* x, const double* y, int64_t n, double* out_dev) {
     check_vec(x, y, n);
-    k_dot<double><<<vec_blocks(), VEC_THREADS, 0, h.stream>>>(x, y, n, h.red_part.p, h.red_count.p, out_dev);
-    EQC_CHECK_LAUNCH();
-    count_launch();
-}
-void dot32(Handle& h, const float* x, const float* y, int64_t n, double* out_dev) {
-    check_vec(x, y, n);
-    k_dot<float><<<vec_blocks(), VEC_THREADS, 0, h.stream>>>(x, y, n, h.red_part.p, h.red_count.p, out_dev);
+    k_dot<double><<<vec_blocks<double>(n), VEC_THREADS, 0, h.stream>>>(x, y, n, h.red_part.p, h.red_count.p, out_dev);
     EQC_CHECK_LAUNCH();
     count_launch();
 }

@@ -585,7 +585,9 @@ static int mu_pitch(int NelX) { return (NelX + 3) & ~1; }
 
 // Tolerance 2^-49: W is a rounded product of weights and rigidity (and of damage factors), a few
 // units in the last place from the product formed here.
-__global__ void k_classify(const double* __restrict__ W, double* __restrict__ mu, int NelX, int NelY, int pitch, int ok) {
+// mu32: the rigidity rounded to FP32; *several counts the elements of several.
+__global__ void k_classify(const double* __restrict__ W, double* __restrict__ mu, float* __restrict__ mu32, int* several,
+                           int NelX, int NelY, int pitch, int ok) {
     EQC_GRID_WAIT();
     const int64_t Nel = (int64_t)NelX * NelY;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < Nel; e += (int64_t)gridDim.x * blockDim.x) {
@@ -596,6 +598,8 @@ __global__ void k_classify(const double* __restrict__ W, double* __restrict__ mu
             for (int i = 0; i < 5; ++i)
                 uni = uni && fabs(w[i + 5 * j] - m * (cUni.w[i] * cUni.w[j])) <= 0x1p-49 * w[i + 5 * j];
         mu[(e / NelX) * pitch + e % NelX + 1] = uni ? m : -1.0;
+        mu32[e] = uni ? (float)m : -1.f;
+        if (!uni) atomicAdd(several, 1);
     }
 }
 
@@ -654,7 +658,8 @@ static_assert(UniTile::OY * UniTile::EX == UNT && UniTile::EY * UniTile::OX <= U
 // one x and y stay in L2), 480 x 960 496 and 248: 48 us of the 60.8 are the pipe's.
 __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUtensorMap umap,
                                                      const __grid_constant__ CUtensorMap mmap, double* __restrict__ y,
-                                                     ApplyArgs<double> A, double sign, int zero_row0, int ntx, int ntiles) {
+                                                     ApplyArgs<double> A, double sign, int zero_row0, int ntx, int ntiles,
+                                                     OpEpi<double> E) {
     EQC_GRID_WAIT();
     if (A.gate && *A.gate != A.gate_val) return;
     using UT = UniTile;
@@ -776,7 +781,8 @@ __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUt
             v[0] += cy[(er - 1) * UT::OX + q];
 #pragma unroll
             for (int l = 0; l < 4; ++l)
-                if (iy0 + l < L.ny) y[(int64_t)(iy0 + l) * L.ld + ix] = (zero_row0 && iy0 + l == 0) ? 0.0 : v[l];
+                if (iy0 + l < L.ny)
+                    epi_store1(E, y, (int64_t)(iy0 + l) * L.ld + ix, (zero_row0 && iy0 + l == 0) ? 0.0 : v[l]);
         }
     }
 }
@@ -984,7 +990,8 @@ __global__ void __launch_bounds__(32 * (ROWS + 1), MINB) k_apply_rows(const floa
         if (iy >= L.ny) break;
         const float z = (zero_row0 && iy == 0) ? 0.f : sign;
         epi_store4(E, y, (int64_t)iy * L.ld + 4 * ex,
-                   make_float4(z * out[j][0], z * out[j][1], z * out[j][2], z * out[j][3]));
+                   make_float4(z * out[j][0], z * out[j][1], z * out[j][2], z * out[j][3]),
+                   make_float4(u[j][0], u[j][1], u[j][2], u[j][3]));
     }
 }
 
@@ -1154,7 +1161,8 @@ __global__ void __launch_bounds__(32 * WK_ROWS, 2) k_apply_walk(const __grid_con
             if (iy >= L.ny) break;
             const float z = (zero_row0 && iy == 0) ? 0.f : sign;
             epi_store4(E, y, (int64_t)iy * L.ld + 4 * ex,
-                       make_float4(z * out[j][0], z * out[j][1], z * out[j][2], z * out[j][3]));
+                       make_float4(z * out[j][0], z * out[j][1], z * out[j][2], z * out[j][3]),
+                       make_float4(u[j][0], u[j][1], u[j][2], u[j][3]));
         }
     }
 }
@@ -1286,12 +1294,20 @@ void tma_init(Handle& h) { tma_init_for(h.tma, h.L, h.W32p.p, h.W64p.p, h.mu64.p
 void classify_elements(Handle& h) {
     const Layout& L = h.L;
     const int mp = mu_pitch(L.NelX);
-    if (!h.mu64.p) h.mu64.alloc((size_t)mp * L.NelY);
     const int64_t Nel = (int64_t)L.NelX * L.NelY;
-    k_classify<<<(int)std::min<int64_t>((Nel + 255) / 256, 4096), 256, 0, h.stream>>>(h.W64.p, h.mu64.p, L.NelX, L.NelY, mp,
-                                                                                      h.uni_ok ? 1 : 0);
+    if (!h.mu64.p) h.mu64.alloc((size_t)mp * L.NelY);
+    if (!h.mu32.p) h.mu32.alloc(Nel);
+    DBuf<int> several;
+    several.alloc(1);
+    k_classify<<<(int)std::min<int64_t>((Nel + 255) / 256, 4096), 256, 0, h.stream>>>(
+        h.W64.p, h.mu64.p, h.mu32.p, several.p, L.NelX, L.NelY, mp, h.uni_ok ? 1 : 0);
     EQC_CHECK_LAUNCH();
     count_launch();
+    int n = 0;
+    several.download(&n, 1, h.stream);
+    EQC_CUDA(cudaStreamSynchronize(h.stream));
+    h.sem_ok = h.uni_ok && (int64_t)n * 8 <= Nel && L.size() < (int64_t)1 << 29 &&   // 32-bit byte offsets
+               L.NelX < 31 * 4096;                                              // partials of a dot product's CTAs
 }
 
 // CTAs of the pipelined apply: as many as fit on every SM at once.
@@ -1322,11 +1338,13 @@ static void uni_setup() {
 // programmatic launch otherwise fills the SMs that its predecessor leaves empty with several CTAs
 // each: 26 us instead of 16 back to back on 61 x 95 elements.)
 static void launch_uni64(const CUtensorMap& um, double* y, const ApplyArgs<double>& A, double sign, int zr,
-                         cudaStream_t s) {
+                         cudaStream_t s, const OpEpi<double>& E = OpEpi<double>()) {
     const int ntx = A.L.NelX / UEX + 1, ntiles = ntx * (A.L.NelY / UEY + 1);
     const int per_sm = std::min(g_uni_per_sm, (ntiles + g_uni_sms - 1) / g_uni_sms);
     const int smem = std::max(UniTile::BYTES, std::min(g_uni_smem, 228 * 1024 / (per_sm + 1) / 128 * 128 + 128));
-    k_apply_uni64<<<std::min(ntiles, per_sm * g_uni_sms), UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles);
+    k_apply_uni64<<<std::min(ntiles, per_sm * g_uni_sms), UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles, E);
+    EQC_CHECK_LAUNCH();
+    count_launch();
 }
 
 // CTAs of the walk apply that are resident at once (its grid never exceeds one wave).
@@ -1473,8 +1491,6 @@ void apply_K(const T* x, T* y, const ApplyArgs<T>& A, T sign, int mode, cudaStre
             const CUtensorMap* uu = (A.tma && A.variant != 1 && A.variant != 2) ? tma_umap_uni(*A.tma, x, A.L) : nullptr;
             if (uu) {
                 launch_uni64(*uu, y, A, sign, mode == 1 ? 1 : 0, s);
-                EQC_CHECK_LAUNCH();
-                count_launch();
                 return;
             }
         }
@@ -1518,6 +1534,14 @@ bool apply_K_epi(const float* x, const ApplyArgs<float>& A, int mode, const OpEp
         return true;
     }
     return false;
+}
+
+bool apply_K_epi(const double* x, const ApplyArgs<double>& A, int mode, const OpEpi<double>& E, cudaStream_t s) {
+    if (mode > 1 || !A.tma || A.variant == 1 || A.variant == 2) return false;
+    const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
+    if (!uu) return false;
+    launch_uni64(*uu, nullptr, A, 1.0, mode, s, E);
+    return true;
 }
 
 template void apply_K<double>(const double*, double*, const ApplyArgs<double>&, double, int, cudaStream_t);

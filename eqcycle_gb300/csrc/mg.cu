@@ -3,6 +3,8 @@
 #include "reduce.cuh"
 #include "epi.cuh"
 #include "mg_pt.cuh"
+#include "sem.h"
+#include <algorithm>
 #include <cmath>
 #include <random>
 #include <utility>
@@ -10,160 +12,212 @@
 namespace eqc {
 
 // ------------------------------------------------------------------ device kernels
+// The vertex-level kernels run on 32 x 8 tiles of the grid, one thread per point (no index division).
+constexpr int VTX = 32, VTY = 8;
+
 template <class T>
-__global__ void k_stencil(const T* __restrict__ A, const T* __restrict__ x, T* __restrict__ y, int cx, int cy,
-                          OpEpi<T> E) {
+__global__ void __launch_bounds__(VTX * VTY) k_stencil(const T* __restrict__ A, const T* __restrict__ x,
+                                                       T* __restrict__ y, int cx, int cy, OpEpi<T> E) {
     EQC_GRID_WAIT();
-    const int64_t N = (int64_t)cx * cy;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
-        epi_store1(E, y, i, stencil_pt<T>(A, x, cx, cy, N, i, LdPlain()));
+    const int ix = blockIdx.x * VTX + threadIdx.x, iy = blockIdx.y * VTY + threadIdx.y;
+    if (ix >= cx || iy >= cy) return;
+    epi_store1(E, y, (int64_t)iy * cx + ix, stencil_pt<T>(A, cx, cy, ix, iy, LdPlain<T>{x, cx}));
 }
 
-// xf[fine] += sum_{a,b} wx_a wy_b xc[coarse]   (fine rows >= 1); xc + pend where the coarse
-// level's post-smoothing left its first step's direction pending (pend non-null)
-template <class T>
-__global__ void k_prolong_add(const T* __restrict__ xc, T* __restrict__ xf, int nfx, int nfy, int ldf, int ldc,
-                              const int* __restrict__ px, const int* __restrict__ py, const T* __restrict__ wx,
-                              const T* __restrict__ wy, const T* __restrict__ pend) {
+// bc = P^T r on coarse rows >= 1 (row 0 = 0), with the coarse level's first smoothing step, for a tile of
+// RCX x RCY coarse points.  One thread per fine point of the tile brings the residual r into shared
+// memory: stored by a separate launch (LdPlain), or formed here from the fine operator (LdResidual),
+// which saves that launch and r's store and load; the coarse points then sum their 3 x 3 fine points.
+constexpr int RCX = 15, RCY = 3, RFX = 2 * RCX + 1, RFY = 2 * RCY + 1;
+template <class T, class Ld>
+__global__ void __launch_bounds__(RFX * RFY) k_restrict(Ld rf, T* __restrict__ bc, Coarsen X, Coarsen Y, ChebFirst<T> F) {
     EQC_GRID_WAIT();
-    const int64_t N = (int64_t)nfx * nfy;
-    LdPend ld;
-    ld.base = xc;
-    ld.pend = pend;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        const int ix = (int)(i % nfx), iy = (int)(i / nfx);
-        if (iy == 0) continue;
-        T* o = xf + (int64_t)iy * ldf + ix;
-        *o = add_rn<T>(*o, prolong_pt<T>(xc, ldc, px, py, wx, wy, ix, iy, ld));
+    __shared__ T rs[RFY][RFX];
+    const int tx = threadIdx.x % RFX, ty = threadIdx.x / RFX;
+    const int cx0 = blockIdx.x * RCX, cy0 = blockIdx.y * RCY;
+    const int fx = min(max(2 * cx0 - 1 + tx, 0), X.nf - 1), fy = min(max(2 * cy0 - 1 + ty, 0), Y.nf - 1);
+    const int cxi = cx0 + threadIdx.x % RCX, cyi = cy0 + threadIdx.x / RCX;
+    const bool mine = threadIdx.x < RCX * RCY && cxi < X.nc && cyi < Y.nc;
+    const int64_t o = (int64_t)cyi * X.nc + cxi;
+    const T di = mine && F.dinv ? F.dinv[o] : T(0);
+    rs[ty][tx] = rf(fx, fy);
+    __syncthreads();
+    if (!mine) return;
+    T s = T(0);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        T w;
+        const int gy = Y.fine_of<T>(cyi, q, w);
+        T sx = T(0);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            T wx;
+            const int gx = X.fine_of<T>(cxi, k, wx);
+            sx = fma_rn<T>(wx, rs[min(max(gy - 2 * cy0 + 1, 0), RFY - 1)][min(max(gx - 2 * cx0 + 1, 0), RFX - 1)], sx);
+        }
+        s = fma_rn<T>(gy == 0 || cyi == 0 ? T(0) : w, sx, s);
     }
+    bc[o] = s;
+    if (F.dinv) F.x[o] = cheb_first_pt<T>(di, s, F.inv_theta);
 }
 
-// bc[coarse] = sum over restriction lists of rf[fine]  (coarse rows >= 1; row 0 = 0)
+// xf = x + P xc on every row (row 0: x)
 template <class T>
-__global__ void k_restrict(const T* __restrict__ rf, T* __restrict__ bc, int ncx, int ncy, int ldf, int ldc,
-                           const int* __restrict__ rpx, const int* __restrict__ rix, const T* __restrict__ rwx,
-                           const int* __restrict__ rpy, const int* __restrict__ riy, const T* __restrict__ rwy,
-                           ChebFirst<T> F) {
+__global__ void __launch_bounds__(VTX * VTY) k_prolong(T* __restrict__ xf, LdProlonged<T> P) {
     EQC_GRID_WAIT();
-    const int64_t N = (int64_t)ncx * ncy;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        const int cxi = (int)(i % ncx), cyi = (int)(i / ncx);
-        const T s = restrict_pt<T>(rf, ldf, rpx, rix, rwx, rpy, riy, rwy, cxi, cyi, LdPlain());
-        bc[(int64_t)cyi * ldc + cxi] = s;
-        cheb_first_pt(F, (int64_t)cyi * ldc + cxi, s);
+    const int ix = blockIdx.x * VTX + threadIdx.x, iy = blockIdx.y * VTY + threadIdx.y;
+    if (ix >= P.X.nf || iy >= P.Y.nf) return;
+    const int64_t i = (int64_t)iy * P.X.nf + ix;
+    xf[i] = iy == 0 ? P.x[i] : P(ix, iy);
+}
+
+// The prolongation and the first post-smoothing step in one launch: x' = x + P xc on a tile and the ring
+// around it in shared memory, one point per thread, then out = x' + (1 / theta) Dinv (b - A x') on the
+// tile; x' is stored too where a second step will need it (xf non-null).
+template <class T>
+__global__ void __launch_bounds__(VTX * VTY) k_prolong_smooth(const T* __restrict__ A, const T* __restrict__ b,
+                                                              const T* __restrict__ dinv, T* __restrict__ xf,
+                                                              T* __restrict__ out, LdProlonged<T> P, T inv_theta) {
+    EQC_GRID_WAIT();
+    __shared__ T xs[VTY][VTX];
+    const int cx = P.X.nf, cy = P.Y.nf;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int ix0 = blockIdx.x * (VTX - 2) - 1, iy0 = blockIdx.y * (VTY - 2) - 1;
+    const int ix = min(max(ix0 + tx, 0), cx - 1), iy = min(max(iy0 + ty, 0), cy - 1);
+    const int64_t i = (int64_t)iy * cx + ix;
+    const bool mine = tx > 0 && tx < VTX - 1 && ty > 0 && ty < VTY - 1 && ix0 + tx < cx && iy0 + ty < cy;
+    T a[9], bi = T(0), di = T(0);
+    if (mine) {
+        bi = b[i];
+        di = dinv[i];
+        stencil_row<T>(A, cx, cy, ix, iy, a);
     }
+    const T xi = iy == 0 ? P.x[i] : P(ix, iy);
+    xs[ty][tx] = xi;
+    __syncthreads();
+    if (!mine) return;
+    const T t = stencil_sum<T>(a, iy, [&](int k) { return xs[ty + k / 3 - 1][tx + k % 3 - 1]; });
+    if (xf) xf[i] = xi;
+    out[i] = cheb_x_pt<T>(xi, xi, bi, t, di, T(0), inv_theta);
 }
 
 // ---- transfers between the spectral-element grid and the element-vertex grid ----------
-// The GLL node at local index k of an element interpolates the element's two vertices with
-// weights lo[k] (lower vertex) and hi[k] (upper vertex), k = 0..3; the last node of the
-// lattice is the last vertex.  Structured: no index tables, no integer division.
+// xf = x + P0 xc; one thread per (vertex column, node row), four nodes each (the last column one).
 template <class T>
-struct GllW {
-    T lo[4], hi[4];
-};
-
-// xf[iy, 4ex + k] += P0 xc  for node rows iy >= 1; one thread per (element column, node row),
-// the thread of the last element column also takes the lattice's last node.
-template <class T>
-__global__ void k_prolong_sem(const T* __restrict__ xc, T* __restrict__ xf, Layout L, int ldc, GllW<T> w,
-                              const T* __restrict__ pend) {
+__global__ void k_prolong_sem(const T* __restrict__ x, const T* __restrict__ xc, T* __restrict__ xf, Layout L, int ldc,
+                              GllW<T> w) {
     EQC_GRID_WAIT();
-    const int ex = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y + 1;
-    if (ex >= L.NelX || iy >= L.ny) return;
-    LdPend ld;
-    ld.base = xc;
-    ld.pend = pend;
-    const int ey = min(iy >> 2, L.NelY - 1), ky = iy - 4 * ey;
-    const T wyl = ky == 4 ? T(0) : w.lo[ky], wyh = ky == 4 ? T(1) : w.hi[ky];
-    const T* c0 = xc + (int64_t)ey * ldc + ex;
-    const T* c1 = c0 + ldc;
-    const T a0 = wyl * ld(c0) + wyh * ld(c1);           // vertex column ex
-    const T a1 = wyl * ld(c0 + 1) + wyh * ld(c1 + 1);   // vertex column ex + 1
-    T* row = xf + (int64_t)iy * L.ld + 4 * ex;
+    const int ex = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y;
+    if (ex > L.NelX) return;
+    const int ey = iy >> 2, j = iy & 3;
+    auto c = [&](int vx, int vy) { return vx <= L.NelX && vy <= L.NelY ? xc[(int64_t)vy * ldc + vx] : T(0); };
+    const T a0 = gll_interp(w, j, c(ex, ey), c(ex, ey + 1));
+    const T a1 = gll_interp(w, j, c(ex + 1, ey), c(ex + 1, ey + 1));
+    const int64_t o = (int64_t)iy * L.ld + 4 * ex;
+    xf[o] = add_rn<T>(x[o], a0);
+    if (ex == L.NelX) return;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) row[k] += w.lo[k] * a0 + w.hi[k] * a1;
-    if (ex == L.NelX - 1) row[4] += a1;
+    for (int k = 1; k < 4; ++k) xf[o + k] = add_rn<T>(x[o + k], gll_interp(w, k, a0, a1));
 }
 
-// bc[vy, vx] = (P0^T rf)[vy, vx] over fine rows iy >= 1; coarse row 0 = 0.  One thread per vertex.
+// bc = P0^T rf over fine rows iy >= 1; coarse row 0 = 0.  One thread per vertex.
 template <class T>
 __global__ void k_restrict_sem(const T* __restrict__ rf, T* __restrict__ bc, Layout L, int ldc, GllW<T> w,
                                ChebFirst<T> F) {
     EQC_GRID_WAIT();
     const int vx = blockIdx.x * blockDim.x + threadIdx.x;
     const int vy = blockIdx.y;
-    const int ncx = L.NelX + 1;
-    if (vx >= ncx) return;
-    T acc = T(0);
-    if (vy >= 1) {
-        for (int dy = -3; dy <= 3; ++dy) {
-            const int iy = 4 * vy + dy;
-            if (iy < 1 || iy >= L.ny) continue;
-            const T wy = dy == 0 ? T(1) : (dy > 0 ? (vy < L.NelY ? w.lo[dy] : T(0)) : w.hi[4 + dy]);
-            const T* row = rf + (int64_t)iy * L.ld;
-            T sx = T(0);
+    if (vx > L.NelX) return;
+    // row sums of element (ex, ey): towards its lower (up = 0) or upper vertex
+    auto row = [&](int ex, int iy, bool up) {
+        T v[4];
 #pragma unroll
-            for (int dx = -3; dx <= 3; ++dx) {
-                const int ix = 4 * vx + dx;
-                if (ix < 0 || ix >= L.nx) continue;
-                const T wx = dx == 0 ? T(1) : (dx > 0 ? (vx < L.NelX ? w.lo[dx] : T(0)) : w.hi[4 + dx]);
-                sx += wx * row[ix];
-            }
-            acc += wy * sx;
+        for (int k = 0; k < 4; ++k) {
+            const int ix = 4 * ex + k;
+            v[k] = ix >= 0 && ix < L.nx && iy >= 1 && iy < L.ny ? rf[(int64_t)iy * L.ld + ix] : T(0);
         }
+        return up ? restrict_hi(w, v[1], v[2], v[3]) : restrict_lo(w, v[0], v[1], v[2], v[3]);
+    };
+    T s[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int ex = vx - (q & 1), ey = vy - (q >> 1);
+        T a[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[j] = row(ex, 4 * ey + j, q & 1);
+        s[q] = (q >> 1) ? restrict_hi(w, a[1], a[2], a[3]) : restrict_lo(w, a[0], a[1], a[2], a[3]);
     }
+    const T acc = vy >= 1 ? restrict_sum(s[0], s[1], s[2], s[3]) : T(0);
     bc[(int64_t)vy * ldc + vx] = acc;
-    cheb_first_pt(F, (int64_t)vy * ldc + vx, acc);
+    cheb_first_store(F, (int64_t)vy * ldc + vx, acc);
 }
 
-// Chebyshev, first step.  with_x: r = Dinv (b - t) with t = A x ; else r = Dinv b, x = 0.
-// d = r/theta ; x += d
+// Chebyshev, first step from x = 0: x = Dinv b / theta
 template <class T>
-__global__ void k_cheb_first(T* __restrict__ x, T* __restrict__ r, T* __restrict__ d, const T* __restrict__ b,
-                             const T* __restrict__ t, const T* __restrict__ Dinv, int64_t n, T inv_theta, int with_x) {
+__global__ void k_cheb_first(T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ Dinv, int64_t n,
+                             T inv_theta) {
     EQC_GRID_WAIT();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        cheb_first_step_pt<T>(x, r, d, b, t, Dinv, i, inv_theta, with_x != 0, LdPlain());
+        x[i] = cheb_first_pt<T>(Dinv[i], b[i], inv_theta);
 }
-// Chebyshev, later step: r -= Dinv t (t = A d) ; d = c1 d + c2 r ; x += d
+// Chebyshev step with t = A x from a separate launch (OpEpi mode 2)
 template <class T>
-__global__ void k_cheb_step(T* __restrict__ x, T* __restrict__ r, T* __restrict__ d, const T* __restrict__ t,
-                            const T* __restrict__ Dinv, int64_t n, T c1, T c2) {
-    EQC_GRID_WAIT();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        T ri = r[i], di = d[i], xi = x[i];
-        cheb_step_pt<T>(ri, di, xi, t[i], Dinv[i], c1, c2);
-        r[i] = ri;
-        d[i] = di;
-        x[i] = xi;
-    }
-}
-// x += d: a post-smoothing's pending first-step direction (OpEpi mode 3) with no later reader
-// to add it
-template <class T>
-__global__ void k_add_pend(T* __restrict__ x, const T* __restrict__ d, int64_t n) {
+__global__ void k_cheb_step(OpEpi<T> E, const T* __restrict__ t, int64_t n) {
     EQC_GRID_WAIT();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] = add_rn<T>(x[i], d[i]);
+        epi_store1<T>(E, nullptr, i, t[i]);
 }
-// r = b - t
+// r = b - t (t may be r)
 template <class T>
-__global__ void k_sub(const T* __restrict__ b, const T* __restrict__ t, T* __restrict__ r, int64_t n) {
+__global__ void k_sub(const T* __restrict__ b, const T* t, T* r, int64_t n) {
     EQC_GRID_WAIT();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         r[i] = b[i] - t[i];
 }
 // x[cx + k] = sum_j Cinv[k][j] b[cx + j]  (one warp per row).  Accumulates in T: FP32 for the
 // FP32 cycle (a preconditioner; GB300's FP64 rate would make this the slowest kernel of it).
+// The right-hand side is staged in shared memory (DNC entries at a time, zero beyond n); each warp reads
+// its row in 16-byte loads, eight in flight.
+constexpr int DNC = 2048, DN_WARPS = 8;
 template <class T>
-__global__ void k_dense_mv(const T* __restrict__ Cinv, const T* __restrict__ b, T* __restrict__ x, int n, int off) {
+__global__ void __launch_bounds__(32 * DN_WARPS) k_dense_mv(const T* __restrict__ Cinv, const T* __restrict__ b,
+                                                            T* __restrict__ x, int n, int pitch, int off) {
+    __shared__ __align__(16) T bs[DNC];
+    constexpr int V = 16 / (int)sizeof(T), U = 8;
+    struct alignas(16) Vec { T v[V]; };
+    const int lane = threadIdx.x & 31, row = blockIdx.x * DN_WARPS + (threadIdx.x >> 5);
+    const T* rw = Cinv + (int64_t)min(row, n - 1) * pitch;
     EQC_GRID_WAIT();
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const T s = dense_row<T>(Cinv, b, n, off, warp, lane, LdPlain());
-    if (lane == 0) x[off + warp] = s;
+    T s[V];
+#pragma unroll
+    for (int q = 0; q < V; ++q) s[q] = T(0);
+    for (int c0 = 0; c0 < n; c0 += DNC) {
+        const int m = min(DNC, pitch - c0);
+        if (c0) __syncthreads();
+        for (int k = threadIdx.x; k < m; k += 32 * DN_WARPS) bs[k] = c0 + k < n ? b[off + c0 + k] : T(0);
+        __syncthreads();
+        for (int j0 = 0; j0 < m; j0 += 32 * V * U) {
+            Vec c[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int j = j0 + (q * 32 + lane) * V;
+                c[q] = j < m ? *reinterpret_cast<const Vec*>(rw + c0 + j) : Vec{};
+            }
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int j = j0 + (q * 32 + lane) * V;
+                if (j >= m) break;
+                const Vec d = *reinterpret_cast<const Vec*>(bs + j);
+#pragma unroll
+                for (int e = 0; e < V; ++e) s[e] = fma_rn<T>(c[q].v[e], d.v[e], s[e]);
+            }
+        }
+    }
+    T v = add_rn<T>(s[0], s[1]);
+    if constexpr (V == 4) v = add_rn<T>(v, add_rn<T>(s[2], s[3]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = add_rn<T>(v, __shfl_down_sync(0xffffffffu, v, o));
+    if (lane == 0 && row < n) x[off + row] = v;
 }
 template <class T>
 __global__ void k_scale(T* x, int64_t n, double s) {
@@ -178,6 +232,7 @@ __global__ void k_mul(const T* a, T* x, int64_t n) {
         x[i] = a[i] * x[i];
 }
 
+static inline dim3 vgrid2(int cx, int cy) { return dim3((cx + VTX - 1) / VTX, (cy + VTY - 1) / VTY); }
 static inline int vb(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 8 * 152); }
 
 // ------------------------------------------------------------------ typed access
@@ -192,10 +247,6 @@ template <> struct Sel<double> {
     static const double* Di(StencilLevel& l) { return l.Dinv64.p; }
     static const double* Di0(MGHier& m) { return m.Dinv0_64.p; }
     static const double* C(MGHier& m) { return m.Cinv64.p; }
-    static const double* wx(DevTransfer& t) { return t.wx64.p; }
-    static const double* wy(DevTransfer& t) { return t.wy64.p; }
-    static const double* rwx(DevTransfer& t) { return t.rwx64.p; }
-    static const double* rwy(DevTransfer& t) { return t.rwy64.p; }
     static ApplyArgs<double> args(Handle& h) { return args64(h); }
 };
 template <> struct Sel<float> {
@@ -208,10 +259,6 @@ template <> struct Sel<float> {
     static const float* Di(StencilLevel& l) { return l.Dinv32.p; }
     static const float* Di0(MGHier& m) { return m.Dinv0_32.p; }
     static const float* C(MGHier& m) { return m.Cinv32.p; }
-    static const float* wx(DevTransfer& t) { return t.wx32.p; }
-    static const float* wy(DevTransfer& t) { return t.wy32.p; }
-    static const float* rwx(DevTransfer& t) { return t.rwx32.p; }
-    static const float* rwy(DevTransfer& t) { return t.rwy32.p; }
     static ApplyArgs<float> args(Handle& h) { return args32(h); }
 };
 
@@ -230,10 +277,19 @@ template <class T>
 static void level_apply(Handle& h, int l, const T* x, T* y) {
     MGHier& m = *h.mg;
     if (l == 0) {
+        if constexpr (sizeof(T) == 4) {
+            if (sem_usable(h)) {
+                SemOp o;
+                o.x = x;
+                o.out = y;
+                sem_launch(h, SL_PLAIN, SE_STORE, SP_NONE, o);
+                return;
+            }
+        }
         apply_K<T>(x, y, Sel<T>::args(h), T(1), 1, h.stream);
     } else {
         StencilLevel& L = m.lev[l - 1];
-        k_stencil<T><<<vb((int64_t)L.cx * L.cy), 256, 0, h.stream>>>(Sel<T>::A(L), x, y, L.cx, L.cy, OpEpi<T>());
+        k_stencil<T><<<vgrid2(L.cx, L.cy), dim3(VTX, VTY), 0, h.stream>>>(Sel<T>::A(L), x, y, L.cx, L.cy, OpEpi<T>());
         EQC_CHECK_LAUNCH();
         count_launch();
     }
@@ -245,15 +301,16 @@ static bool epi_apply(Handle& h, int l, const float* x, const OpEpi<float>& E) {
     if (!h.fuse) return false;
     if (l == 0) return apply_K_epi(x, args32(h), 1, E, h.stream);
     StencilLevel& L = h.mg->lev[l - 1];
-    k_stencil<float><<<vb((int64_t)L.cx * L.cy), 256, 0, h.stream>>>(L.A32.p, x, nullptr, L.cx, L.cy, E);
+    k_stencil<float><<<vgrid2(L.cx, L.cy), dim3(VTX, VTY), 0, h.stream>>>(L.A32.p, x, nullptr, L.cx, L.cy, E);
     EQC_CHECK_LAUNCH();
     count_launch();
     return true;
 }
 static bool epi_apply(Handle& h, int l, const double* x, const OpEpi<double>& E) {
-    if (l == 0 || !h.fuse) return false;   // the FP64 spectral-element apply has no epilogue
+    if (!h.fuse) return false;
+    if (l == 0) return apply_K_epi(x, args64(h), 1, E, h.stream);
     StencilLevel& L = h.mg->lev[l - 1];
-    k_stencil<double><<<vb((int64_t)L.cx * L.cy), 256, 0, h.stream>>>(L.A64.p, x, nullptr, L.cx, L.cy, E);
+    k_stencil<double><<<vgrid2(L.cx, L.cy), dim3(VTX, VTY), 0, h.stream>>>(L.A64.p, x, nullptr, L.cx, L.cy, E);
     EQC_CHECK_LAUNCH();
     count_launch();
     return true;
@@ -280,156 +337,203 @@ static void cheb_coeffs(const MGHier& m, int l, int deg, double* inv_theta, doub
     }
 }
 
-// Chebyshev smoothing of A_l x = b (deg steps), x = 0 initially when !with_x.  first_done: the
-// first step (from x = 0) already ran inside the restriction that produced b.  Steps run fused
-// into the operator (r, x updated in place, the direction alternating between the d and t work
-// vectors) when the level's operator kernel has the epilogue; the first step from x then leaves
-// x += d pending (OpEpi mode 3) for the second step, or, with one step, returns d for the
-// caller's next reader of x to add (null: x is complete).
+// The level's vectors by their use in one cycle of `deg` smoothing steps each way: the pre-smoothing's
+// iterates alternate between post0 and pre and end in pre; the prolongation puts pre + P xc into
+// post0, whose post-smoothed iterates alternate between post1 and post0 and end in x (the third
+// vector: a launch that forms pre + P xc itself still reads pre around its points).
 template <class T>
-static const T* chebyshev(Handle& h, int l, T* x, const T* b, bool with_x, bool first_done = false) {
+struct CycleVecs {
+    T *pre, *post0, *post1;
+    int deg;
+    T* pre_iter(int k) const { return ((deg - k) & 1) ? post1 : pre; }   // pre-smoothing iterate k = 1..deg
+};
+template <class T>
+static CycleVecs<T> cycle_vecs(const MGHier& m, MGWork& w, int l, T* x) {
+    const int deg = std::max(l == 0 ? m.deg : m.deg_coarse, 1);
+    const bool even = (deg & 1) == 0;
+    return {Sel<T>::t(w), even ? x : Sel<T>::d(w), even ? Sel<T>::d(w) : x, deg};
+}
+
+// One Chebyshev step of level l from x (OpEpi mode 2), in the operator's launch where it has the
+// epilogue.
+template <class T>
+static void cheb_step(Handle& h, int l, const T* x, const T* xp, bool xp_zero, T* out, const T* b, T c1, T c2) {
     MGHier& m = *h.mg;
-    MGWork& w = m.work[l];
+    OpEpi<T> E;
+    E.mode = 2;
+    E.b = b;
+    E.dinv = (l == 0) ? Sel<T>::Di0(m) : Sel<T>::Di(m.lev[l - 1]);
+    E.x = x;
+    E.xp = xp;
+    E.xp_zero = xp_zero;
+    E.out = out;
+    E.c1 = c1;
+    E.c2 = c2;
+    if (epi_apply(h, l, x, E)) return;
+    T* t = Sel<T>::r(m.work[l]);
     const int64_t n = level_size(h, l);
-    const T* Dinv = (l == 0) ? Sel<T>::Di0(m) : Sel<T>::Di(m.lev[l - 1]);
-    const int deg = (l == 0) ? m.deg : m.deg_coarse;
-    std::vector<double> cc1(std::max(deg, 1)), cc2(std::max(deg, 1));
-    double inv_theta = 0.0;
-    cheb_coeffs(m, l, deg, &inv_theta, cc1.data(), cc2.data());
-    T* r = Sel<T>::r(w);
-    T* d = Sel<T>::d(w);
-    T* t = Sel<T>::t(w);
-    bool pend = false;
-    if (!first_done) {
-        OpEpi<T> E;
-        E.mode = 3;
-        E.b = b;
-        E.r = r;
-        E.dinv = Dinv;
-        E.dnew = d;
-        E.inv_theta = (T)inv_theta;
-        if (with_x && epi_apply(h, l, x, E)) {
-            pend = true;
-        } else {
-            if (with_x) level_apply<T>(h, l, x, t);
-            k_cheb_first<T><<<vb(n), 256, 0, h.stream>>>(x, r, d, b, t, Dinv, n, (T)inv_theta, with_x ? 1 : 0);
-            count_launch();
-        }
-    }
-    T* dcur = d;
-    T* dnext = t;
-    for (int k = 1; k < deg; ++k) {
-        const T c1 = (T)cc1[k], c2 = (T)cc2[k];
-        OpEpi<T> E;
-        E.mode = 2;
-        E.r = r;
-        E.dinv = Dinv;
-        E.dold = dcur;
-        E.dnew = dnext;
-        E.x = x;
-        E.c1 = c1;
-        E.c2 = c2;
-        E.x_pend = pend;
-        if (epi_apply(h, l, dcur, E)) {
-            std::swap(dcur, dnext);
-        } else {
-            if (pend) {
-                k_add_pend<T><<<vb(n), 256, 0, h.stream>>>(x, dcur, n);
-                count_launch();
-            }
-            level_apply<T>(h, l, dcur, t);
-            k_cheb_step<T><<<vb(n), 256, 0, h.stream>>>(x, r, dcur, t, Dinv, n, c1, c2);
-            count_launch();
-        }
-        pend = false;
-    }
+    level_apply<T>(h, l, x, t);
+    k_cheb_step<T><<<vb(n), 256, 0, h.stream>>>(E, t, n);
     EQC_CHECK_LAUNCH();
-    return pend ? dcur : nullptr;
+    count_launch();
 }
 
-// 1 / theta of level l's Chebyshev interval (as chebyshev() computes it)
-static double cheb_inv_theta(const MGHier& m, int l) {
-    double it = 0.0;
-    cheb_coeffs(m, l, 1, &it, nullptr, nullptr);
-    return it;
-}
+// The V-cycle on the spectral-element level with its vector work in the operator's launches (sem.cu):
+// the first pre-smoothing step and the prolongation are formed as the operand is loaded, the
+// residual goes straight into the restriction, and the last launch leaves z.r for the CG.
+static void vcycle_sem(Handle& h, float* x, const float* b, CGState* S);
 
-// first_done: the restriction that produced b already took level l's first smoothing step.
-// Returns the post-smoothing's pending direction (chebyshev), null when x is complete.
+// One V-cycle of level l on A_l x = b from x = 0.  first_done: the restriction that produced b already
+// stored the first smoothing step's iterate.
 template <class T>
-static const T* vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) {
+static void vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) {
     MGHier& m = *h.mg;
     const int L = (int)m.lev.size();
-    if (l == L) {  // coarsest: dense solve on rows >= 1
+    cudaStream_t s = h.stream;
+    if (l == L) {  // coarsest: dense solve on rows >= 1 (row 0 of its vectors stays 0)
         StencilLevel& c = m.lev[L - 1];
-        const int64_t n = (int64_t)c.cx * c.cy;
-        EQC_CUDA(cudaMemsetAsync(x, 0, sizeof(T) * c.cx, h.stream));
-        k_dense_mv<T><<<(m.nc * 32 + 255) / 256, 256, 0, h.stream>>>(Sel<T>::C(m), b, x, m.nc, c.cx);
+        k_dense_mv<T><<<(m.nc + DN_WARPS - 1) / DN_WARPS, 32 * DN_WARPS, 0, s>>>(Sel<T>::C(m), b, x, m.nc, m.nc_pitch, c.cx);
         EQC_CHECK_LAUNCH();
         count_launch();
-        (void)n;
-        return nullptr;
+        return;
     }
     MGWork& w = m.work[l];
     const int64_t n = level_size(h, l);
-    chebyshev<T>(h, l, x, b, false, first_done);   // from x = 0: nothing pending
-    // residual r = b - A x, fused into the operator where it has the epilogue
-    T* t = Sel<T>::t(w);
-    T* r = Sel<T>::r(w);
-    OpEpi<T> E;
-    E.mode = 1;
-    E.b = b;
-    E.r = r;
-    if (!epi_apply(h, l, x, E)) {
-        level_apply<T>(h, l, x, t);
-        k_sub<T><<<vb(n), 256, 0, h.stream>>>(b, t, r, n);
+    const CycleVecs<T> V = cycle_vecs<T>(m, w, l, x);
+    std::vector<double> cc1(V.deg), cc2(V.deg);
+    double it = 0.0;
+    cheb_coeffs(m, l, V.deg, &it, cc1.data(), cc2.data());
+    const T inv_theta = (T)it;
+    // pre-smoothing from x = 0
+    if (!first_done) {
+        k_cheb_first<T><<<vb(n), 256, 0, s>>>(V.pre_iter(1), b, (l == 0) ? Sel<T>::Di0(m) : Sel<T>::Di(m.lev[l - 1]), n,
+                                              inv_theta);
+        EQC_CHECK_LAUNCH();
         count_launch();
     }
-    DevTransfer& tr = m.T[l];
+    for (int k = 1; k < V.deg; ++k)
+        cheb_step<T>(h, l, V.pre_iter(k), k > 1 ? V.pre_iter(k - 1) : nullptr, k == 1, V.pre_iter(k + 1), b, (T)cc1[k],
+                     (T)cc2[k]);
+    // restriction of the residual b - A x, with the coarse level's first smoothing step (not into the
+    // dense level)
+    const StencilLevel& lc = m.lev[l];
     MGWork& wc = m.work[l + 1];
     T* bc = Sel<T>::b(wc);
     T* xc = Sel<T>::x(wc);
-    const GllW<T> gw = gll_weights<T>(m);
-    // the coarse level's first smoothing step rides on the restriction (not into the dense level)
     ChebFirst<T> F;
-    const bool fuse = h.fuse && l + 1 < L;
-    if (fuse) {
+    if (l + 1 < L) {
+        double itc = 0.0;
+        cheb_coeffs(m, l + 1, 1, &itc, nullptr, nullptr);
         F.dinv = Sel<T>::Di(m.lev[l]);
-        F.x = xc;
-        F.r = Sel<T>::r(wc);
-        F.d = Sel<T>::d(wc);
-        F.inv_theta = (T)cheb_inv_theta(m, l + 1);
+        F.x = cycle_vecs<T>(m, wc, l + 1, xc).pre_iter(1);
+        F.inv_theta = (T)itc;
     }
-    if (l == 0) {
-        k_restrict_sem<T><<<dim3((tr.ncx + 127) / 128, tr.ncy), 128, 0, h.stream>>>(r, bc, h.L, tr.ldc, gw, F);
+    const dim3 cgrid((lc.cx + RCX - 1) / RCX, (lc.cy + RCY - 1) / RCY);
+    const Coarsen X = {l > 0 ? m.lev[l - 1].cx : 0, lc.cx}, Y = {l > 0 ? m.lev[l - 1].cy : 0, lc.cy};   // vertex levels
+    if (l > 0 && h.fuse) {
+        StencilLevel& lev = m.lev[l - 1];
+        k_restrict<T><<<cgrid, RFX * RFY, 0, s>>>(LdResidual<T>{Sel<T>::A(lev), V.pre, b, lev.cx, lev.cy}, bc, X, Y, F);
     } else {
-        k_restrict<T><<<vb((int64_t)tr.ncx * tr.ncy), 256, 0, h.stream>>>(r, bc, tr.ncx, tr.ncy, tr.ldf, tr.ldc,
-                                                                           tr.rpx.p, tr.rix.p, Sel<T>::rwx(tr), tr.rpy.p,
-                                                                           tr.riy.p, Sel<T>::rwy(tr), F);
-    }
-    count_launch();
-    const T* pc = vcycle<T>(h, l + 1, xc, bc, fuse);
-    if (l == 0) {
-        k_prolong_sem<T><<<dim3((h.L.NelX + 127) / 128, h.L.ny - 1), 128, 0, h.stream>>>(xc, x, h.L, tr.ldc, gw, pc);
-    } else {
-        k_prolong_add<T><<<vb((int64_t)tr.nfx * tr.nfy), 256, 0, h.stream>>>(xc, x, tr.nfx, tr.nfy, tr.ldf, tr.ldc,
-                                                                             tr.px.p, tr.py.p, Sel<T>::wx(tr),
-                                                                             Sel<T>::wy(tr), pc);
+        T* r = Sel<T>::r(w);
+        OpEpi<T> E;
+        E.mode = 1;
+        E.b = b;
+        E.out = r;
+        if (!epi_apply(h, l, V.pre, E)) {
+            level_apply<T>(h, l, V.pre, r);
+            k_sub<T><<<vb(n), 256, 0, s>>>(b, r, r, n);
+            count_launch();
+        }
+        if (l == 0)
+            k_restrict_sem<T><<<dim3((lc.cx + 127) / 128, lc.cy), 128, 0, s>>>(r, bc, h.L, lc.cx, gll_weights<T>(m), F);
+        else
+            k_restrict<T><<<cgrid, RFX * RFY, 0, s>>>(LdPlain<T>{r, X.nf}, bc, X, Y, F);
     }
     count_launch();
     EQC_CHECK_LAUNCH();
-    return chebyshev<T>(h, l, x, b, true);
+    vcycle<T>(h, l + 1, xc, bc, l + 1 < L);
+    // prolongation and post-smoothing
+    if (l > 0 && h.fuse) {
+        StencilLevel& lev = m.lev[l - 1];
+        k_prolong_smooth<T><<<dim3((lev.cx + VTX - 3) / (VTX - 2), (lev.cy + VTY - 3) / (VTY - 2)), dim3(VTX, VTY), 0, s>>>(
+            Sel<T>::A(lev), b, Sel<T>::Di(lev), V.deg > 1 ? V.post0 : nullptr, V.post1, LdProlonged<T>{V.pre, xc, X, Y},
+            inv_theta);
+        count_launch();
+    } else {
+        if (l == 0)
+            k_prolong_sem<T><<<dim3((h.L.NelX + 127) / 128, h.L.ny), 128, 0, s>>>(V.pre, xc, V.post0, h.L, lc.cx,
+                                                                                gll_weights<T>(m));
+        else
+            k_prolong<T><<<vgrid2(X.nf, Y.nf), dim3(VTX, VTY), 0, s>>>(V.post0, LdProlonged<T>{V.pre, xc, X, Y});
+        count_launch();
+        cheb_step<T>(h, l, V.post0, nullptr, false, V.post1, b, T(0), inv_theta);
+    }
+    EQC_CHECK_LAUNCH();
+    for (int k = 1; k < V.deg; ++k) {   // iterate k in post1 (k odd) or post0, the one before it in the other
+        T* cur = (k & 1) ? V.post1 : V.post0;
+        T* other = (k & 1) ? V.post0 : V.post1;
+        cheb_step<T>(h, l, cur, other, false, other, b, (T)cc1[k], (T)cc2[k]);
+    }
 }
 
-// The whole V-cycle on level 0 with any pending direction added to x.
-template <class T>
-static void vcycle0(Handle& h, T* x, const T* b) {
-    const T* p = vcycle<T>(h, 0, x, b);
-    if (p) {
-        const int64_t n = level_size(h, 0);
-        k_add_pend<T><<<vb(n), 256, 0, h.stream>>>(x, p, n);
+static void vcycle_sem(Handle& h, float* x, const float* b, CGState* S) {
+    MGHier& m = *h.mg;
+    const int L = (int)m.lev.size();
+    MGWork& w = m.work[0];
+    MGWork& wc = m.work[1];
+    const CycleVecs<float> V = cycle_vecs<float>(m, w, 0, x);
+    std::vector<double> cc1(V.deg), cc2(V.deg);
+    double it = 0.0;
+    cheb_coeffs(m, 0, V.deg, &it, cc1.data(), cc2.data());
+    SemOp o;
+    o.b = b;
+    o.dinv = m.Dinv0_32.p;
+    o.inv_theta = (float)it;
+    o.w = gll_weights<float>(m);
+    if (V.deg == 1) {
+        const int64_t n = h.L.size();
+        k_cheb_first<float><<<vb(n), 256, 0, h.stream>>>(V.pre, b, o.dinv, n, o.inv_theta);
         EQC_CHECK_LAUNCH();
         count_launch();
+    }
+    for (int k = 1; k < V.deg; ++k) {
+        o.x = V.pre_iter(k);
+        o.out = V.pre_iter(k + 1);
+        o.xp = k > 2 ? V.pre_iter(k - 1) : nullptr;
+        o.c1 = (float)cc1[k];
+        o.c2 = (float)cc2[k];
+        sem_launch(h, k == 1 ? SL_FIRST : SL_PLAIN, SE_CHEB, k == 1 ? SP_ZERO : (k == 2 ? SP_FIRST : SP_VEC), o);
+    }
+    o.x = V.pre;
+    o.bc = wc.b32.p;
+    if (L > 1) {
+        double itc = 0.0;
+        cheb_coeffs(m, 1, 1, &itc, nullptr, nullptr);
+        o.first.dinv = m.lev[0].Dinv32.p;
+        o.first.x = cycle_vecs<float>(m, wc, 1, wc.x32.p).pre_iter(1);
+        o.first.inv_theta = (float)itc;
+    }
+    sem_launch(h, SL_PLAIN, SE_RESTRICT, SP_NONE, o);
+    vcycle<float>(h, 1, wc.x32.p, wc.b32.p, L > 1);
+    o.xc = wc.x32.p;
+    o.uout = V.post0;
+    o.out = V.post1;
+    o.c1 = 0.f;
+    o.c2 = (float)it;
+    o.S = S;
+    o.part = h.red_part.p;
+    o.count = h.red_count.p;
+    o.dot = V.deg == 1 ? 1 : 0;
+    sem_launch(h, SL_PROLONG, SE_CHEB, SP_NONE, o);
+    for (int k = 1; k < V.deg; ++k) {   // iterate k in post1 (k odd) or post0, the one before it in the other
+        float* other = (k & 1) ? V.post0 : V.post1;
+        o.x = (k & 1) ? V.post1 : V.post0;
+        o.xp = other;
+        o.out = other;
+        o.c1 = (float)cc1[k];
+        o.c2 = (float)cc2[k];
+        o.dot = k + 1 == V.deg ? 1 : 0;
+        sem_launch(h, SL_PLAIN, SE_CHEB, SP_VEC, o);
     }
 }
 
@@ -437,44 +541,20 @@ static void vcycle0(Handle& h, T* x, const T* b) {
 void mg_apply64(Handle& h, const double* r, double* z) {
     if (!h.mg) throw Error(EQC_E_STATE, "multigrid not built");
     const int64_t ld = h.L.ld;
-    vcycle0<double>(h, z - ld, r - ld);
+    vcycle<double>(h, 0, z - ld, r - ld);
 }
-void mg_apply32(Handle& h, const float* r, float* z) {
+bool mg_apply32(Handle& h, const float* r, float* z, CGState* S) {
     if (!h.mg) throw Error(EQC_E_STATE, "multigrid not built");
     const int64_t ld = h.L.ld;
-    vcycle0<float>(h, z - ld, r - ld);
+    if (h.fuse && sem_usable(h)) {
+        vcycle_sem(h, z - ld, r - ld, S);
+        return true;
+    }
+    vcycle<float>(h, 0, z - ld, r - ld);
+    return false;
 }
 
 // ------------------------------------------------------------------ setup
-static void upload_transfer(Handle& h, DevTransfer& d, const Transfer1D& tx, const Transfer1D& ty, int ldf, int ldc) {
-    cudaStream_t s = h.stream;
-    d.nfx = tx.nf;
-    d.nfy = ty.nf;
-    d.ncx = tx.nc;
-    d.ncy = ty.nc;
-    d.ldf = ldf;
-    d.ldc = ldc;
-    auto up_i = [&](DBuf<int>& b, const std::vector<int>& v) { b.alloc(v.size()); b.upload(v.data(), v.size(), s); };
-    auto up_w = [&](DBuf<double>& b64, DBuf<float>& b32, const std::vector<double>& v) {
-        b64.alloc(v.size());
-        b64.upload(v.data(), v.size(), s);
-        std::vector<float> f(v.begin(), v.end());
-        b32.alloc(f.size());
-        b32.upload(f.data(), f.size(), s);
-    };
-    up_i(d.px, tx.p_idx);
-    up_i(d.py, ty.p_idx);
-    up_w(d.wx64, d.wx32, tx.p_w);
-    up_w(d.wy64, d.wy32, ty.p_w);
-    up_i(d.rpx, tx.r_ptr);
-    up_i(d.rix, tx.r_idx);
-    up_w(d.rwx64, d.rwx32, tx.r_w);
-    up_i(d.rpy, ty.r_ptr);
-    up_i(d.riy, ty.r_idx);
-    up_w(d.rwy64, d.rwy32, ty.r_w);
-    EQC_CUDA(cudaStreamSynchronize(s));
-}
-
 static void alloc_work(MGWork& w, int64_t n) {
     for (DBuf<double>* b : {&w.x64, &w.b64, &w.r64, &w.d64, &w.t64}) b->alloc(n);
     for (DBuf<float>* b : {&w.x32, &w.b32, &w.r32, &w.d32, &w.t32}) b->alloc(n);
@@ -581,20 +661,19 @@ void mg_build(Handle& h) {
         lv.Dinv32.upload(df.data(), N, s);
         EQC_CUDA(cudaStreamSynchronize(s));
     }
-    // transfers: T[0] SEM -> vertex grid, T[k] lev[k-1] -> lev[k]
-    m.T.resize(m.lev.size());
-    upload_transfer(h, m.T[0], tx[0], ty[0], L.ld, m.lev[0].cx);
-    for (size_t k = 1; k < m.lev.size(); ++k)
-        upload_transfer(h, m.T[k], tx[k], ty[k], m.lev[k - 1].cx, m.lev[k].cx);
     // coarsest dense inverse
     {
         StencilLevel& c = m.lev.back();
         std::vector<double> inv = dense_inverse_spd(c.A, c.cx, c.cy, m.nc);
-        std::vector<float> f(inv.begin(), inv.end());
-        m.Cinv64.alloc(inv.size());
-        m.Cinv64.upload(inv.data(), inv.size(), s);
+        m.nc_pitch = (m.nc + 3) / 4 * 4;
+        std::vector<double> d((size_t)m.nc * m.nc_pitch, 0.0);
+        for (int r = 0; r < m.nc; ++r) std::copy_n(inv.begin() + (size_t)r * m.nc, m.nc, d.begin() + (size_t)r * m.nc_pitch);
+        std::vector<float> f(d.begin(), d.end());
+        m.Cinv64.alloc(d.size());
+        m.Cinv64.upload(d.data(), d.size(), s);
         m.Cinv32.alloc(f.size());
         m.Cinv32.upload(f.data(), f.size(), s);
+        EQC_CUDA(cudaStreamSynchronize(s));
     }
     // work vectors
     m.work.resize(m.lev.size() + 1);

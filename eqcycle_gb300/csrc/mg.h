@@ -28,15 +28,6 @@ struct Transfer1D {
     std::vector<double> r_w;
 };
 
-struct DevTransfer {
-    int nfx, nfy, ncx, ncy;      // grid sizes (with the fault row)
-    int ldf, ldc;                // row pitches
-    int rmaxx, rmaxy;            // max restriction row lengths
-    DBuf<int> px, py, rpx, rpy, rix, riy;
-    DBuf<double> wx64, wy64, rwx64, rwy64;
-    DBuf<float> wx32, wy32, rwx32, rwy32;
-};
-
 struct StencilLevel {
     int cx = 0, cy = 0;          // vertex grid size including the fault row (row 0 unused)
     std::vector<double> A;       // host [9][cx*cy], offsets (dx,dy) in {-1,0,1}^2, k = (dy+1)*3+(dx+1)
@@ -60,9 +51,8 @@ struct MGHier {
     DBuf<double> Dinv0_64;
     DBuf<float> Dinv0_32;
     std::vector<StencilLevel> lev;    // levels 1..L
-    std::vector<DevTransfer> T;       // T[0]: SEM -> lev[0]; T[k]: lev[k-1] -> lev[k]
     std::vector<MGWork> work;         // work[0]: SEM level; work[k]: lev[k-1]
-    int nc = 0;                       // coarsest dense size
+    int nc = 0, nc_pitch = 0;         // coarsest dense size, row pitch of its inverse
     DBuf<double> Cinv64;
     DBuf<float> Cinv32;
     int64_t launches_per_vcycle = 0;

@@ -57,6 +57,8 @@ constexpr int KD_REFRESH = 256;
 // Device-resident scalars of one CG solve.
 struct CGState {
     double rho, rho_prev, pq, rr, bb;
+    double alpha, beta;         // rho / pq, rho / rho_prev: divided once, by the reductions' last CTAs
+    float alpha32, beta32;
     double nb, reltol, res, rmax;
     int it, maxit;
     int done;          // 0 running, 1 converged, 2 maxit reached, 3 non-finite residual
@@ -68,6 +70,8 @@ struct CGState {
     double sigma;      // mixed precision: the FP32 recurrence vectors hold sigma * (true value),
                        // sigma a power of two near 1 / ||b|| (keeps tiny residuals out of
                        // FP32 underflow); 1 in FP64.  rr is in those scaled units.
+    double inv_sigma;  // 1 / sigma
+    int sigma_exp;     // sigma = 2^sigma_exp
     double rr_guess;   // ||r||^2 with the initial-guess increment applied
     int guess_keep;    // the increment lowered the residual and is kept
 };
@@ -148,6 +152,8 @@ struct Handle {
     // element data
     DBuf<double> W64, W64p;
     DBuf<double> mu64;   // rigidity per element, -1 where it varies within one (classify_elements)
+    DBuf<float> mu32;    // the same in FP32, without the shifted column
+    bool sem_ok = false; // the FP32 operator of sem.cu pays (classify_elements)
     bool uni_ok = false; // H admits the one-contraction lines of the FP64 apply
     DBuf<float> W32, W32p;
     DBuf<float> W32lo;   // W - W32p rounded to FP32 (padded like W32p): W as double-float
@@ -182,6 +188,7 @@ struct Handle {
     // CG work vectors
     DBuf<double> r64, z64, p64, q64;
     DBuf<float> r32, z32, p32, q32, x32;
+    DBuf<float> p32b;     // the other iterations' direction where the operator's launch forms it (sem.cu)
     DBuf<float> g32;      // initial-guess increment added to d before the first solve of a step
     // multigrid
     MGHier* mg = nullptr;     // owned; released by mg_destroy
@@ -227,18 +234,17 @@ void set_H_df(const double* H, cudaStream_t s);
 bool apply_K_df(Handle& h, const double* x, double* y, double sign, int mode, cudaStream_t s,
                 const int* gate = nullptr, int gate_val = 0);
 void tma_init_for(TmaCache& c, const Layout& L, const float* W32p, const double* W64p, const double* mu);
-// FP32 apply y = K x (mode 0/1 as apply_K) whose owned nodes are finished by the epilogue E
+// Apply y = K x (mode 0/1 as apply_K) whose owned nodes are finished by the epilogue E
 // (residual or Chebyshev step) instead of stored; false when the selected kernel has none.
 bool apply_K_epi(const float* x, const ApplyArgs<float>& A, int mode, const OpEpi<float>& E, cudaStream_t s);
+bool apply_K_epi(const double* x, const ApplyArgs<double>& A, int mode, const OpEpi<double>& E, cudaStream_t s);
 // y = K x (FP32) on the node rows 0..3 of the fault's element row, by the element-per-lane
 // arithmetic of the full FP32 applies (variants 0 and 4-8): row 0 has the bits of their row 0.
 // False when the padded element data or 16-byte aligned vectors are missing.
 bool apply_K_fault32(const float* x, float* y, const ApplyArgs<float>& A, cudaStream_t s);
 
 // blas.cu
-int vec_blocks();   // grid of the vector and reduction kernels
 void dot64(Handle& h, const double* x, const double* y, int64_t n, double* out_dev);
-void dot32(Handle& h, const float* x, const float* y, int64_t n, double* out_dev);
 
 // solver.cu
 // Enqueues one CG solve on h.stream.  graph: inside a stream capture, the iteration loop
@@ -299,7 +305,8 @@ double fault_dtevol(Handle& h, double dt, double dtmin, const double* Vf, int is
 void mg_build(Handle& h);
 void mg_destroy(Handle& h);
 void mg_apply64(Handle& h, const double* r, double* z);
-void mg_apply32(Handle& h, const float* r, float* z);
+// ... true when its last launch also left rho = z.r and beta in S
+bool mg_apply32(Handle& h, const float* r, float* z, CGState* S);
 
 }  // namespace eqc
 

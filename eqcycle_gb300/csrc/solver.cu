@@ -17,27 +17,30 @@
 #include "reduce.cuh"
 #include "vec.cuh"
 #include "epi.cuh"
+#include "cg.cuh"
+#include "sem.h"
 #include <cmath>
-#include <cstddef>
 
 namespace eqc {
 
-// Slots of the scalar block the vector kernels address (the leading doubles of CGState).
-enum { S_RHO = 0, S_RHOP = 1, S_PQ = 2, S_RR = 3, S_BB = 4 };
-static_assert(offsetof(CGState, rho_prev) == 8 * S_RHOP && offsetof(CGState, pq) == 8 * S_PQ &&
-                  offsetof(CGState, rr) == 8 * S_RR && offsetof(CGState, bb) == 8 * S_BB,
-              "CGState must start with rho, rho_prev, pq, rr, bb");
+template <class T> __device__ __forceinline__ T cg_alpha(const CGState* S);
+template <> __device__ __forceinline__ float cg_alpha<float>(const CGState* S) { return S->alpha32; }
+template <> __device__ __forceinline__ double cg_alpha<double>(const CGState* S) { return S->alpha; }
+template <class T> __device__ __forceinline__ T cg_beta(const CGState* S);
+template <> __device__ __forceinline__ float cg_beta<float>(const CGState* S) { return S->beta32; }
+template <> __device__ __forceinline__ double cg_beta<double>(const CGState* S) { return S->beta; }
 
-// The vector kernels run on a fixed grid of VEC_BLOCKS x VEC_THREADS threads over 4-wide
-// chunks (n is a multiple of 4: every vector is a whole number of 8-entry-aligned rows);
-// reductions are deterministic (fixed slices, partials summed in CTA order).
+// The vector kernels run on a fixed grid (vec_blocks) over 4-wide chunks (n is a multiple of 4: every
+// vector is a whole number of 8-entry-aligned rows); reductions are deterministic (fixed slices,
+// partials summed in a fixed order).  No thread but a reduction's last one divides in FP64: a division
+// by every thread (alpha = rho / pq) held the FP64 pipe of an SM for 2 us per launch.
 
-// dot into S_RHO, shifting the previous value into S_RHOP
+// pq = 0: rho = x.y (the previous value into rho_prev) and beta = rho / rho_prev;
+// pq = 1: pq = x.y and alpha = rho / pq
 template <class T>
-__global__ void __launch_bounds__(VEC_THREADS) k_dot_rho(const T* __restrict__ x, const T* __restrict__ y, int64_t n,
-                                                         double* part, unsigned* count, double* S) {
+__global__ void __launch_bounds__(VEC_THREADS, VEC_PER_SM<T>) k_dot_cg(const T* __restrict__ x, const T* __restrict__ y, int64_t n,
+                                                        double* part, unsigned* count, CGState* S, int pq) {
     EQC_GRID_WAIT();
-    __shared__ double sh[32];
     DotAcc<T> acc;
     for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
         T a[4], b[4];
@@ -46,25 +49,21 @@ __global__ void __launch_bounds__(VEC_THREADS) k_dot_rho(const T* __restrict__ x
 #pragma unroll
         for (int k = 0; k < 4; ++k) acc.add(a[k], b[k]);
     }
-    const double s = block_sum(acc.value(), sh);
-    finish_reduction(s, part, count, sh, [&](double t) {
-        S[S_RHOP] = S[S_RHO];
-        S[S_RHO] = t;
-    });
+    grid_sum(acc, part, count, [&](double t) { cg_take_dot(S, t, pq != 0); });
 }
 
 // u = z + (rho / rho_prev) u   (u = z after a restart)
 template <class T>
-__global__ void __launch_bounds__(VEC_THREADS) k_pupdate(const T* __restrict__ z, T* __restrict__ u, int64_t n,
-                                                         const double* S, const int* restart) {
+__global__ void __launch_bounds__(VEC_THREADS, VEC_PER_SM<T>) k_pupdate(const T* __restrict__ z, T* __restrict__ u, int64_t n,
+                                                         const CGState* S) {
     EQC_GRID_WAIT();
-    const T b = *restart ? T(0) : (T)(S[S_RHO] / S[S_RHOP]);
+    const T b = S->restart ? T(0) : cg_beta<T>(S);
     for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
         T zz[4], uu[4];
         ld4(z + i, zz);
         ld4(u + i, uu);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) uu[k] = zz[k] + b * uu[k];
+        for (int k = 0; k < 4; ++k) uu[k] = fma_rn<T>(b, uu[k], zz[k]);
         st4(u + i, uu);
     }
 }
@@ -80,46 +79,40 @@ struct CheckA {
 __device__ __forceinline__ int cg_check_a(CGState* S, double delta);
 __device__ __forceinline__ int cg_check64(CGState* S);
 
-// x += alpha u ; r -= alpha q ; S_RR = r.r   (alpha = rho / (u.q)); then the update decision
-// (ck.on: S is the CGState)
-template <class TX, class T>
-__global__ void __launch_bounds__(VEC_THREADS) k_xr_update(TX* __restrict__ x, T* __restrict__ r, const T* __restrict__ u,
-                                                           const T* __restrict__ q, int64_t n, double* part,
-                                                           unsigned* count, double* S, CheckA ck) {
+// x += alpha u ; r -= alpha q ; rr = r.r   (alpha = rho / (u.q)); then the update decision
+template <class T>
+__global__ void __launch_bounds__(VEC_THREADS, VEC_PER_SM<T>) k_xr_update(T* __restrict__ x, T* __restrict__ r, const T* __restrict__ u,
+                                                           const T* __restrict__ u_odd, const T* __restrict__ q, int64_t n,
+                                                           double* part, unsigned* count, CGState* S, CheckA ck) {
     EQC_GRID_WAIT();
-    __shared__ double sh[32];
-    const double alpha = S[S_RHO] / S[S_PQ];
-    const T a = (T)alpha;
-    const TX ax = (TX)alpha;
+    if (u_odd && (S->it & 1)) u = u_odd;   // the direction of odd iterations (read before the last CTA's check)
+    const T a = cg_alpha<T>(S);
     DotAcc<T> acc;
     for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
-        TX xx[4];
-        T rr[4], uu[4], qq[4];
+        T xx[4], rr[4], uu[4], qq[4];
         ld4(x + i, xx);
         ld4(r + i, rr);
         ld4(u + i, uu);
         ld4(q + i, qq);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            xx[k] = xx[k] + ax * (TX)uu[k];
+            xx[k] = xx[k] + a * uu[k];
             rr[k] = rr[k] - a * qq[k];
             acc.add(rr[k], rr[k]);
         }
         st4(x + i, xx);
         st4(r + i, rr);
     }
-    const double s = block_sum(acc.value(), sh);
-    finish_reduction(s, part, count, sh, [&](double t) {
-        S[S_RR] = t;
-        CGState* cs = reinterpret_cast<CGState*>(S);
+    grid_sum(acc, part, count, [&](double t) {
+        S->rr = t;
         if (ck.on == 1) {
-            const int need = cg_check_a(cs, ck.delta);
+            const int need = cg_check_a(S, ck.delta);
             if (ck.use_cond) {
                 cudaGraphSetConditional(ck.hi, need ? 1u : 0u);
-                cudaGraphSetConditional(ck.hw, cs->done == 0 ? 1u : 0u);
+                cudaGraphSetConditional(ck.hw, S->done == 0 ? 1u : 0u);
             }
         } else if (ck.on == 2) {
-            const int st = cg_check64(cs);
+            const int st = cg_check64(S);
             if (ck.use_cond) cudaGraphSetConditional(ck.hw, st == 0 ? 1u : 0u);
         }
     });
@@ -141,8 +134,8 @@ __global__ void k_jacobi(const T* __restrict__ r, const T* __restrict__ dg, T* _
 __global__ void __launch_bounds__(VEC_THREADS) k_fold(double* __restrict__ x, float* __restrict__ y,
                                                       double* __restrict__ dx, int64_t n, const CGState* S) {
     EQC_GRID_WAIT();
-    const double inv = 1.0 / S->sigma;
-    const int es = -ilogb(S->sigma);
+    const double inv = S->inv_sigma;
+    const int es = -S->sigma_exp;
     const bool incr = dx && S->upd_incr;
     for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
         double xx[4], dd[4];
@@ -169,7 +162,7 @@ __global__ void k_dx_init(double* __restrict__ dx, const float* __restrict__ g, 
     EQC_GRID_WAIT();
     const bool keep = g && S->guess_keep;
     const double sg = S->sigma;
-    const int es = ilogb(sg);
+    const int es = S->sigma_exp;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         dx[i] = keep ? pow2_scale(f32_to_f64(g[i]), es, sg) : 0.0;
 }
@@ -183,9 +176,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_demote_norm(double* __restrict_
                                                              int64_t n, double* part, unsigned* count, CGState* S,
                                                              const double* __restrict__ kdx, double* __restrict__ dx) {
     EQC_GRID_WAIT();
-    __shared__ double sh[32];
-    const double sg = S->sigma;
-    const int es = ilogb(sg);
+    const double sg = S->sigma, inv = S->inv_sigma;
+    const int es = S->sigma_exp;
     const bool incr = kdx && S->upd_incr;
     DotAcc<float> acc;
     for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
@@ -193,7 +185,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_demote_norm(double* __restrict_
         float f[4];
         ld4(r64 + i, v);
         if (incr) {
-            const double inv = 1.0 / sg;   // a power of two: exact
             double t[4];
             ld4(kdx + i, t);
 #pragma unroll
@@ -211,8 +202,7 @@ __global__ void __launch_bounds__(VEC_THREADS) k_demote_norm(double* __restrict_
         }
         st4(r32 + i, f);
     }
-    const double s = block_sum(acc.value(), sh);
-    finish_reduction(s, part, count, sh, [&](double t) { S->rr = t; });
+    grid_sum(acc, part, count, [&](double t) { S->rr = t; });
 }
 
 // Scale of the FP32 recurrence for this solve: sigma = 2^-e with 2^e <= ||b|| < 2^(e+1)
@@ -220,10 +210,13 @@ __global__ void __launch_bounds__(VEC_THREADS) k_demote_norm(double* __restrict_
 __global__ void k_set_sigma(CGState* S, int mixed) {
     EQC_GRID_WAIT();
     const double nb = sqrt(S->bb);
-    S->sigma = (mixed && nb > 0 && isfinite(nb)) ? ldexp(1.0, -ilogb(nb)) : 1.0;
+    const int e = (mixed && nb > 0 && isfinite(nb)) ? -ilogb(nb) : 0;
+    S->sigma_exp = e;
+    S->sigma = ldexp(1.0, e);
+    S->inv_sigma = 1.0 / S->sigma;   // a power of two: exact
 }
 
-static inline dim3 vgrid() { return dim3(vec_blocks()); }
+template <class T> static inline dim3 vgrid(int64_t n) { return dim3(vec_blocks<T>(n)); }
 
 // ---- device-side control of the CG loop -----------------------------------------------
 // Every control kernel is a single thread: it owns the CGState and is the only caller of
@@ -235,7 +228,7 @@ __global__ void k_cg_init(CGState* S, double tol, int maxit, int rule, int incr_
     EQC_GRID_WAIT();
     S->incr_ok = incr_ok;
     S->upd_incr = 0;
-    const double nb = sqrt(S->bb), r = sqrt(S->rr) / S->sigma;
+    const double nb = sqrt(S->bb), r = sqrt(S->rr) * S->inv_sigma;
     const double reltol = (rule == EQC_TOL_R0 ? r : nb) * tol;
     S->nb = nb;
     S->reltol = reltol;
@@ -255,7 +248,7 @@ __global__ void k_cg_init(CGState* S, double tol, int maxit, int rule, int incr_
 // End of an FP64 iteration: the loop goes on until ||r|| <= reltol or maxit.
 __device__ __forceinline__ int cg_check64(CGState* S) {
     S->it += 1;
-    const double r = sqrt(S->rr) / S->sigma;
+    const double r = sqrt(S->rr) * S->inv_sigma;
     S->res = r;
     const int st = !isfinite(r) ? 3 : (r <= S->reltol ? 1 : (S->it >= S->maxit ? 2 : 0));
     S->done = st;
@@ -267,7 +260,7 @@ __device__ __forceinline__ int cg_check64(CGState* S) {
 __device__ __forceinline__ int cg_check_a(CGState* S, double delta) {
     S->it += 1;
     S->restart = 0;   // consumed by this iteration's direction update
-    const double rs = sqrt(S->rr) / S->sigma;
+    const double rs = sqrt(S->rr) * S->inv_sigma;
     int need = 0;
     if (!isfinite(rs)) {
         S->done = 3;
@@ -288,7 +281,7 @@ __global__ void k_cg_check_b(CGState* S, Ctrl* C, cudaGraphConditionalHandle hw,
     EQC_GRID_WAIT();
     if (S->done != 3) {
         if (S->need_update) {
-            const double rs = sqrt(S->rr) / S->sigma;
+            const double rs = sqrt(S->rr) * S->inv_sigma;
             // the true residual left the recurrence's (the FP32 recurrences drifted, e.g. from a
             // guess far from the solution): continue from the true residual with a fresh direction
             if (rs > 2.0 * S->res) {
@@ -339,10 +332,9 @@ __global__ void k_carry_rows(double* __restrict__ r64, const double* __restrict_
 
 // Carried residual after the guess increment g: r32 -= sigma K_II g (t = K_II g in FP32),
 // S->rr_guess = ||r32||^2 (S->rr keeps the residual without the increment).
-__global__ void __launch_bounds__(VEC_THREADS) k_guess_residual(float* __restrict__ r32, const float* __restrict__ t,
+__global__ void __launch_bounds__(VEC_THREADS, VEC_PER_SM<float>) k_guess_residual(float* __restrict__ r32, const float* __restrict__ t,
                                                                 int64_t n, double* part, unsigned* count, CGState* S) {
     EQC_GRID_WAIT();
-    __shared__ double sh[32];
     const float sg = (float)S->sigma;
     DotAcc<float> acc;
     for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
@@ -356,8 +348,7 @@ __global__ void __launch_bounds__(VEC_THREADS) k_guess_residual(float* __restric
         }
         st4(r32 + i, rr);
     }
-    const double s = block_sum(acc.value(), sh);
-    finish_reduction(s, part, count, sh, [&](double tt2) { S->rr_guess = tt2; });
+    grid_sum(acc, part, count, [&](double tt2) { S->rr_guess = tt2; });
 }
 
 // The previous-step guess judges the increment: keep it only if it lowered ||r||.
@@ -400,27 +391,10 @@ static const CGState& read_cg(Handle& h) {
 }
 
 template <class T>
-static void precond(Handle& h, const T* r, T* z, int64_t n);
-
-template <>
-void precond<double>(Handle& h, const double* r, double* z, int64_t n) {
-    if (h.opt.precond == EQC_PC_AMG) {
-        mg_apply64(h, r, z);
-    } else {
-        k_jacobi<double><<<vgrid(), VEC_THREADS, 0, h.stream>>>(r, h.diag64.p + h.L.ld, z, n);
-        EQC_CHECK_LAUNCH();
-        count_launch();
-    }
-}
-template <>
-void precond<float>(Handle& h, const float* r, float* z, int64_t n) {
-    if (h.opt.precond == EQC_PC_AMG) {
-        mg_apply32(h, r, z);
-    } else {
-        k_jacobi<float><<<vgrid(), VEC_THREADS, 0, h.stream>>>(r, h.diag32.p + h.L.ld, z, n);
-        EQC_CHECK_LAUNCH();
-        count_launch();
-    }
+static void jacobi(Handle& h, const T* r, const T* dg, T* z, int64_t n) {
+    k_jacobi<T><<<vgrid<T>(n), VEC_THREADS, 0, h.stream>>>(r, dg + h.L.ld, z, n);
+    EQC_CHECK_LAUNCH();
+    count_launch();
 }
 
 // Right-hand side: S->bb = ||b||^2 with b = -K_IF F on rows 1..4 (d holds F on row 0).
@@ -441,7 +415,7 @@ static void setup_residual_full(Handle& h, bool mixed) {
     CGState* S = h.cg.p;
     apply_K<double>(h.d.p, h.r64.p, args64(h), -1.0, 1, h.stream);     // r = -(K d)_I
     if (mixed) {
-        k_demote_norm<<<vgrid(), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p,
+        k_demote_norm<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p,
                                                              h.red_count.p, S, nullptr, h.dx64.p ? h.dx64.p + ld : nullptr);
         EQC_CHECK_LAUNCH();
         count_launch();
@@ -456,22 +430,22 @@ static void setup_residual_full(Handle& h, bool mixed) {
 static void setup_residual_carry(Handle& h, const float* guess) {
     const int64_t ld = h.L.ld, n = h.L.size() - ld;
     apply_K<double>(h.tmp64b.p, h.tmp64c.p, args64(h), -1.0, 2, h.stream);
-    k_carry_rows<<<vgrid(), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.tmp64c.p + ld, 4 * ld);
-    k_demote_norm<<<vgrid(), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p,
+    k_carry_rows<<<vgrid<double>(4 * ld), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.tmp64c.p + ld, 4 * ld);
+    k_demote_norm<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p,
                                                          h.red_count.p, h.cg.p, nullptr, h.dx64.p ? h.dx64.p + ld : nullptr);
     EQC_CHECK_LAUNCH();
     count_launch(2);
     if (guess) {
         apply_K<float>(guess, h.q32.p, args32(h), 1.0f, 1, h.stream);
-        k_guess_residual<<<vgrid(), VEC_THREADS, 0, h.stream>>>(h.r32.p + ld, h.q32.p + ld, n, h.red_part.p,
+        k_guess_residual<<<vgrid<float>(n), VEC_THREADS, 0, h.stream>>>(h.r32.p + ld, h.q32.p + ld, n, h.red_part.p,
                                                                 h.red_count.p, h.cg.p);
         k_guess_decide<<<1, 1, 0, h.stream>>>(h.cg.p, h.ctrl.p);
-        k_guess_revert<<<vgrid(), VEC_THREADS, 0, h.stream>>>(h.cg.p, h.d.p + ld, guess + ld, h.r32.p + ld,
+        k_guess_revert<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.cg.p, h.d.p + ld, guess + ld, h.r32.p + ld,
                                                               h.r64.p + ld, n);
         EQC_CHECK_LAUNCH();
         count_launch(3);
         if (h.dx64.p) {   // r64 is the residual without the kept increment
-            k_dx_init<<<vgrid(), VEC_THREADS, 0, h.stream>>>(h.dx64.p + ld, guess + ld, h.cg.p, n);
+            k_dx_init<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.dx64.p + ld, guess + ld, h.cg.p, n);
             EQC_CHECK_LAUNCH();
             count_launch();
         }
@@ -488,19 +462,19 @@ static void iter_fp64(Handle& h, cudaGraphConditionalHandle hw, int use_cond) {
     double* z = h.z64.p + ld;
     double* u = h.p64.p + ld;
     double* q = h.q64.p + ld;
-    precond<double>(h, r, z, n);
-    k_dot_rho<double><<<vgrid(), VEC_THREADS, 0, h.stream>>>(z, r, n, h.red_part.p, h.red_count.p, &S->rho);
-    k_pupdate<double><<<vgrid(), VEC_THREADS, 0, h.stream>>>(z, u, n, &S->rho, &S->restart);
+    if (h.opt.precond == EQC_PC_AMG) mg_apply64(h, r, z);
+    else jacobi(h, r, h.diag64.p, z, n);
+    k_dot_cg<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(z, r, n, h.red_part.p, h.red_count.p, S, 0);
+    k_pupdate<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(z, u, n, S);
     apply_K<double>(h.p64.p, h.q64.p, args64(h), 1.0, 1, h.stream);
-    dot64(h, u, q, n, &S->pq);
+    k_dot_cg<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(u, q, n, h.red_part.p, h.red_count.p, S, 1);
     CheckA ck;
     ck.on = 2;
     ck.use_cond = use_cond;
     ck.hw = hw;
-    k_xr_update<double, double><<<vgrid(), VEC_THREADS, 0, h.stream>>>(x, r, u, q, n, h.red_part.p, h.red_count.p,
-                                                                       &S->rho, ck);
+    k_xr_update<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(x, r, u, nullptr, q, n, h.red_part.p, h.red_count.p, S, ck);
     EQC_CHECK_LAUNCH();
-    count_launch(3);
+    count_launch(4);
 }
 
 // Mixed precision: FP32 recurrences of one iteration, ending with the update decision (hi) and,
@@ -515,21 +489,48 @@ static void iter_mixed_a(Handle& h, double delta, cudaGraphConditionalHandle hi,
     float* u = h.p32.p + ld;
     float* q = h.q32.p + ld;
     float* y = h.x32.p + ld;   // correction accumulated since the last reliable update
-    precond<float>(h, r, z, n);
-    k_dot_rho<float><<<vgrid(), VEC_THREADS, 0, h.stream>>>(z, r, n, h.red_part.p, h.red_count.p, &S->rho);
-    k_pupdate<float><<<vgrid(), VEC_THREADS, 0, h.stream>>>(z, u, n, &S->rho, &S->restart);
-    apply_K<float>(h.p32.p, h.q32.p, args32(h), 1.0f, 1, h.stream);
-    dot32(h, u, q, n, &S->pq);
+    bool rho_done = false;
+    if (h.opt.precond == EQC_PC_AMG) rho_done = mg_apply32(h, r, z, S);
+    else jacobi(h, r, h.diag32.p, z, n);
+    if (!rho_done) {
+        k_dot_cg<float><<<vgrid<float>(n), VEC_THREADS, 0, h.stream>>>(z, r, n, h.red_part.p, h.red_count.p, S, 0);
+        count_launch();
+    }
+    const float* u_odd = nullptr;
+    if (h.fuse && sem_usable(h)) {   // u = z + beta u, q = K u and u.q in one launch
+        SemOp o;
+        o.x = h.z32.p;
+        o.p0 = h.p32.p;
+        o.p1 = h.p32b.p;
+        o.out = h.q32.p;
+        o.dot = 2;
+        o.S = S;
+        o.part = h.red_part.p;
+        o.count = h.red_count.p;
+        sem_launch(h, SL_DIR, SE_STORE, SP_NONE, o);
+        u_odd = h.p32b.p + ld;
+    } else {
+        k_pupdate<float><<<vgrid<float>(n), VEC_THREADS, 0, h.stream>>>(z, u, n, S);
+        if (sem_usable(h)) {
+            SemOp o;
+            o.x = h.p32.p;
+            o.out = h.q32.p;
+            sem_launch(h, SL_PLAIN, SE_STORE, SP_NONE, o);
+        } else {
+            apply_K<float>(h.p32.p, h.q32.p, args32(h), 1.0f, 1, h.stream);
+        }
+        k_dot_cg<float><<<vgrid<float>(n), VEC_THREADS, 0, h.stream>>>(u, q, n, h.red_part.p, h.red_count.p, S, 1);
+        count_launch(2);
+    }
     CheckA ck;
     ck.on = 1;
     ck.use_cond = use_cond;
     ck.delta = delta;
     ck.hi = hi;
     ck.hw = hw;
-    k_xr_update<float, float><<<vgrid(), VEC_THREADS, 0, h.stream>>>(y, r, u, q, n, h.red_part.p, h.red_count.p,
-                                                                     &S->rho, ck);
+    k_xr_update<float><<<vgrid<float>(n), VEC_THREADS, 0, h.stream>>>(y, r, u, u_odd, q, n, h.red_part.p, h.red_count.p, S, ck);
     EQC_CHECK_LAUNCH();
-    count_launch(3);
+    count_launch();
 }
 
 // Reliable update: x += y ; r = b - K_II x in FP64 ; r32 = r ; S->rr = ||r||^2.
@@ -548,7 +549,7 @@ static void update_mixed(Handle& h) {
     const int64_t ld = L.ld, n = L.size() - ld;
     CGState* S = h.cg.p;
     const bool incr = incr_updates(h, true) != 0;
-    k_fold<<<vgrid(), VEC_THREADS, 0, h.stream>>>(h.d.p + ld, h.x32.p + ld, incr ? h.dx64.p + ld : nullptr, n, S);
+    k_fold<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.d.p + ld, h.x32.p + ld, incr ? h.dx64.p + ld : nullptr, n, S);
     ApplyArgs<double> a64 = args64(h);
     if (incr) {
         a64.gate = &S->upd_incr;
@@ -556,7 +557,7 @@ static void update_mixed(Handle& h) {
         apply_K_df(h, h.dx64.p, h.kdx64.p, -1.0, 1, h.stream, &S->upd_incr, 1);   // -K_II dx
     }
     apply_K<double>(h.d.p, h.r64.p, a64, -1.0, 1, h.stream);                    // r = -(K d)_I
-    k_demote_norm<<<vgrid(), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p, h.red_count.p,
+    k_demote_norm<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p, h.red_count.p,
                                                          S, incr ? h.kdx64.p + ld : nullptr, incr ? h.dx64.p + ld : nullptr);
     EQC_CHECK_LAUNCH();
     count_launch(2);
@@ -608,7 +609,8 @@ void enqueue_solve(Handle& h, double tol, int maxit, bool graph, bool carry, con
         setup_residual_full(h, mixed);
     }
     if (mixed) {
-        EQC_CUDA(cudaMemsetAsync(h.p32.p, 0, sizeof(float) * L.size(), h.stream));
+        float* p_before = h.fuse && sem_usable(h) ? h.p32b.p : h.p32.p;   // the direction before iteration 0
+        EQC_CUDA(cudaMemsetAsync(p_before, 0, sizeof(float) * L.size(), h.stream));
         EQC_CUDA(cudaMemsetAsync(h.x32.p, 0, sizeof(float) * L.size(), h.stream));
     } else {
         EQC_CUDA(cudaMemsetAsync(h.p64.p, 0, sizeof(double) * L.size(), h.stream));

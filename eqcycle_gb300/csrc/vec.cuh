@@ -5,14 +5,19 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "df.cuh"
 
 namespace eqc {
 
-// 3 CTAs of 256 threads per SM of a GB300: the reductions' last-CTA tickets and partials cost
-// less than with 8 per SM, and 4-wide grid-stride loops keep enough loads in flight (dz480
-// quasi-static steps: 73.0 ms for 20 with 8 per SM, 72.6 with 4, 71.9 with 3, 72.1 with 2)
-constexpr int VEC_BLOCKS = 3 * 152;
-constexpr int VEC_THREADS = 256;
+// One wave of CTAs of 1,024 threads, two per SM of a GB300 for FP32 vectors (32 registers a thread), one
+// for FP64 ones, fewer where n has fewer 4-wide chunks: every thread slot of the SMs in use holds loads
+// in flight, and a reduction pays one ticket and one partial per CTA.
+constexpr int VEC_THREADS = 1024;
+template <class T> constexpr int VEC_PER_SM = sizeof(T) == 4 ? 2 : 1;
+template <class T> inline int vec_blocks(int64_t n) {
+    const int64_t b = (n / 4 + VEC_THREADS - 1) / VEC_THREADS, most = 152 * VEC_PER_SM<T>;
+    return (int)(b < 1 ? 1 : (b < most ? b : most));
+}
 
 __device__ __forceinline__ void ld4(const float* p, float (&a)[4]) {
     const float4 v = *reinterpret_cast<const float4*>(p);
@@ -32,17 +37,50 @@ __device__ __forceinline__ void st4(double* p, const double (&a)[4]) {
 
 // Dot-product accumulator.  FP64 vectors accumulate in FP64.  FP32 vectors accumulate the
 // exact products (a*b = p + e, e by FMA) in an unevaluated FP32 pair (hi + lo, Knuth's
-// TwoSum), about 44 significant bits, then hand a double to the cross-thread reduction:
-// FP64-class dot products of FP32 vectors without FP64 arithmetic per element (GB300's FP64
-// and FP32<->FP64 conversion rates are a small fraction of its FP32 rate).
+// TwoSum), about 44 significant bits, and are summed as pairs over threads and CTAs (reduce.cuh):
+// FP64-class dot products of FP32 vectors without FP64 arithmetic before the total (an FP64
+// instruction holds an SM's FP64 pipe for 16 clocks per warp and its result comes late: with FP64 sums
+// of the warps, the CTA and the CTAs' partials a reduction's tail took 5 us of every launch).
 template <class T> struct DotAcc;
 template <> struct DotAcc<double> {
+    using Part = double;   // what crosses warps and CTAs
     double s = 0.0;
     __device__ __forceinline__ void add(double a, double b) { s = fma(a, b, s); }
+    __device__ __forceinline__ Part part() const { return s; }
+    __device__ __forceinline__ void merge(Part p) { s += p; }
     __device__ __forceinline__ double value() const { return s; }
+    __device__ __forceinline__ void warp_sum() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    }
 };
 template <> struct DotAcc<float> {
+    using Part = float2;
     float hi = 0.f, lo = 0.f;
+    __device__ __forceinline__ Part part() const { return make_float2(hi, lo); }
+    __device__ __forceinline__ void merge(Part p) { add_pair(p.x, p.y); }
+    // (hi, lo) += (h, l): the accurate double-float addition (relative error 3 x 2^-48)
+    __device__ __forceinline__ void add_pair(float h, float l) {
+        float s, e, t, f;
+        two_sum(hi, h, s, e);
+        two_sum(lo, l, t, f);
+        e = __fadd_rn(e, t);
+        fast_two_sum(s, e, hi, e);
+        e = __fadd_rn(e, f);
+        fast_two_sum(hi, e, s, lo);
+        hi = s;
+    }
+    __device__ __forceinline__ void warp_sum() {
+        float s, e;
+        two_sum(hi, lo, s, e);   // a proper pair first
+        hi = s;
+        lo = e;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float h = __shfl_down_sync(0xffffffffu, hi, o), l = __shfl_down_sync(0xffffffffu, lo, o);
+            add_pair(h, l);
+        }
+    }
     __device__ __forceinline__ void add(float a, float b) {
         const float p = __fmul_rn(a, b);
         const float e = __fmaf_rn(a, b, -p);
