@@ -14,8 +14,9 @@
 //   k_apply_walk   the same arithmetic fed by TMA, one wave of CTAs each walking up a strip
 //                  (variant 8; the autotuner's usual choice);
 //   k_apply_uni64  FP64: persistent tiles with a TMA pipeline, node-line form, one contraction per
-//                  line where the elements have one rigidity (the FP64 default, variant 3);
-//   k_apply_pipe   FP32 variant 3: the same tiles and pipeline with both contractions of a line;
+//                  line where the elements have one rigidity (the FP64 default);
+//   k_apply_pipe   the same pipeline with both contractions of every line (variant 3, and the K d
+//                  refresh of the mixed method's dynamic steps);
 //                  k_apply_tma / k_apply_lines: one tile per CTA (1, 2);
 //   k_apply        the strip modes 2 and 3 (first element row only).
 // The FP32 element kernels take an epilogue (epi.cuh) that finishes the V-cycle's residual or
@@ -1311,7 +1312,9 @@ void classify_elements(Handle& h) {
 }
 
 // CTAs of the pipelined apply: as many as fit on every SM at once.
-static int g_pipe_blocks = 0;
+static int g_pipe_blocks[2] = {0, 0};
+template <class T>
+static int pipe_blocks() { return g_pipe_blocks[sizeof(T) == 8 ? 1 : 0]; }
 
 template <class K>
 static int resident_blocks(K kernel, int threads, int bytes) {
@@ -1447,7 +1450,8 @@ bool set_H(const double* H, cudaStream_t s) {
                                   (int)apply_smem<double>()));
     EQC_CUDA(cudaFuncSetAttribute(k_apply<float, TEX, TEY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)apply_smem<float>()));
-    g_pipe_blocks = resident_blocks(k_apply_pipe<float, LTEX, LTEY, LNT>, LNT, PipeLayout<float, LTEX, LTEY>::BYTES);
+    g_pipe_blocks[0] = resident_blocks(k_apply_pipe<float, LTEX, LTEY, LNT>, LNT, PipeLayout<float, LTEX, LTEY>::BYTES);
+    g_pipe_blocks[1] = resident_blocks(k_apply_pipe<double, LTEX, LTEY, LNT>, LNT, PipeLayout<double, LTEX, LTEY>::BYTES);
     uni_setup();
     g_walk_slots = resident_blocks(k_apply_walk, 32 * WK_ROWS, WK_BYTES);
     return uni;
@@ -1488,7 +1492,7 @@ void apply_K(const T* x, T* y, const ApplyArgs<T>& A, T sign, int mode, cudaStre
             }
         }
         if constexpr (sizeof(T) == 8) {
-            const CUtensorMap* uu = (A.tma && A.variant != 1 && A.variant != 2) ? tma_umap_uni(*A.tma, x, A.L) : nullptr;
+            const CUtensorMap* uu = (A.tma && (A.variant == 0 || A.variant > 3)) ? tma_umap_uni(*A.tma, x, A.L) : nullptr;
             if (uu) {
                 launch_uni64(*uu, y, A, sign, mode == 1 ? 1 : 0, s);
                 return;
@@ -1497,11 +1501,10 @@ void apply_K(const T* x, T* y, const ApplyArgs<T>& A, T sign, int mode, cudaStre
         const CUtensorMap* um = (A.tma && A.variant != 2) ? tma_umap<T>(*A.tma, x, A.L) : nullptr;
         if (um && A.variant == 1) {
             k_apply_tma<T, LTEX, LTEY, LNT><<<grid, LNT, 0, s>>>(*um, tma_wmap<T>(*A.tma), y, A, sign, mode == 1 ? 1 : 0);
-        } else if (um && sizeof(T) == 4) {
+        } else if (um) {
             const int ntx = (int)grid.x, ntiles = (int)(grid.x * grid.y);
-            if constexpr (sizeof(T) == 4)
-                k_apply_pipe<T, LTEX, LTEY, LNT><<<std::min(ntiles, g_pipe_blocks), LNT, PipeLayout<T, LTEX, LTEY>::BYTES,
-                                                   s>>>(*um, tma_wmap<T>(*A.tma), y, A, sign, mode == 1 ? 1 : 0, ntx, ntiles);
+            k_apply_pipe<T, LTEX, LTEY, LNT><<<std::min(ntiles, pipe_blocks<T>()), LNT, PipeLayout<T, LTEX, LTEY>::BYTES, s>>>(
+                *um, tma_wmap<T>(*A.tma), y, A, sign, mode == 1 ? 1 : 0, ntx, ntiles);
         } else {
             k_apply_lines<T, LTEX, LTEY, LNT><<<grid, LNT, 0, s>>>(x, y, A, sign, mode == 1 ? 1 : 0);
         }
@@ -1537,7 +1540,7 @@ bool apply_K_epi(const float* x, const ApplyArgs<float>& A, int mode, const OpEp
 }
 
 bool apply_K_epi(const double* x, const ApplyArgs<double>& A, int mode, const OpEpi<double>& E, cudaStream_t s) {
-    if (mode > 1 || !A.tma || A.variant == 1 || A.variant == 2) return false;
+    if (mode > 1 || !A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
     const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
     if (!uu) return false;
     launch_uni64(*uu, nullptr, A, 1.0, mode, s, E);

@@ -928,6 +928,10 @@ static void enqueue_dyn_mixed_fused(Handle& h) {
     if (h.capturing) h.pdl_off = true;
     const int64_t n = h.L.size();
     const int* full = &h.ctrl.p->kd_full;
+    // K d is refreshed with both contractions of every line, as the increments' FP32 apply takes them: one
+    // launch in KD_REFRESH steps, and the accumulated K d keeps one rounding of K throughout
+    ApplyArgs<double> refresh = args64(h);
+    if (refresh.variant == 0 || refresh.variant > 3) refresh.variant = 3;
     auto gated = [&](auto A, int val) {
         A.gate = full;
         A.gate_val = val;
@@ -957,7 +961,7 @@ static void enqueue_dyn_mixed_fused(Handle& h) {
     EQC_CHECK_LAUNCH();
     EQC_CUDA(cudaEventRecord(h.ev_fork2, s));
     EQC_CUDA(cudaStreamWaitEvent(h.side_stream2, h.ev_fork2, 0));
-    apply_K<double>(h.d.p, h.Kd.p, gated(args64(h), 1), 1.0, 0, h.side_stream2);
+    apply_K<double>(h.d.p, h.Kd.p, gated(refresh, 1), 1.0, 0, h.side_stream2);
     EQC_CUDA(cudaEventRecord(h.ev_join2, h.side_stream2));
     apply_K<float>(h.g32.p, h.q32.p, gated(args32(h), 0), 1.0f, 0, s);
     EQC_CUDA(cudaStreamWaitEvent(s, h.ev_join2, 0));
@@ -978,6 +982,8 @@ static void enqueue_dyn(Handle& h, bool graph) {
     }
     if (h.opt.precision == EQC_MIXED) {
         // FP64 accumulation of d and of K d, FP32 apply of the step's increment
+        ApplyArgs<double> refresh = args64(h);   // as in enqueue_dyn_mixed_fused
+        if (refresh.variant == 0 || refresh.variant > 3) refresh.variant = 3;
         if (graph) {
             const cudaGraphConditionalHandle hf = cond_handle(h), hi = cond_handle(h);
             k_dyn_predict_inc<<<vblocks4(n), 256, 0, s>>>(h.d.p, h.v.p, h.a.p, h.F.vPre.p, h.g32.p, h.F.Nf, n,
@@ -985,7 +991,7 @@ static void enqueue_dyn(Handle& h, bool graph) {
             count_launch();
             const int64_t t0 = capture_tally();
             cond_begin(h, cudaGraphCondTypeIf, hf);
-            apply_K<double>(h.d.p, h.Kd.p, args64(h), 1.0, 0, h.stream);
+            apply_K<double>(h.d.p, h.Kd.p, refresh, 1.0, 0, h.stream);
             cond_end(h);
             const int64_t t1 = capture_tally();
             cond_begin(h, cudaGraphCondTypeIf, hi);
@@ -1002,7 +1008,7 @@ static void enqueue_dyn(Handle& h, bool graph) {
             int full = 0;
             EQC_CUDA(cudaMemcpyAsync(&full, &h.ctrl.p->kd_full, sizeof(int), cudaMemcpyDeviceToHost, s));
             EQC_CUDA(cudaStreamSynchronize(s));
-            if (full) apply_K<double>(h.d.p, h.Kd.p, args64(h), 1.0, 0, s);
+            if (full) apply_K<double>(h.d.p, h.Kd.p, refresh, 1.0, 0, s);
             else apply_K<float>(h.g32.p, h.q32.p, args32(h), 1.0f, 0, s);
         }
         k_dyn_force<<<vblocks4(n), 256, 0, s>>>(h.Kd.p, h.q32.p, h.a.p, n, h.ctrl.p);
