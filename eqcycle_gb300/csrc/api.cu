@@ -340,6 +340,8 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
     F.NFBC0 = nfbc;
     h.creep_prefix = true;
     for (auto g : lCreep) h.creep_prefix = h.creep_prefix && g < nfbc;
+    h.fault_count.alloc(1);
+    h.fault_part.alloc(3 * (size_t)((Nf + 31) / 32));
     {   // the mixed method's four-kernel dynamic step needs iBcL on column ix = 0 and iBcT on row
         // iy = ny - 1, each node listed once (the reference's BoundaryMatrix edges x = -LX, y = LY)
         std::vector<double> cL(L.ny, 0.0), cT(L.nx, 0.0);
@@ -359,8 +361,6 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
         if (h.nm_fused) {
             h.edgeL0has = hL[0];
             h.edgeL0 = cL[0];
-            h.fault_count.alloc(1);
-            h.fault_part.alloc(3 * (size_t)((Nf + 31) / 32));
             up_d(h.edgeL, cL.data(), L.ny);
             up_d(h.edgeT, cT.data(), L.nx);
             h.edgeLhas.alloc(L.ny);

@@ -140,7 +140,7 @@ struct Handle {
     bool nm_fused = false;       // the lists lie on those edges, once each, and creep_prefix
     int edgeL0has = 0;           // the fault's bottom node (0, 0) is in iBcL, with coefficient
     double edgeL0 = 0.0;
-    DBuf<unsigned> fault_count;  // CTAs of k_dyn_fault_nm done (its last one runs the control)
+    DBuf<unsigned> fault_count;  // CTAs of the control's launch done (the last one takes the decision)
     DBuf<double> fault_part;     // their partial reductions (three doubles' room each)
     // the fault row of that step runs on a second stream beside the other rows, the FP64
     // recomputation of K d (refresh steps) on a third beside the FP32 apply of the increment

@@ -366,14 +366,24 @@ __global__ void __launch_bounds__(FNT) k_dyn_fault(double* __restrict__ a, const
     }
 }
 
-// a = a / M ; v += dt/2 a   (main.jl:336-339).  inv: M holds 1/M (mixed method: a multiply
-// instead of GB300's slow FP64 division; the plain method divides as the reference does).
-__global__ void k_dyn_correct(double* __restrict__ a, double* __restrict__ v, const double* __restrict__ M, int64_t n,
-                              const Ctrl* C, int inv) {
+// a / m from inv = 1 / m rounded: the quotient a inv and one correction by its exact remainder, which gives
+// the correctly rounded a / m (Markstein, IBM J. Res. Dev. 34, 1990) with three FP64 operations where
+// the division takes a dozen.  Where the quotient or the remainder could leave the normal numbers, or an
+// operand is not finite, the division itself.  (5e8 random pairs: every bit the division's.)
+__device__ __forceinline__ double div_by(double a, double m, double inv) {
+    const int e = (__double2hiint(a) >> 20) & 0x7ff, em = (__double2hiint(m) >> 20) & 0x7ff;
+    const double q = __dmul_rn(a, inv);
+    if (e >= 300 && e <= 1700 && em >= 824 && em <= 1224) return __fma_rn(__fma_rn(-q, m, a), inv, q);
+    return ((__double2hiint(a) << 1) | __double2loint(a)) == 0 && em - 1u < 0x7feu ? q : a / m;
+}
+
+// a = a / M ; v += dt/2 a   (main.jl:336-339), the plain method's rounding of the division
+__global__ void k_dyn_correct(double* __restrict__ a, double* __restrict__ v, const double* __restrict__ M,
+                              const double* __restrict__ invM, int64_t n, const Ctrl* C) {
     EQC_GRID_WAIT();
     const double hdt = C->half_dt;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double ai = inv ? a[i] * M[i] : a[i] / M[i];
+        const double ai = div_by(a[i], M[i], invM[i]);
         a[i] = ai;
         v[i] = v[i] + hdt * ai;
     }
@@ -463,21 +473,46 @@ __device__ __forceinline__ void ctl_finish(const CtlAcc& c, Ctrl* C) {
     }
 }
 
-// One CTA (up to 1024 threads) over the fault row.
-__global__ void __launch_bounds__(FT) k_control(const double* __restrict__ v, FaultArgs f, Ctrl* C) {
+// The last CTA of a launch of one-warp CTAs to arrive (counted in *count, which it clears again) combines
+// the per-CTA partials and takes the decision.
+__device__ __forceinline__ void ctl_last(CtlAcc acc, CtlAcc* part, unsigned* count, Ctrl* C) {
+    __shared__ bool last;
+    acc = ctl_warp(acc);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = acc;
+        __threadfence();
+        last = atomicAdd(count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    CtlAcc c = ctl_init();
+    for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
+        CtlAcc o;
+        o.vmax = __ldcg(&part[q].vmax);
+        o.imax = __ldcg(&part[q].imax);
+        o.nan = __ldcg(&part[q].nan);
+        o.dmin = __ldcg(&part[q].dmin);
+        ctl_merge(c, o);
+    }
+    c = ctl_warp(c);
+    if (threadIdx.x == 0) {
+        ctl_finish(c, C);
+        *count = 0u;
+    }
+}
+
+// The control over the fault row, one warp per CTA: a node's division and comparisons are FP64, and each
+// such instruction of a warp holds its SM's FP64 pipe for 16 clocks (one CTA of 32 warps: 12 us for 245
+// nodes, 16 for 961; here 4).
+__global__ void __launch_bounds__(FNT) k_control(const double* __restrict__ v, FaultArgs f, Ctrl* C, CtlAcc* part,
+                                                 unsigned* count) {
     EQC_GRID_WAIT();
-    __shared__ CtlAcc sh[32];
     const double Vpl = C->Vpl;
     CtlAcc c = ctl_init();
-    for (int k = threadIdx.x; k < f.Nf; k += blockDim.x) ctl_add(c, k, v[k], f.XiLf[k], f.NFBC0, Vpl);
-    c = ctl_warp(c);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        CtlAcc t = sh[0];
-        for (int q = 1; q < (int)(blockDim.x >> 5); ++q) ctl_merge(t, sh[q]);
-        ctl_finish(t, C);
-    }
+    for (int k = threadIdx.x + blockIdx.x * blockDim.x; k < f.Nf; k += blockDim.x * gridDim.x)
+        ctl_add(c, k, v[k], f.XiLf[k], f.NFBC0, Vpl);
+    ctl_last(c, part, count, C);
 }
 
 // The fault row of the mixed method's dynamic step, from a = -(K d)[iFlt] (t0, the FP64 strip
@@ -495,7 +530,6 @@ __global__ void __launch_bounds__(FNT) k_dyn_fault_nm(double* __restrict__ a, do
                                                       const double* __restrict__ invM, int hasL0, double cL0,
                                                       CtlAcc* part, unsigned* count) {
     EQC_GRID_WAIT();
-    __shared__ bool last;
     const double dt = C->dt_step, hdt = C->half_dt, Vpl = C->Vpl;
     const int full = C->kd_full;
     CtlAcc acc = ctl_init();
@@ -560,29 +594,7 @@ __global__ void __launch_bounds__(FNT) k_dyn_fault_nm(double* __restrict__ a, do
         v[k] = vk;
         ctl_add(acc, k, vk, xilf, f.NFBC0, Vpl);
     }
-    acc = ctl_warp(acc);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = acc;
-        __threadfence();
-        last = atomicAdd(count, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    CtlAcc c = ctl_init();
-    for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
-        CtlAcc o;
-        o.vmax = __ldcg(&part[q].vmax);
-        o.imax = __ldcg(&part[q].imax);
-        o.nan = __ldcg(&part[q].nan);
-        o.dmin = __ldcg(&part[q].dmin);
-        ctl_merge(c, o);
-    }
-    c = ctl_warp(c);
-    if (threadIdx.x == 0) {
-        ctl_finish(c, C);
-        *count = 0u;
-    }
+    ctl_last(acc, part, count, C);
 }
 
 // Gather d, v, a at receivers (main.jl:433-435) into out[3*ns] (v and a of the step's end where
@@ -1029,7 +1041,7 @@ static void enqueue_dyn(Handle& h, bool graph) {
     const bool zero_fused = mixed && h.creep_prefix;
     if (mixed) k_dyn_correct_inv<<<vblocks4(n), 256, 0, s>>>(h.a.p, h.v.p, h.invM.p, n, h.ctrl.p,
                                                             zero_fused ? (int64_t)h.F.NFBC0 : 0);
-    else k_dyn_correct<<<vblocks(n), 256, 0, s>>>(h.a.p, h.v.p, h.M.p, n, h.ctrl.p, 0);
+    else k_dyn_correct<<<vblocks(n), 256, 0, s>>>(h.a.p, h.v.p, h.M.p, h.invM.p, n, h.ctrl.p);
     count_launch(3);
     if (h.nCreep && !zero_fused) {
         k_zero_list<<<1, 256, 0, s>>>(h.iCreep.p, h.nCreep, h.v.p, h.a.p, nullptr);
@@ -1059,7 +1071,8 @@ void enqueue_step(Handle& h, int iso, bool graph) {
     if (iso == 1) enqueue_qs(h, graph);
     else enqueue_dyn(h, graph);
     if (!fused) {
-        k_control<<<1, FT, 0, h.stream>>>(h.v.p, fargs(h, h.bcflag.p), h.ctrl.p);
+        k_control<<<fblocks(h.F.Nf), FNT, 0, h.stream>>>(h.v.p, fargs(h, h.bcflag.p), h.ctrl.p,
+                                                          reinterpret_cast<CtlAcc*>(h.fault_part.p), h.fault_count.p);
         launch_check();
         count_launch();
     }
