@@ -20,6 +20,7 @@ Handle::~Handle() {
     if (h_ctrl) cudaFreeHost(h_ctrl);
     if (h_scal) cudaFreeHost(h_scal);
     if (h_cg) cudaFreeHost(h_cg);
+    if (F.h_io) cudaFreeHost(F.h_io);
     for (cudaStream_t c : cap_streams)
         if (c) cudaStreamDestroy(c);
     for (cudaStream_t c : {side_stream, side_stream2})
@@ -371,9 +372,17 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
         }
     }
     for (DBuf<double>* b : {&F.fo, &F.Vo, &F.xLf, &F.cca, &F.ccb, &F.Seff, &F.tauo, &F.XiLf, &F.FltB, &F.FltZ, &F.FltX,
-                            &F.Mf, &F.psi, &F.psi1, &F.psi2, &F.tau, &F.tau1, &F.tau2, &F.Vf, &F.Vf0, &F.Vf1, &F.Vf2,
-                            &F.FltVfree, &F.vPre, &F.Flast})
+                            &F.Mf, &F.tau, &F.Vf0, &F.vPre, &F.Flast})
         b->alloc(Nf);
+    F.io.alloc((size_t)IO_ARRAYS * Nf + 1);
+    EQC_CUDA(cudaMallocHost(&F.h_io, sizeof(double) * (IO_ARRAYS * (size_t)Nf + 1)));
+    {
+        double* p = F.io.p;
+        for (DBuf<double>* b : {&F.psi, &F.Vf, &F.FltVfree, &F.psi1, &F.Vf1, &F.tau1, &F.psi2, &F.Vf2, &F.tau2}) {
+            b->view(p, Nf);
+            p += Nf;
+        }
+    }
     F.fo.upload(m.fo, Nf, s);
     F.Vo.upload(m.Vo, Nf, s);
     F.xLf.upload(m.xLf, Nf, s);
@@ -430,27 +439,7 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
     h.setup_ms[4] = ms_since(t0);   // multigrid hierarchy (host Galerkin products, device bounds)
 }
 
-// Reference numbering <-> node layout on the host's cores: ref2lay is one-to-one, so the
-// chunks write disjoint entries (the layout's row padding stays zero).
-static void to_layout(const Handle& h, const double* ref, std::vector<double>& lay) {
-    constexpr int64_t CH = 1 << 14;   // nodes per work item
-    const int64_t N = h.L.size();
-    lay.resize(N);
-    parallel_for((N + CH - 1) / CH, [&](int64_t c) {
-        std::fill(lay.begin() + c * CH, lay.begin() + std::min(N, (c + 1) * CH), 0.0);
-    }, 1);
-    parallel_for((h.nglob + CH - 1) / CH, [&](int64_t c) {
-        for (int64_t g = c * CH; g < std::min(h.nglob, (c + 1) * CH); ++g) lay[h.ref2lay[g]] = ref[g];
-    }, 1);
-}
-static void from_layout(const Handle& h, const std::vector<double>& lay, double* ref) {
-    constexpr int64_t CH = 1 << 14;
-    parallel_for((h.nglob + CH - 1) / CH, [&](int64_t c) {
-        for (int64_t g = c * CH; g < std::min(h.nglob, (c + 1) * CH); ++g) ref[g] = lay[h.ref2lay[g]];
-    }, 1);
-}
-
-// The same maps on the device, for the state transfers of eqc_get_state / eqc_set_state: the
+// Reference numbering <-> node layout on the device, for every entry point that takes host fields: the
 // field crosses PCIe / C2C in the reference numbering and is permuted by a kernel (the padding
 // entries of the layout are zero).
 __global__ void k_ref_to_layout(const double* __restrict__ ref, const int* __restrict__ map, int64_t n,
@@ -474,6 +463,20 @@ static void ensure_ref_maps(Handle& h) {
     EQC_CUDA(cudaStreamSynchronize(h.stream));
 }
 static int ref_blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 8 * 152); }
+static void to_layout(Handle& h, const double* ref, double* lay) {
+    ensure_ref_maps(h);
+    h.ref_stage.upload(ref, h.nglob, h.stream);
+    k_ref_to_layout<<<ref_blocks(h.nglob), 256, 0, h.stream>>>(h.ref_stage.p, h.d_ref2lay.p, h.nglob, lay);
+    EQC_CHECK_LAUNCH();
+    count_launch();
+}
+static void from_layout(Handle& h, const double* lay, double* ref) {
+    ensure_ref_maps(h);
+    k_layout_to_ref<<<ref_blocks(h.nglob), 256, 0, h.stream>>>(lay, h.d_ref2lay.p, h.nglob, h.ref_stage.p);
+    EQC_CHECK_LAUNCH();
+    count_launch();
+    h.ref_stage.download(ref, h.nglob, h.stream);
+}
 
 static thread_local std::string g_create_err;
 void set_thread_error(const std::string& msg) { g_create_err = msg; }
@@ -568,14 +571,11 @@ eqc_status eqc_apply_K(eqc_handle* H, const double* x, double* y) {
     if (!H || !x || !y) return EQC_E_ARG;
     return guarded(H, [&] {
         Handle& h = H->h;
-        std::vector<double> xl, yl(h.L.size());
-        to_layout(h, x, xl);
-        h.tmp64a.upload(xl.data(), xl.size(), h.stream);
+        to_layout(h, x, h.tmp64a.p);
         apply_K<double>(h.tmp64a.p, h.tmp64b.p, args64(h), 1.0, 0, h.stream);
-        h.tmp64b.download(yl.data(), yl.size(), h.stream);
-        EQC_CUDA(cudaStreamSynchronize(h.stream));
         check_apply_err(h);
-        from_layout(h, yl, y);
+        from_layout(h, h.tmp64b.p, y);
+        EQC_CUDA(cudaStreamSynchronize(h.stream));
     });
 }
 
@@ -587,16 +587,13 @@ eqc_status eqc_qs_solve(eqc_handle* H, const double* F_fault, double* d_inout, d
         const int64_t N = h.L.size();
         // keep the time-loop displacement intact
         EQC_CUDA(cudaMemcpyAsync(h.dPre.p, h.d.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, h.stream));
-        std::vector<double> dl;
-        to_layout(h, d_inout, dl);
-        for (int k = 0; k < h.F.Nf; ++k) dl[k] = F_fault[k];
-        h.d.upload(dl.data(), N, h.stream);
+        to_layout(h, d_inout, h.d.p);
+        h.d.upload(F_fault, h.F.Nf, h.stream);
         double rr = 0;
         int it = qs_solve_device(h, tol, maxit, &rr);
-        h.d.download(dl.data(), N, h.stream);
+        from_layout(h, h.d.p, d_inout);
         EQC_CUDA(cudaMemcpyAsync(h.d.p, h.dPre.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, h.stream));
         EQC_CUDA(cudaStreamSynchronize(h.stream));
-        from_layout(h, dl, d_inout);
         if (iters) *iters = it;
         if (relres) *relres = rr;
         if (it < 0) throw Error(EQC_E_CG, "CG reached maxit");
@@ -656,11 +653,7 @@ eqc_status eqc_get_state(eqc_handle* H, const char* name, double* out) {
         if (fault) {
             b->download(out, h.F.Nf, h.stream);
         } else {
-            ensure_ref_maps(h);
-            k_layout_to_ref<<<ref_blocks(h.nglob), 256, 0, h.stream>>>(b->p, h.d_ref2lay.p, h.nglob, h.ref_stage.p);
-            EQC_CHECK_LAUNCH();
-            count_launch();
-            h.ref_stage.download(out, h.nglob, h.stream);
+            from_layout(h, b->p, out);
         }
         EQC_CUDA(cudaStreamSynchronize(h.stream));
     });
@@ -677,12 +670,8 @@ eqc_status eqc_set_state(eqc_handle* H, const char* name, const double* in) {
         if (fault) {
             b->upload(in, h.F.Nf, h.stream);
         } else {
-            ensure_ref_maps(h);
-            h.ref_stage.upload(in, h.nglob, h.stream);
             b->zero(h.stream);
-            k_ref_to_layout<<<ref_blocks(h.nglob), 256, 0, h.stream>>>(h.ref_stage.p, h.d_ref2lay.p, h.nglob, b->p);
-            EQC_CHECK_LAUNCH();
-            count_launch();
+            to_layout(h, in, b->p);
         }
         invalidate_residual(h);
         EQC_CUDA(cudaStreamSynchronize(h.stream));

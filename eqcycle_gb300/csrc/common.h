@@ -43,12 +43,13 @@ template <class T>
 struct DBuf {
     T* p = nullptr;
     size_t n = 0;
+    bool own = true;   // false: a part of another buffer (view)
     DBuf() = default;
     DBuf(const DBuf&) = delete;
     DBuf& operator=(const DBuf&) = delete;
-    DBuf(DBuf&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+    DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), own(o.own) { o.p = nullptr; o.n = 0; }
     DBuf& operator=(DBuf&& o) noexcept {
-        if (this != &o) { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; }
+        if (this != &o) { release(); p = o.p; n = o.n; own = o.own; o.p = nullptr; o.n = 0; }
         return *this;
     }
     ~DBuf() { release(); }
@@ -67,9 +68,16 @@ struct DBuf {
         EQC_CUDA(cudaDeviceSynchronize());
     }
     void release() {
-        if (p) cudaFree(p);
+        if (p && own) cudaFree(p);
         p = nullptr;
         n = 0;
+        own = true;
+    }
+    void view(T* q, size_t count) {
+        release();
+        p = q;
+        n = count;
+        own = false;
     }
     void upload(const T* h, size_t count, cudaStream_t s) {
         if (count) EQC_CUDA(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, s));

@@ -12,9 +12,16 @@ struct FaultDev {
     int NFBC0 = 0;  // first friction node (0-based), NFBC - 1 of src/main.jl:186
     DBuf<double> fo, Vo, xLf, cca, ccb, Seff, tauo, XiLf, FltB, FltZ, FltX, Mf;
     DBuf<double> psi, psi1, psi2, tau, tau1, tau2, Vf, Vf0, Vf1, Vf2, FltVfree, vPre;
+    // the arrays of the fault entry points, one after the other in io (IO_PSI.. below, plus one slot), and
+    // page-locked staging memory of the same layout
+    DBuf<double> io;
+    double* h_io = nullptr;
     DBuf<double> Flast;   // fault displacement the carried CG residual belongs to
     DBuf<int> creep;   // 1 for fault nodes listed in iFBC (creeping), [Nf]
 };
+
+// Positions in FaultDev::io: psi, Vf, FltVfree, then the outputs psi1, Vf1, tau1, psi2, Vf2, tau2.
+constexpr int IO_PSI = 0, IO_PSI1 = 3, IO_ARRAYS = 9;
 
 // Device-side control block of the time loop.
 struct Ctrl {

@@ -15,6 +15,8 @@
 #include "vec.cuh"
 #include "df.cuh"
 #include <cmath>
+#include <cstring>
+#include <initializer_list>
 #include <algorithm>
 #include <chrono>
 
@@ -366,17 +368,6 @@ __global__ void __launch_bounds__(FNT) k_dyn_fault(double* __restrict__ a, const
     }
 }
 
-// a / m from inv = 1 / m rounded: the quotient a inv and one correction by its exact remainder, which gives
-// the correctly rounded a / m (Markstein, IBM J. Res. Dev. 34, 1990) with three FP64 operations where
-// the division takes a dozen.  Where the quotient or the remainder could leave the normal numbers, or an
-// operand is not finite, the division itself.  (5e8 random pairs: every bit the division's.)
-__device__ __forceinline__ double div_by(double a, double m, double inv) {
-    const int e = (__double2hiint(a) >> 20) & 0x7ff, em = (__double2hiint(m) >> 20) & 0x7ff;
-    const double q = __dmul_rn(a, inv);
-    if (e >= 300 && e <= 1700 && em >= 824 && em <= 1224) return __fma_rn(__fma_rn(-q, m, a), inv, q);
-    return ((__double2hiint(a) << 1) | __double2loint(a)) == 0 && em - 1u < 0x7feu ? q : a / m;
-}
-
 // a = a / M ; v += dt/2 a   (main.jl:336-339), the plain method's rounding of the division
 __global__ void k_dyn_correct(double* __restrict__ a, double* __restrict__ v, const double* __restrict__ M,
                               const double* __restrict__ invM, int64_t n, const Ctrl* C) {
@@ -665,70 +656,77 @@ __global__ void __launch_bounds__(FNT) k_api_fbc(FaultArgs f, double dt, int* fa
     EQC_GRID_WAIT();
     for (int k = threadIdx.x + blockIdx.x * blockDim.x; k < f.Nf; k += blockDim.x * gridDim.x) {
         if (k < f.NFBC0) continue;
-        const double vf = f.Vf[k], vfree = f.FltVfree[k];
-        const double p1 = dev_IDS(f.xLf[k], f.Vo[k], f.psi[k], dt, vf, 1e-5);
+        // every input before the first store (which may alias them for all the compiler knows)
+        const double vf = f.Vf[k], vfree = f.FltVfree[k], psi = f.psi[k];
+        const double fo = __ldg(f.fo + k), Vo = __ldg(f.Vo + k), cca = __ldg(f.cca + k), ccb = __ldg(f.ccb + k);
+        const double Seff = __ldg(f.Seff + k), tauo = __ldg(f.tauo + k), FltZ = __ldg(f.FltZ + k), xLf = __ldg(f.xLf + k);
+        const double p1 = dev_IDS(xLf, Vo, psi, dt, vf, 1e-5);
+        double V1, T1, V2, T2;
+        dev_NR(fo, Vo, cca, ccb, Seff, 0.0, tauo, p1, FltZ, vfree, &V1, &T1);
+        if (vf > 1e10 || isnan(vf) || isnan(T1)) atomicMin(fail, k + 1);
+        const double p2 = dev_IDS2(xLf, Vo, psi, p1, dt, vf, V1);
+        dev_NR(fo, Vo, cca, ccb, Seff, T1, tauo, p2, FltZ, vfree, &V2, &T2);
         f.psi1[k] = p1;
-        double V1, T1;
-        dev_NR(f.fo[k], f.Vo[k], f.cca[k], f.ccb[k], f.Seff[k], 0.0, f.tauo[k], p1, f.FltZ[k], vfree, &V1, &T1);
         f.Vf1[k] = V1;
         f.tau1[k] = T1;
-        if (vf > 1e10 || isnan(vf) || isnan(T1)) atomicMin(fail, k + 1);
-        const double p2 = dev_IDS2(f.xLf[k], f.Vo[k], f.psi[k], p1, dt, vf, V1);
         f.psi2[k] = p2;
-        double V2, T2;
-        dev_NR(f.fo[k], f.Vo[k], f.cca[k], f.ccb[k], f.Seff[k], T1, f.tauo[k], p2, f.FltZ[k], vfree, &V2, &T2);
         f.Vf2[k] = V2;
         f.tau2[k] = T2;
     }
 }
 
+// The fault entry points' host arrays cross in page-locked staging memory laid out as the fault arrays lie
+// on the device (FaultDev::io): one transfer in and one out per run of neighbouring arrays.
+static void io_in(Handle& h, int slot, std::initializer_list<const double*> arrays) {
+    const int Nf = h.F.Nf;
+    double* p = h.F.h_io + (size_t)slot * Nf;
+    for (const double* a : arrays) {
+        std::memcpy(p, a, sizeof(double) * Nf);
+        p += Nf;
+    }
+    EQC_CUDA(cudaMemcpyAsync(h.F.io.p + (size_t)slot * Nf, h.F.h_io + (size_t)slot * Nf, sizeof(double) * Nf * arrays.size(),
+                             cudaMemcpyHostToDevice, h.stream));
+}
+// after io_out_begin and a synchronisation, io_out hands out the arrays
+static void io_out_begin(Handle& h, int slot, size_t doubles) {
+    const size_t o = (size_t)slot * h.F.Nf;
+    EQC_CUDA(cudaMemcpyAsync(h.F.h_io + o, h.F.io.p + o, sizeof(double) * doubles, cudaMemcpyDeviceToHost, h.stream));
+    EQC_CUDA(cudaStreamSynchronize(h.stream));
+}
+static void io_out(Handle& h, int slot, std::initializer_list<double*> arrays) {
+    const int Nf = h.F.Nf;
+    const double* p = h.F.h_io + (size_t)slot * Nf;
+    for (double* a : arrays) {
+        std::memcpy(a, p, sizeof(double) * Nf);
+        p += Nf;
+    }
+}
+
 void fault_slrFunc(Handle& h, const double* psi, double* psi1, const double* Vf, double* Vf1, const double* tau1,
                    double dt) {
-    FaultDev& F = h.F;
-    const int Nf = F.Nf;
-    cudaStream_t s = h.stream;
-    F.psi.upload(psi, Nf, s);
-    F.Vf.upload(Vf, Nf, s);
-    F.tau1.upload(tau1, Nf, s);
-    F.psi1.upload(psi1, Nf, s);
-    F.Vf1.upload(Vf1, Nf, s);
-    k_api_slr<<<fblocks(h.F.Nf), FNT, 0, s>>>(fargs(h, h.bcflag.p), dt);
+    io_in(h, IO_PSI, {psi, Vf});
+    io_in(h, IO_PSI1, {psi1, Vf1, tau1});
+    k_api_slr<<<fblocks(h.F.Nf), FNT, 0, h.stream>>>(fargs(h, h.bcflag.p), dt);
     launch_check();
     count_launch();
-    F.psi1.download(psi1, Nf, s);
-    F.Vf1.download(Vf1, Nf, s);
-    EQC_CUDA(cudaStreamSynchronize(s));
+    io_out_begin(h, IO_PSI1, 2 * (size_t)h.F.Nf);
+    io_out(h, IO_PSI1, {psi1, Vf1});
 }
 
 int fault_FBC(Handle& h, double* psi1, double* Vf1, double* tau1, double* psi2, double* Vf2, double* tau2,
               const double* psi, const double* Vf, const double* FltVfree, double dt) {
-    FaultDev& F = h.F;
-    const int Nf = F.Nf;
-    cudaStream_t s = h.stream;
-    F.psi.upload(psi, Nf, s);
-    F.Vf.upload(Vf, Nf, s);
-    F.FltVfree.upload(FltVfree, Nf, s);
-    F.psi1.upload(psi1, Nf, s);
-    F.Vf1.upload(Vf1, Nf, s);
-    F.tau1.upload(tau1, Nf, s);
-    F.psi2.upload(psi2, Nf, s);
-    F.Vf2.upload(Vf2, Nf, s);
-    F.tau2.upload(tau2, Nf, s);
-    int big = 0x7fffffff;
-    EQC_CUDA(cudaMemcpyAsync(&h.ctrl.p->fail, &big, sizeof(int), cudaMemcpyHostToDevice, s));
-    k_api_fbc<<<fblocks(h.F.Nf), FNT, 0, s>>>(fargs(h, h.bcflag.p), dt, &h.ctrl.p->fail);
+    const size_t Nf = h.F.Nf;
+    int* fail = reinterpret_cast<int*>(h.F.h_io + IO_ARRAYS * Nf);   // one slot past the arrays
+    *fail = 0x7fffffff;
+    EQC_CUDA(cudaMemcpyAsync(h.F.io.p + IO_ARRAYS * Nf, fail, sizeof(int), cudaMemcpyHostToDevice, h.stream));
+    io_in(h, IO_PSI, {psi, Vf, FltVfree, psi1, Vf1, tau1, psi2, Vf2, tau2});
+    k_api_fbc<<<fblocks(h.F.Nf), FNT, 0, h.stream>>>(fargs(h, h.bcflag.p), dt,
+                                                     reinterpret_cast<int*>(h.F.io.p + IO_ARRAYS * Nf));
     launch_check();
     count_launch();
-    F.psi1.download(psi1, Nf, s);
-    F.Vf1.download(Vf1, Nf, s);
-    F.tau1.download(tau1, Nf, s);
-    F.psi2.download(psi2, Nf, s);
-    F.Vf2.download(Vf2, Nf, s);
-    F.tau2.download(tau2, Nf, s);
-    int fail = 0;
-    EQC_CUDA(cudaMemcpyAsync(&fail, &h.ctrl.p->fail, sizeof(int), cudaMemcpyDeviceToHost, s));
-    EQC_CUDA(cudaStreamSynchronize(s));
-    return fail == 0x7fffffff ? 0 : fail;
+    io_out_begin(h, IO_PSI1, 6 * Nf + 1);
+    io_out(h, IO_PSI1, {psi1, Vf1, tau1, psi2, Vf2, tau2});
+    return *fail == 0x7fffffff ? 0 : *fail;
 }
 
 __global__ void k_api_dtevol(const double* Vf, FaultArgs f, double dt, double dtmin, int isolver, double* out) {
