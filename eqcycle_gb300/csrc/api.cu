@@ -176,7 +176,7 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
     std::memcpy(h.H, m.H, sizeof(h.H));
     h.uni_ok = set_H(h.H, s);
     set_H_df(h.H, s);
-    set_H_sem(h.H, s);
+    h.sem_scale = set_H_sem(h.H, s);
     {   // the double-float apply uses the even-odd form: H must be centro-antisymmetric
         double hmax = 0.0, asym = 0.0;
         for (int k = 0; k < 25; ++k) hmax = std::max(hmax, std::fabs(h.H[k]));

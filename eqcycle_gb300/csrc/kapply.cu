@@ -586,9 +586,9 @@ static int mu_pitch(int NelX) { return (NelX + 3) & ~1; }
 
 // Tolerance 2^-49: W is a rounded product of weights and rigidity (and of damage factors), a few
 // units in the last place from the product formed here.
-// mu32: the rigidity rounded to FP32; *several counts the elements of several.
+// mu32: the rigidity over `unit` rounded to FP32; *several counts the elements of several.
 __global__ void k_classify(const double* __restrict__ W, double* __restrict__ mu, float* __restrict__ mu32, int* several,
-                           int NelX, int NelY, int pitch, int ok) {
+                           int NelX, int NelY, int pitch, double unit, int ok) {
     EQC_GRID_WAIT();
     const int64_t Nel = (int64_t)NelX * NelY;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < Nel; e += (int64_t)gridDim.x * blockDim.x) {
@@ -599,7 +599,7 @@ __global__ void k_classify(const double* __restrict__ W, double* __restrict__ mu
             for (int i = 0; i < 5; ++i)
                 uni = uni && fabs(w[i + 5 * j] - m * (cUni.w[i] * cUni.w[j])) <= 0x1p-49 * w[i + 5 * j];
         mu[(e / NelX) * pitch + e % NelX + 1] = uni ? m : -1.0;
-        mu32[e] = uni ? (float)m : -1.f;
+        mu32[e] = uni ? (float)(m / unit) : -1.f;
         if (!uni) atomicAdd(several, 1);
     }
 }
@@ -1301,7 +1301,7 @@ void classify_elements(Handle& h) {
     DBuf<int> several;
     several.alloc(1);
     k_classify<<<(int)std::min<int64_t>((Nel + 255) / 256, 4096), 256, 0, h.stream>>>(
-        h.W64.p, h.mu64.p, h.mu32.p, several.p, L.NelX, L.NelY, mp, h.uni_ok ? 1 : 0);
+        h.W64.p, h.mu64.p, h.mu32.p, several.p, L.NelX, L.NelY, mp, h.mu_unit, h.uni_ok ? 1 : 0);
     EQC_CHECK_LAUNCH();
     count_launch();
     int n = 0;
@@ -1320,6 +1320,13 @@ template <class K>
 static int resident_blocks(K kernel, int threads, int bytes) {
     EQC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     int per_sm = 0, dev = 0, nsm = 0;
+    if (h.mu_unit == 0.0) {
+        double w = 0.0;
+        EQC_CUDA(cudaMemcpyAsync(&w, h.W64.p + 25 * (Nel - 1) + 12, sizeof(w), cudaMemcpyDeviceToHost, h.stream));
+        EQC_CUDA(cudaStreamSynchronize(h.stream));
+        w /= (32.0 / 45.0) * (32.0 / 45.0);
+        h.mu_unit = w > 0.0 && std::isfinite(w) ? w : 1.0;
+    }
     EQC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes));
     EQC_CUDA(cudaGetDevice(&dev));
     EQC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));

@@ -159,7 +159,9 @@ struct Handle {
     // element data
     DBuf<double> W64, W64p;
     DBuf<double> mu64;   // rigidity per element, -1 where it varies within one (classify_elements)
-    DBuf<float> mu32;    // the same in FP32, without the shifted column
+    DBuf<float> mu32;    // the same in FP32 over mu_unit, without the shifted column
+    double mu_unit = 0.0;    // the far field's rigidity (exact in mu32) when the elements were first classified
+    double sem_scale = 1.0;  // set_H_sem
     bool sem_ok = false; // the FP32 operator of sem.cu pays (classify_elements)
     bool uni_ok = false; // H admits the one-contraction lines of the FP64 apply
     DBuf<float> W32, W32p;

@@ -16,11 +16,16 @@
 #include "vec.cuh"
 #include "cg.cuh"
 #include <algorithm>
+#include <cmath>
 
 namespace eqc {
 
+// rho: the row sums, which vanish but for the rounding of the two contractions' coefficients (1.6e-7).  They
+// stay in so that an element has one operator in either form, to 1e-8 on smooth fields (set_H_sem): CG stops
+// at the error that this operator's difference from the FP64 one leaves, 2e-9 of |d| on 480 x 960 elements
+// at a tolerance of 1e-10, and a second operator stops 1.5e-9 away from it.
 struct UniCoefF {
-    float a[2][2], b[2][2], d[2];
+    float a[2][2], b[2][2], d[2], rho[3];
 };
 struct EOCoefF {
     float a[2][2], b[2][2], g[2], d[2];
@@ -34,11 +39,11 @@ __device__ __forceinline__ void uni_line(const float (&v)[5], float (&s)[5]) {
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
         const float P = fmaf(cUniF.a[p][1], o1, cUniF.a[p][0] * o0);
-        const float Q = fmaf(cUniF.b[p][1], e1, cUniF.b[p][0] * e0);
+        const float Q = fmaf(cUniF.rho[p], v[2], fmaf(cUniF.b[p][1], e1, cUniF.b[p][0] * e0));
         s[p] = Q + P;
         s[4 - p] = Q - P;
     }
-    s[2] = fmaf(cUniF.d[1], e1, cUniF.d[0] * e0);
+    s[2] = fmaf(cUniF.rho[2], v[2], fmaf(cUniF.d[1], e1, cUniF.d[0] * e0));
 }
 __device__ __forceinline__ void eo_line(const float (&v)[5], float (&s)[5], const EOCoefF& c) {
     const float e0 = v[0] + v[4], e1 = v[1] + v[3], o0 = v[0] - v[4], o1 = v[1] - v[3];
@@ -56,7 +61,7 @@ __device__ __forceinline__ void eo_line(const float (&v)[5], float (&s)[5], cons
 struct SemGeom {
     Layout L;
     const float *mu, *Wp;
-    float cx[3], cy[3];   // c1 w_j, c2 w_i
+    float cx[3], cy[3];   // c1 w_j, c2 w_i, times the unit of mu and the scale of the coefficients
     float c1, c2;
     int rows, ldc;
 };
@@ -350,6 +355,16 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_sem(SemGeom G, SemOp
     }
 }
 
+// c w_j in FP32, each remainder carried into the next smaller one: 2 + 2 + 1 of them sum to 2 c within 4e-9,
+// where each rounded by itself would scale the operator by up to 3e-8.
+static void line_weights(double c, float* out) {
+    const double w[3] = {0.1 * c, 49.0 / 90.0 * c, 32.0 / 45.0 * c};
+    out[2] = (float)w[2];
+    const double t = w[1] + 0.5 * (w[2] - out[2]);
+    out[1] = (float)t;
+    out[0] = (float)(w[0] + (t - out[1]));
+}
+
 bool sem_usable(const Handle& h) { return h.sem_ok && h.opt.apply_variant == 0; }
 
 void sem_launch(Handle& h, SemLoad load, SemEpi epi, SemPrev prev, const SemOp& o) {
@@ -360,11 +375,8 @@ void sem_launch(Handle& h, SemLoad load, SemEpi epi, SemPrev prev, const SemOp& 
     G.Wp = h.W32p.p;
     G.c1 = (float)h.c1;
     G.c2 = (float)h.c2;
-    const double gw[3] = {0.1, 49.0 / 90.0, 32.0 / 45.0};
-    for (int k = 0; k < 3; ++k) {
-        G.cx[k] = (float)(h.c1 * gw[k]);
-        G.cy[k] = (float)(h.c2 * gw[k]);
-    }
+    line_weights(h.c1 * h.mu_unit * h.sem_scale, G.cx);
+    line_weights(h.c2 * h.mu_unit * h.sem_scale, G.cy);
     G.ldc = L.NelX + 1;
     const int nsx = (L.NelX + 1 + 30) / 31;
     // rows per warp: the fewest with which every warp is resident at once (16 on each of 152 SMs)
@@ -388,36 +400,53 @@ void sem_launch(Handle& h, SemLoad load, SemEpi epi, SemPrev prev, const SemOp& 
     count_launch();
 }
 
-void set_H_sem(const double* H, cudaStream_t s) {
+// S = D2 diag(w) D1 with D1 and D2 the two contractions as their FP32 coefficients have them.  Its entries
+// are rounded once more; the scale that gives a linear field's energy back goes into the lines' weights.
+double set_H_sem(const double* H, cudaStream_t s) {
     const double gw[5] = {0.1, 49.0 / 90.0, 32.0 / 45.0, 49.0 / 90.0, 0.1};
-    auto S = [&](int i, int k) {
-        long double t = 0.0L;
-        for (int p = 0; p < 5; ++p) t += (long double)H[i + 5 * p] * gw[p] * H[k + 5 * p];
-        return (double)t;
-    };
-    UniCoefF u;
     EOCoefF c[2];
-    for (int p = 0; p < 2; ++p) {
-        for (int m = 0; m < 2; ++m) {
-            u.a[p][m] = (float)(0.5 * (S(p, m) - S(p, 4 - m)));
-            u.b[p][m] = (float)(0.5 * (S(p, m) + S(p, 4 - m)));
-        }
-        u.d[p] = (float)S(2, p);
-    }
+    double D[2][5][5];
     for (int t = 0; t < 2; ++t) {
         auto M = [&](int r, int q) { return t == 0 ? H[q + 5 * r] : H[r + 5 * q]; };
         for (int p = 0; p < 2; ++p) {
             for (int m = 0; m < 2; ++m) {
-                c[t].a[p][m] = (float)(0.5 * (M(p, m) - M(p, 4 - m)));
-                c[t].b[p][m] = (float)(0.5 * (M(p, m) + M(p, 4 - m)));
+                const double a = c[t].a[p][m] = (float)(0.5 * (M(p, m) - M(p, 4 - m)));
+                const double b = c[t].b[p][m] = (float)(0.5 * (M(p, m) + M(p, 4 - m)));
+                D[t][p][m] = a + b;
+                D[t][p][4 - m] = b - a;
+                D[t][4 - p][m] = a - b;
+                D[t][4 - p][4 - m] = -a - b;
             }
-            c[t].g[p] = (float)M(p, 2);
-            c[t].d[p] = (float)M(2, p);
+            D[t][p][2] = c[t].g[p] = (float)M(p, 2);
+            D[t][4 - p][2] = -D[t][p][2];
+            D[t][2][p] = c[t].d[p] = (float)M(2, p);
+            D[t][2][4 - p] = -D[t][2][p];
         }
+        D[t][2][2] = 0.0;
     }
+    auto S = [&](int i, int k) {
+        long double t = 0.0L;
+        for (int p = 0; p < 5; ++p) t += (long double)D[1][i][p] * gw[p] * D[0][p][k];
+        return t;
+    };
+    UniCoefF u;
+    const double xi[2] = {1.0, std::sqrt(3.0 / 7.0)};
+    double exact = 0.0, rounded = 0.0;
+    for (int p = 0; p < 2; ++p) {
+        for (int m = 0; m < 2; ++m) {
+            const double a = (double)(0.5L * (S(p, m) - S(p, 4 - m)));
+            u.a[p][m] = (float)a;
+            u.b[p][m] = (float)(0.5L * (S(p, m) + S(p, 4 - m)));
+            exact += xi[p] * xi[m] * a;
+            rounded += xi[p] * xi[m] * u.a[p][m];
+        }
+        u.d[p] = (float)S(2, p);
+    }
+    for (int p = 0; p < 3; ++p) u.rho[p] = (float)(S(p, 0) + S(p, 1) + S(p, 2) + S(p, 3) + S(p, 4));
     EQC_CUDA(cudaMemcpyToSymbolAsync(cUniF, &u, sizeof(u), 0, cudaMemcpyHostToDevice, s));
     EQC_CUDA(cudaMemcpyToSymbolAsync(cEOF, c, sizeof(c), 0, cudaMemcpyHostToDevice, s));
     EQC_CUDA(cudaStreamSynchronize(s));
+    return rounded > 0.0 && exact > 0.0 ? exact / rounded : 1.0;
 }
 
 }  // namespace eqc

@@ -45,6 +45,6 @@ struct SemOp {
 // rigidity).
 bool sem_usable(const Handle& h);
 void sem_launch(Handle& h, SemLoad load, SemEpi epi, SemPrev prev, const SemOp& o);
-void set_H_sem(const double* H, cudaStream_t s);
+double set_H_sem(const double* H, cudaStream_t s);   // returns Handle::sem_scale
 
 }  // namespace eqc
