@@ -237,7 +237,7 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
                              &h.q64, &h.Kd})
         b->alloc(N);
     for (DBuf<float>* b : {&h.r32, &h.z32, &h.p32, &h.q32, &h.x32, &h.g32, &h.p32b}) b->alloc(N);
-    if (h.opt.precision == EQC_MIXED && std::getenv("EQC_NO_DF_UPDATE") == nullptr) {
+    if (h.opt.precision == EQC_MIXED && h.df_ok && df_pays(L) && std::getenv("EQC_NO_DF_UPDATE") == nullptr) {
         h.dx64.alloc(N);    // the intermediate reliable updates' correction and its K dx
         h.kdx64.alloc(N);
     }
@@ -418,7 +418,8 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
     tma_init(h);
     EQC_CUDA(cudaMallocHost(&h.h_ctrl, sizeof(Ctrl)));
     std::memset(h.h_ctrl, 0, sizeof(Ctrl));
-    h.red_part.alloc(2 * 4096);
+    // one partial per CTA of a reducing launch: the widest is the double-float apply's (31 x 6 elements a CTA)
+    h.red_part.alloc(std::max<size_t>(8192, (size_t)(L.NelX / 31 + 1) * (L.NelY / 6 + 1)));
     h.red_count.alloc(64);
     h.scal.alloc(16);
     EQC_CUDA(cudaMallocHost(&h.h_scal, sizeof(double) * 16));

@@ -76,18 +76,16 @@ EQC_HD df df_mul(df x, df y) {
 EQC_HD df df_from_double(double x) {
     const int64_t b = df_bits64(x);
     const int32_t e = (int32_t)((b >> 52) & 0x7ff);
-    if (e < 1023 - 90 || e > 1023 + 120) return df{0.f, 0.f};
+    const bool in = e >= 1023 - 90 && e <= 1023 + 120;   // selected at the end: branches would serialise a caller's loads
     const int32_t sgn = (int32_t)((uint64_t)b >> 63) << 31;
     const int64_t m = b & 0xfffffffffffffLL;                 // 52 fraction bits
-    const float hi = df_from_bits32(sgn | ((e - 1023 + 127) << 23) | (int32_t)(m >> 29));
+    const int32_t hi = sgn | (int32_t)((uint32_t)(e - 1023 + 127) << 23) | (int32_t)(m >> 29);
     const int32_t rem = (int32_t)(m & 0x1fffffff);          // 29 remaining fraction bits
     // lo = +-rem * 2^(e - 1023 - 52): rem as a float (rounded to 24 bits), then the exponent
-    const float rf = (float)rem;                             // < 2^29, exact up to rounding
-    if (rem == 0) return df{hi, 0.f};
-    const int32_t rb = df_bits32(rf);
+    const int32_t rb = df_bits32((float)rem);                // < 2^29, exact up to rounding
     const int32_t re = ((rb >> 23) & 0xff) + (e - 1023 - 52);  // biased exponent of lo
-    if (re <= 0) return df{hi, 0.f};
-    return df{hi, df_from_bits32(sgn | (re << 23) | (rb & 0x7fffff))};
+    const int32_t lo = sgn | (int32_t)((uint32_t)re << 23) | (rb & 0x7fffff);
+    return df{df_from_bits32(in ? hi : 0), df_from_bits32(in && rem != 0 && re > 0 ? lo : 0)};
 }
 
 // double-float -> FP64 (one FP64 add; the widenings are exact and use integer operations)

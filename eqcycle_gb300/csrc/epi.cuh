@@ -172,18 +172,32 @@ __device__ __forceinline__ void epi_store4(const OpEpi<float>& E, float* y, int6
         cheb_x_pt(xo.z, xp.z, b.z, t.z, di.z, E.c1, E.c2), cheb_x_pt(xo.w, xp.w, b.w, t.w, di.w, E.c1, E.c2));
 }
 
-// One node (any precision).
+// One node (any precision): the operands' loads and what becomes of t with them.
+template <class T>
+struct EpiIn {
+    T b, dinv, x, xp;
+};
+template <class T>
+__device__ __forceinline__ EpiIn<T> epi_load1(const OpEpi<T>& E, int64_t i) {
+    EpiIn<T> v{};
+    if (E.mode >= 1) v.b = E.b[i];
+    if (E.mode == 2) {
+        v.dinv = E.dinv[i];
+        v.x = E.x[i];
+        if (E.xp) v.xp = E.xp[i];
+    }
+    return v;
+}
+template <class T>
+__device__ __forceinline__ void epi_finish1(const OpEpi<T>& E, T* y, int64_t i, T t, const EpiIn<T>& v) {
+    if (E.mode == 0) y[i] = t;
+    else if (E.mode == 1) E.out[i] = sub_rn<T>(v.b, t);
+    else if (!E.xp && !E.xp_zero) E.out[i] = fma_rn<T>(E.c2, mul_rn<T>(v.dinv, sub_rn<T>(v.b, t)), v.x);   // c1 = 0
+    else E.out[i] = cheb_x_pt<T>(v.x, v.xp, v.b, t, v.dinv, E.c1, E.c2);
+}
 template <class T>
 __device__ __forceinline__ void epi_store1(const OpEpi<T>& E, T* y, int64_t i, T t) {
-    if (E.mode == 0) {
-        y[i] = t;
-    } else if (E.mode == 1) {
-        E.out[i] = sub_rn<T>(E.b[i], t);
-    } else {
-        const T x = E.x[i];
-        const T xp = E.xp_zero ? T(0) : (E.xp ? E.xp[i] : x);
-        E.out[i] = cheb_x_pt<T>(x, xp, E.b[i], t, E.dinv[i], E.c1, E.c2);
-    }
+    epi_finish1(E, y, i, t, epi_load1(E, i));
 }
 
 #endif  // __CUDACC__

@@ -24,6 +24,7 @@
 #include "model.h"
 #include "vec.cuh"
 #include "epi.cuh"
+#include "cg.cuh"
 #include <cstdlib>
 #include <cmath>
 #include <type_traits>
@@ -582,8 +583,6 @@ __global__ void __launch_bounds__(NT) k_apply_pipe(const __grid_constant__ CUten
 // Rigidity of every element with one rigidity (k_classify), -1 for the others, on a grid shifted by
 // one column (column ex + 1; zero columns and rows outside the mesh).  An element outside the mesh
 // has rigidity 0.
-static int mu_pitch(int NelX) { return (NelX + 3) & ~1; }
-
 // Tolerance 2^-49: W is a rounded product of weights and rigidity (and of damage factors), a few
 // units in the last place from the product formed here.
 // mu32: the rigidity over `unit` rounded to FP32; *several counts the elements of several.
@@ -657,12 +656,17 @@ static_assert(UniTile::OY * UniTile::EX == UNT && UniTile::EY * UniTile::OX <= U
 // Back to back on the damage-zone models, before (both contractions, 8 x 7 tiles) and now: 61 x 95
 // elements 19.4 and 10.4 us, 120 x 240 37.1 and 21.9, 240 x 480 134.2 and 68.6 (122.8 and 60.8 where
 // one x and y stay in L2), 480 x 960 496 and 248: 48 us of the 60.8 are the pipe's.
+// RES: the mixed solver's residual r64 = -K_II x with ResidualOut's work (sign -1, zero_row0).
+template <bool RES>
 __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUtensorMap umap,
                                                      const __grid_constant__ CUtensorMap mmap, double* __restrict__ y,
                                                      ApplyArgs<double> A, double sign, int zero_row0, int ntx, int ntiles,
-                                                     OpEpi<double> E) {
+                                                     OpEpi<double> E, ResidualOut R) {
     EQC_GRID_WAIT();
     if (A.gate && *A.gate != A.gate_val) return;
+    const double sg = RES ? R.S->sigma : 0.0;
+    const int es = RES ? R.S->sigma_exp : 0;
+    DotAcc<float> acc;
     using UT = UniTile;
     const Layout& L = A.L;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -742,7 +746,7 @@ __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUt
                     for (int it = 0; it < MBAR_SPIN_LIMIT; ++it)
                         if (mbar_try_wait(&bar[j % PSTAGES], (uint32_t)((j / PSTAGES) & 1))) break;
             }
-            return;
+            break;
         }
         double v[4];
         if (has_y) {
@@ -772,20 +776,38 @@ __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUt
                 for (int l = 0; l < 4; ++l) v[l] = fma(kap, s[l], ys[(4 * (er - 1) + l) * UT::OX + q]);
             }
         }
+        // the epilogue's operands, in flight across the barrier
+        const int ix = 4 * ex0 + q, iy0 = 4 * (ey0 + er - 1);
+        const bool mine = has_y && er > 0 && ix < L.nx;
+        const int64_t o0 = (int64_t)iy0 * L.ld + ix;
+        EpiIn<double> in[4];
+        if (mine && !RES) {
+#pragma unroll
+            for (int l = 0; l < 4; ++l)
+                if (iy0 + l < L.ny) in[l] = epi_load1(E, o0 + (int64_t)l * L.ld);
+        }
         __syncthreads();   // cy written; every read of this stage and of ys done
         if (threadIdx.x == 0) {
             const int tn = t + PSTAGES * gridDim.x;
             if (tn < ntiles) issue(tn, st);
         }
-        const int ix = 4 * ex0 + q, iy0 = 4 * (ey0 + er - 1);
-        if (has_y && er > 0 && ix < L.nx) {
+        if (mine) {
             v[0] += cy[(er - 1) * UT::OX + q];
 #pragma unroll
             for (int l = 0; l < 4; ++l)
-                if (iy0 + l < L.ny)
-                    epi_store1(E, y, (int64_t)(iy0 + l) * L.ld + ix, (zero_row0 && iy0 + l == 0) ? 0.0 : v[l]);
+                if (iy0 + l < L.ny) {
+                    const int64_t o = o0 + (int64_t)l * L.ld;
+                    const double t = (zero_row0 && iy0 + l == 0) ? 0.0 : v[l];
+                    if constexpr (RES) {
+                        R.r64[o] = t;
+                        R.r32[o] = residual32(t, es, sg, acc);
+                    } else {
+                        epi_finish1(E, y, o, t, in[l]);
+                    }
+                }
         }
     }
+    if constexpr (RES) residual_done(R, acc);
 }
 
 // ---- element-per-lane version (FP32) --------------------------------------------------------
@@ -1298,6 +1320,13 @@ void classify_elements(Handle& h) {
     const int64_t Nel = (int64_t)L.NelX * L.NelY;
     if (!h.mu64.p) h.mu64.alloc((size_t)mp * L.NelY);
     if (!h.mu32.p) h.mu32.alloc(Nel);
+    if (h.mu_unit == 0.0) {
+        double w = 0.0;
+        EQC_CUDA(cudaMemcpyAsync(&w, h.W64.p + 25 * (Nel - 1) + 12, sizeof(w), cudaMemcpyDeviceToHost, h.stream));
+        EQC_CUDA(cudaStreamSynchronize(h.stream));
+        w /= (32.0 / 45.0) * (32.0 / 45.0);
+        h.mu_unit = w > 0.0 && std::isfinite(w) ? w : 1.0;
+    }
     DBuf<int> several;
     several.alloc(1);
     k_classify<<<(int)std::min<int64_t>((Nel + 255) / 256, 4096), 256, 0, h.stream>>>(
@@ -1320,13 +1349,6 @@ template <class K>
 static int resident_blocks(K kernel, int threads, int bytes) {
     EQC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     int per_sm = 0, dev = 0, nsm = 0;
-    if (h.mu_unit == 0.0) {
-        double w = 0.0;
-        EQC_CUDA(cudaMemcpyAsync(&w, h.W64.p + 25 * (Nel - 1) + 12, sizeof(w), cudaMemcpyDeviceToHost, h.stream));
-        EQC_CUDA(cudaStreamSynchronize(h.stream));
-        w /= (32.0 / 45.0) * (32.0 / 45.0);
-        h.mu_unit = w > 0.0 && std::isfinite(w) ? w : 1.0;
-    }
     EQC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes));
     EQC_CUDA(cudaGetDevice(&dev));
     EQC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1334,25 +1356,29 @@ static int resident_blocks(K kernel, int threads, int bytes) {
 }
 
 // Launch shape of k_apply_uni64: g_uni_sms SMs, at most g_uni_per_sm CTAs on each.
-static int g_uni_sms = 0, g_uni_per_sm = 0, g_uni_smem = 0;
+static int g_uni_sms = 0, g_uni_per_sm[2] = {0, 0};   // [RES]
+constexpr int UNI_SMEM = 120 * 1024;   // the most a CTA asks for: then one fits an SM
 static void uni_setup() {
     int dev = 0;
     EQC_CUDA(cudaGetDevice(&dev));
     EQC_CUDA(cudaDeviceGetAttribute(&g_uni_sms, cudaDevAttrMultiProcessorCount, dev));
-    EQC_CUDA(cudaDeviceGetAttribute(&g_uni_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    g_uni_per_sm = resident_blocks(k_apply_uni64, UNT, UniTile::BYTES) / g_uni_sms;
-    EQC_CUDA(cudaFuncSetAttribute(k_apply_uni64, cudaFuncAttributeMaxDynamicSharedMemorySize, g_uni_smem));
+    g_uni_per_sm[0] = resident_blocks(k_apply_uni64<false>, UNT, UniTile::BYTES) / g_uni_sms;
+    g_uni_per_sm[1] = resident_blocks(k_apply_uni64<true>, UNT, UniTile::BYTES) / g_uni_sms;
+    EQC_CUDA(cudaFuncSetAttribute(k_apply_uni64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, UNI_SMEM));
+    EQC_CUDA(cudaFuncSetAttribute(k_apply_uni64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, UNI_SMEM));
 }
 // The FP64 pipe of each SM bounds the kernel, so its CTAs have to be spread evenly: per SM no more than
 // an even spread of the tiles needs, kept to that by the shared memory that a CTA asks for.  (A
 // programmatic launch otherwise fills the SMs that its predecessor leaves empty with several CTAs
 // each: 26 us instead of 16 back to back on 61 x 95 elements.)
 static void launch_uni64(const CUtensorMap& um, double* y, const ApplyArgs<double>& A, double sign, int zr,
-                         cudaStream_t s, const OpEpi<double>& E = OpEpi<double>()) {
+                         cudaStream_t s, const OpEpi<double>& E = OpEpi<double>(), const ResidualOut* R = nullptr) {
     const int ntx = A.L.NelX / UEX + 1, ntiles = ntx * (A.L.NelY / UEY + 1);
-    const int per_sm = std::min(g_uni_per_sm, (ntiles + g_uni_sms - 1) / g_uni_sms);
-    const int smem = std::max(UniTile::BYTES, std::min(g_uni_smem, 228 * 1024 / (per_sm + 1) / 128 * 128 + 128));
-    k_apply_uni64<<<std::min(ntiles, per_sm * g_uni_sms), UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles, E);
+    const int per_sm = std::min(g_uni_per_sm[R != nullptr], (ntiles + g_uni_sms - 1) / g_uni_sms);
+    const int smem = std::max(UniTile::BYTES, std::min(UNI_SMEM, 228 * 1024 / (per_sm + 1) / 128 * 128 + 128));
+    const int grid = std::min(ntiles, per_sm * g_uni_sms);
+    if (R) k_apply_uni64<true><<<grid, UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles, E, *R);
+    else k_apply_uni64<false><<<grid, UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles, E, ResidualOut());
     EQC_CHECK_LAUNCH();
     count_launch();
 }
@@ -1551,6 +1577,14 @@ bool apply_K_epi(const double* x, const ApplyArgs<double>& A, int mode, const Op
     const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
     if (!uu) return false;
     launch_uni64(*uu, nullptr, A, 1.0, mode, s, E);
+    return true;
+}
+
+bool apply_K_residual(const double* x, const ApplyArgs<double>& A, const ResidualOut& R, cudaStream_t s) {
+    if (!A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
+    const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
+    if (!uu) return false;
+    launch_uni64(*uu, nullptr, A, -1.0, 1, s, OpEpi<double>(), &R);
     return true;
 }
 

@@ -79,6 +79,7 @@ struct CGState {
                        // FP32 underflow); 1 in FP64.  rr is in those scaled units.
     double inv_sigma;  // 1 / sigma
     int sigma_exp;     // sigma = 2^sigma_exp
+    int dx_clear;      // dx64 counts as zero whatever it holds (x's change since r64 was last exact)
     double rr_guess;   // ||r||^2 with the initial-guess increment applied
     int guess_keep;    // the increment lowered the residual and is kept
 };
@@ -225,6 +226,7 @@ void materialize_dyn_state(Handle& h);
 // kapply.cu
 // Uploads the derivative matrix; true when it admits one-contraction lines (Handle::uni_ok).
 bool set_H(const double* H, cudaStream_t s);
+inline int mu_pitch(int NelX) { return (NelX + 3) & ~1; }   // row pitch of mu64
 // mu64 from W64 (after every change of W64)
 void classify_elements(Handle& h);
 template <class T>
@@ -239,9 +241,29 @@ inline ApplyArgs<float> args32(Handle& h) {
 }
 void tma_init(Handle& h);
 void set_H_df(const double* H, cudaStream_t s);
-// y = sign K x (FP64 vectors, mode 0/1) in double-float arithmetic; false when unavailable.
+// What an FP64-class apply of the mixed solver does with t = -(K v)_i at its nodes beside storing the
+// residual: r32 = (float) (sigma r64), S->rr = r32.r32 and, with check, the end of a reliable update
+// (cg_check_b).  incr: r64 += t / sigma (t of the scaled change dx), else r64 = t.
+struct ResidualOut {
+    double* r64 = nullptr;
+    float* r32 = nullptr;
+    double* part = nullptr;
+    unsigned* count = nullptr;
+    CGState* S = nullptr;
+    Ctrl* C = nullptr;
+    cudaGraphConditionalHandle hw = 0;
+    int use_cond = 0, check = 0;
+};
+// The double-float apply takes 27 us on any small mesh (one CTA's chain of instructions), the FP64 one
+// (kapply.cu's one-contraction lines) 14.6 us on 48 x 48 elements, 27 on 120 x 240 (double-float 29), 40 on
+// 180 x 300 (30), 71 on 240 x 480 (39), 250 on 480 x 960 (127): the line lies between the third and the fourth.
+inline bool df_pays(const Layout& L) { return (int64_t)L.NelX * L.NelY >= 32000; }
+// y = sign K x (FP64 vectors, mode 0/1) in double-float arithmetic, or in FP64 where that is faster; with R, K_II x of the scaled change
+// straight into the residual (y and sign unused).  False when unavailable.
 bool apply_K_df(Handle& h, const double* x, double* y, double sign, int mode, cudaStream_t s,
-                const int* gate = nullptr, int gate_val = 0);
+                const int* gate = nullptr, int gate_val = 0, const ResidualOut* R = nullptr);
+// r64 = -K_II x in FP64 with ResidualOut's work in the launch; false when the FP64 apply in use has none.
+bool apply_K_residual(const double* x, const ApplyArgs<double>& A, const ResidualOut& R, cudaStream_t s);
 void tma_init_for(TmaCache& c, const Layout& L, const float* W32p, const double* W64p, const double* mu);
 // Apply y = K x (mode 0/1 as apply_K) whose owned nodes are finished by the epilogue E
 // (residual or Chebyshev step) instead of stored; false when the selected kernel has none.

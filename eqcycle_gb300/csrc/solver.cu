@@ -136,18 +136,18 @@ __global__ void __launch_bounds__(VEC_THREADS) k_fold(double* __restrict__ x, fl
     EQC_GRID_WAIT();
     const double inv = S->inv_sigma;
     const int es = -S->sigma_exp;
-    const bool incr = dx && S->upd_incr;
+    const bool incr = dx && S->upd_incr, clear = S->dx_clear;
     for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
         double xx[4], dd[4];
         float yy[4];
         ld4(x + i, xx);
         ld4(y + i, yy);
-        if (incr) ld4(dx + i, dd);
+        if (incr && !clear) ld4(dx + i, dd);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const double yw = f32_to_f64(yy[k]);
             xx[k] += pow2_scale(yw, es, inv);
-            if (incr) dd[k] += yw;
+            if (incr) dd[k] = clear ? yw : dd[k] + yw;
         }
         st4(x + i, xx);
         if (incr) st4(dx + i, dd);
@@ -158,51 +158,41 @@ __global__ void __launch_bounds__(VEC_THREADS) k_fold(double* __restrict__ x, fl
 
 // dx64 = sigma times the kept initial-guess increment (r64 is the residual without it), else 0.
 // (widening and the power-of-two scaling by integer operations: the bits of (double) g * sigma)
-__global__ void k_dx_init(double* __restrict__ dx, const float* __restrict__ g, const CGState* S, int64_t n) {
+__global__ void k_dx_init(double* __restrict__ dx, const float* __restrict__ g, CGState* S, int64_t n) {
     EQC_GRID_WAIT();
+    if (blockIdx.x == 0 && threadIdx.x == 0) S->dx_clear = 0;
     const bool keep = g && S->guess_keep;
     const double sg = S->sigma;
     const int es = S->sigma_exp;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         dx[i] = keep ? pow2_scale(f32_to_f64(g[i]), es, sg) : 0.0;
 }
-// [intermediate reliable update (kdx given and S->upd_incr): r64 += kdx / sigma, kdx the
-// double-float -K dx of the scaled change] ; r32 = (float) (sigma r64) ; S->rr = r32.r32 (the
-// scaled norm, of the FP32 residual: within 1e-7 of sigma^2 r64.r64)
-// (kdx given: a reliable update's end; r64 is then exact for x, so dx64 = 0.)  The scaling and
-// the rounding to FP32 use integer operations (pow2_scale, f64_to_f32) and the norm the FP32
-// compensated sum: GB300's FP64 rate is a small fraction of its FP32 and integer rates.
-__global__ void __launch_bounds__(VEC_THREADS) k_demote_norm(double* __restrict__ r64, float* __restrict__ r32,
-                                                             int64_t n, double* part, unsigned* count, CGState* S,
-                                                             const double* __restrict__ kdx, double* __restrict__ dx) {
+// The residual where its apply's launch did not also demote it: [intermediate reliable update (kdx given
+// and S->upd_incr): r64 += kdx / sigma, kdx the double-float -K dx of the scaled change] ; r32 = (float)
+// (sigma r64) ; S->rr = r32.r32 (the scaled norm, of the FP32 residual: within 1e-7 of sigma^2 r64.r64).
+// r64 is then exact for x (dx_clear).
+__global__ void __launch_bounds__(VEC_THREADS) k_demote_norm(ResidualOut R, int64_t n, const double* __restrict__ kdx) {
     EQC_GRID_WAIT();
-    const double sg = S->sigma, inv = S->inv_sigma;
-    const int es = S->sigma_exp;
-    const bool incr = kdx && S->upd_incr;
+    const double sg = R.S->sigma, inv = R.S->inv_sigma;
+    const int es = R.S->sigma_exp;
+    const bool incr = kdx && R.S->upd_incr;
     DotAcc<float> acc;
     for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
         double v[4];
         float f[4];
-        ld4(r64 + i, v);
+        ld4(R.r64 + i, v);
         if (incr) {
             double t[4];
             ld4(kdx + i, t);
 #pragma unroll
             for (int k = 0; k < 4; ++k) v[k] = __fma_rn(t[k], inv, v[k]);
-            st4(r64 + i, v);
-        }
-        if (dx) {
-            const double zero[4] = {0.0, 0.0, 0.0, 0.0};
-            st4(dx + i, zero);
+            st4(R.r64 + i, v);
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            f[k] = f64_to_f32(pow2_scale(v[k], es, sg));
-            acc.add(f[k], f[k]);
-        }
-        st4(r32 + i, f);
+        for (int k = 0; k < 4; ++k) f[k] = residual32(v[k], es, sg, acc);
+        st4(R.r32 + i, f);
     }
-    grid_sum(acc, part, count, [&](double t) { S->rr = t; });
+    residual_done(R, acc);
 }
 
 // Scale of the FP32 recurrence for this solve: sigma = 2^-e with 2^e <= ||b|| < 2^(e+1)
@@ -275,28 +265,10 @@ __device__ __forceinline__ int cg_check_a(CGState* S, double delta) {
     return need;
 }
 
-// Mixed precision, end of the iteration: take the FP64 residual of a reliable update and
-// decide whether the loop goes on.
+// The end of a reliable update where the apply's launch does not carry it.
 __global__ void k_cg_check_b(CGState* S, Ctrl* C, cudaGraphConditionalHandle hw, int use_cond) {
     EQC_GRID_WAIT();
-    if (S->done != 3) {
-        if (S->need_update) {
-            const double rs = sqrt(S->rr) * S->inv_sigma;
-            // the true residual left the recurrence's (the FP32 recurrences drifted, e.g. from a
-            // guess far from the solution): continue from the true residual with a fresh direction
-            if (rs > 2.0 * S->res) {
-                S->restart = 1;
-                C->cg_restarts += 1;
-            }
-            S->res = rs;
-            S->rmax = rs;
-            S->need_update = 0;
-            C->cg_updates += 1;
-        }
-        const double r = S->res;
-        S->done = !isfinite(r) ? 3 : (r <= S->reltol ? 1 : (S->it >= S->maxit ? 2 : 0));
-    }
-    if (use_cond) cudaGraphSetConditional(hw, S->done == 0 ? 1u : 0u);
+    cg_check_b(S, C, hw, use_cond);
 }
 
 // After the loop: solve counters and failure flags in the control block.  mark_valid: the
@@ -407,21 +379,36 @@ static void setup_rhs(Handle& h, bool mixed) {
     count_launch();
 }
 
+// r64, r32 and the reduction's scratch as an apply's launch writes them; slices of rows >= 1 for the vector
+// kernels (interior)
+static ResidualOut residual_out(Handle& h, bool interior) {
+    const int64_t o = interior ? h.L.ld : 0;
+    ResidualOut R;
+    R.r64 = h.r64.p + o;
+    R.r32 = h.r32.p + o;
+    R.part = h.red_part.p;
+    R.count = h.red_count.p;
+    R.S = h.cg.p;
+    R.C = h.ctrl.p;
+    return R;
+}
+static void demote(Handle& h, const ResidualOut& R, const double* kdx) {
+    const int64_t n = h.L.size() - h.L.ld;
+    k_demote_norm<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(R, n, kdx);
+    EQC_CHECK_LAUNCH();
+    count_launch();
+}
+
 // Full initial residual: r64 = b - K_II d_I (rows >= 1, row 0 zero), S->rr = ||r||^2, and in
 // mixed precision r32 = (float) r64.
 static void setup_residual_full(Handle& h, bool mixed) {
     const Layout& L = h.L;
     const int64_t ld = L.ld, n = L.size() - ld;
     CGState* S = h.cg.p;
+    if (mixed && apply_K_residual(h.d.p, args64(h), residual_out(h, false), h.stream)) return;
     apply_K<double>(h.d.p, h.r64.p, args64(h), -1.0, 1, h.stream);     // r = -(K d)_I
-    if (mixed) {
-        k_demote_norm<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p,
-                                                             h.red_count.p, S, nullptr, h.dx64.p ? h.dx64.p + ld : nullptr);
-        EQC_CHECK_LAUNCH();
-        count_launch();
-    } else {
-        dot64(h, h.r64.p + ld, h.r64.p + ld, n, &S->rr);
-    }
+    if (mixed) demote(h, residual_out(h, true), nullptr);
+    else dot64(h, h.r64.p + ld, h.r64.p + ld, n, &S->rr);
 }
 
 // Carried residual: r64 -= K_IF (F - Flast) on rows 1..4 (tmp64b row 0 holds F - Flast), then
@@ -431,10 +418,9 @@ static void setup_residual_carry(Handle& h, const float* guess) {
     const int64_t ld = h.L.ld, n = h.L.size() - ld;
     apply_K<double>(h.tmp64b.p, h.tmp64c.p, args64(h), -1.0, 2, h.stream);
     k_carry_rows<<<vgrid<double>(4 * ld), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.tmp64c.p + ld, 4 * ld);
-    k_demote_norm<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p,
-                                                         h.red_count.p, h.cg.p, nullptr, h.dx64.p ? h.dx64.p + ld : nullptr);
     EQC_CHECK_LAUNCH();
-    count_launch(2);
+    count_launch();
+    demote(h, residual_out(h, true), nullptr);
     if (guess) {
         apply_K<float>(guess, h.q32.p, args32(h), 1.0f, 1, h.stream);
         k_guess_residual<<<vgrid<float>(n), VEC_THREADS, 0, h.stream>>>(h.r32.p + ld, h.q32.p + ld, n, h.red_part.p,
@@ -544,23 +530,33 @@ static void iter_mixed_a(Handle& h, double delta, cudaGraphConditionalHandle hi,
 static int incr_updates(const Handle& h, bool mixed) {
     return (mixed && h.df_ok && h.dx64.p && h.kdx64.p) ? 1 : 0;
 }
-static void update_mixed(Handle& h) {
+static void update_mixed(Handle& h, cudaGraphConditionalHandle hw, int use_cond) {
     const Layout& L = h.L;
     const int64_t ld = L.ld, n = L.size() - ld;
     CGState* S = h.cg.p;
     const bool incr = incr_updates(h, true) != 0;
     k_fold<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.d.p + ld, h.x32.p + ld, incr ? h.dx64.p + ld : nullptr, n, S);
+    EQC_CHECK_LAUNCH();
+    count_launch();
     ApplyArgs<double> a64 = args64(h);
     if (incr) {
         a64.gate = &S->upd_incr;
         a64.gate_val = 0;
-        apply_K_df(h, h.dx64.p, h.kdx64.p, -1.0, 1, h.stream, &S->upd_incr, 1);   // -K_II dx
     }
-    apply_K<double>(h.d.p, h.r64.p, a64, -1.0, 1, h.stream);                    // r = -(K d)_I
-    k_demote_norm<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.r64.p + ld, h.r32.p + ld, n, h.red_part.p, h.red_count.p,
-                                                         S, incr ? h.kdx64.p + ld : nullptr, incr ? h.dx64.p + ld : nullptr);
+    ResidualOut R = residual_out(h, false);
+    R.hw = hw;
+    R.use_cond = use_cond;
+    R.check = 1;
+    if (apply_K_residual(h.d.p, a64, R, h.stream)) {                            // r = -(K d)_I
+        if (incr) apply_K_df(h, h.dx64.p, nullptr, -1.0, 1, h.stream, &S->upd_incr, 1, &R);   // r -= K_II dx
+        return;
+    }
+    if (incr) apply_K_df(h, h.dx64.p, h.kdx64.p, -1.0, 1, h.stream, &S->upd_incr, 1);
+    apply_K<double>(h.d.p, h.r64.p, a64, -1.0, 1, h.stream);
+    demote(h, residual_out(h, true), incr ? h.kdx64.p + ld : nullptr);
+    k_cg_check_b<<<1, 1, 0, h.stream>>>(S, h.ctrl.p, hw, use_cond);
     EQC_CHECK_LAUNCH();
-    count_launch(2);
+    count_launch();
 }
 
 constexpr double RELIABLE_DELTA = 1e-3;   // default residual-replacement factor
@@ -627,9 +623,7 @@ void enqueue_solve(Handle& h, double tol, int maxit, bool graph, bool carry, con
             iter_mixed_a(h, delta, hi, hw, 1);
             const int64_t t1 = capture_tally();
             cond_begin(h, cudaGraphCondTypeIf, hi);
-            update_mixed(h);
-            k_cg_check_b<<<1, 1, 0, h.stream>>>(S, h.ctrl.p, hw, 1);
-            count_launch();
+            update_mixed(h, hw, 1);
             cond_end(h);
             if (h.capturing) {
                 h.capturing->k_update = capture_tally() - t1;
@@ -652,11 +646,7 @@ void enqueue_solve(Handle& h, double tol, int maxit, bool graph, bool carry, con
             if (mixed) {
                 iter_mixed_a(h, delta, 0, 0, 0);
                 hs = &read_cg(h);
-                if (hs->need_update) {
-                    update_mixed(h);
-                    k_cg_check_b<<<1, 1, 0, h.stream>>>(S, h.ctrl.p, 0, 0);
-                    count_launch();
-                }
+                if (hs->need_update) update_mixed(h, 0, 0);
             } else {
                 iter_fp64(h, 0, 0);
             }
