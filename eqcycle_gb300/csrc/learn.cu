@@ -5,6 +5,8 @@
 // the same seed gives bitwise the same weights.
 #include "learn.h"
 #include "reduce.cuh"
+#include "vec.cuh"
+#include "gemm32.cuh"
 #include <cmath>
 #include <random>
 #include <algorithm>
@@ -19,70 +21,194 @@ __device__ __forceinline__ float gelu_grad(float x) {
     return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
-// ---- GEMM: C[m][n] = sum_k A(m,k) B(k,n) (+ bias[n]); optional GELU copy.  64x64 tiles,
-// 16-deep k slices, 256 threads with 4x4 outputs each; operands BF16 or FP32, FP32 products.
-template <class TA, class TB>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const TA* __restrict__ A, int64_t sam, int64_t sak,
-                                              const TB* __restrict__ B, int64_t sbk, int64_t sbn, float* __restrict__ C,
-                                              int64_t ldc, const float* __restrict__ bias, float* __restrict__ Cg) {
-    EQC_GRID_WAIT();
-    __shared__ float As[16][65];
-    __shared__ float Bs[16][65];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            int kk, mm;
-            if (sak == 1) { mm = e >> 4; kk = e & 15; } else { kk = e >> 6; mm = e & 63; }
-            const int m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < K) ? tof(A[(int64_t)m * sam + (int64_t)k * sak]) : 0.f;
-        }
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            int kk, nn;
-            if (sbn == 1) { kk = e >> 6; nn = e & 63; } else { nn = e >> 4; kk = e & 15; }
-            const int n = n0 + nn, k = k0 + kk;
-            Bs[kk][nn] = (n < N && k < K) ? tof(B[(int64_t)k * sbk + (int64_t)n * sbn]) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
+// ---- layers as tiled products (gemm32.cuh) ------------------------------------------------
+// What becomes of C(m, n).  sum, sum_done: the row sums of A, where the layer's bias needs them.
+struct EpNoSum {
+    __device__ void sum(const float (&)[8], int) {}
+    __device__ void sum_done(int, int, int) {}
+};
+struct EpLinear : EpNoSum {   // C = v + bias[n], and its GELU where the next layer takes that
+    float* C;
+    int64_t ldc;
+    const float* bias;
+    float* Cg;
+    __device__ int64_t npos(int n) const { return n; }
+    __device__ void put(int m, int n, int64_t, float v) const {
+        v += bias ? bias[n] : 0.f;
+        C[m * ldc + n] = v;
+        if (Cg) Cg[m * ldc + n] = gelu(v);
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
-            if (m < M && n < N) {
-                const float v = acc[i][j] + (bias ? bias[n] : 0.f);
-                C[(int64_t)m * ldc + n] = v;
-                if (Cg) Cg[(int64_t)m * ldc + n] = gelu(v);
-            }
+};
+struct EpGeluGrad : EpNoSum {   // C = v GELU'(z)
+    float* C;
+    const float* z;
+    int64_t ldc;
+    __device__ int64_t npos(int n) const { return n; }
+    __device__ void put(int m, int n, int64_t, float v) const { C[m * ldc + n] = v * gelu_grad(z[m * ldc + n]); }
+};
+struct EpConv : EpNoSum {   // n = (b, t), m = channel: z = v + bias[m], a = GELU(z)
+    float *z, *a;
+    const float* bias;
+    int T;
+    __device__ int64_t npos(int n) const { return (int64_t)(n / T) * GN_C * T + n % T; }
+    __device__ void put(int m, int, int64_t np, float v) const {
+        v += bias[m];
+        z[np + (int64_t)m * T] = v;
+        a[np + (int64_t)m * T] = gelu(v);
+    }
+};
+struct EpConvGrad : EpNoSum {   // n = (b, u) for the positions 2 u + par: g = v GELU'(z)
+    float* g;
+    const float* z;
+    int T, U, par;
+    __device__ int64_t npos(int n) const { return (int64_t)(n / U) * GN_C * T + 2 * (n % U) + par; }
+    __device__ void put(int m, int, int64_t np, float v) const {
+        const int64_t i = np + (int64_t)m * T;
+        g[i] = v * gelu_grad(z[i]);
+    }
+};
+// Weight and bias gradients: whole sums (a fully connected layer's K is the batch) or a split's share.
+template <bool KF, bool PART>
+struct EpWeight {
+    float* C;
+    float* db;         // !PART
+    double* db_part;   // PART: [split][M]
+    int M, N;
+    RowSum<KF> rs;
+    __device__ void sum(const float (&v)[8], int n0) {
+        if (n0 == 0) rs.add(v);
+    }
+    __device__ void sum_done(int m0, int n0, int) {
+        if (n0 != 0) return;
+        rs.done(m0, M, [&](int m, double d) {
+            if (PART) db_part[(int64_t)blockIdx.z * M + m] = d;
+            else db[m] = (float)d;
+        });
+    }
+    __device__ int64_t npos(int n) const { return (PART ? (int64_t)blockIdx.z * M * N : 0) + n; }
+    __device__ void put(int m, int, int64_t np, float v) const { C[np + (int64_t)m * N] = v; }
+};
+// gW and gb from the splits' shares, to FP64's accuracy: 32 results a CTA, every eighth split a warp (481 splits of
+// conv1's 640 weights: 73 us with a thread to each result).
+__global__ void __launch_bounds__(256) k_weight_sum(const float* __restrict__ part, const double* __restrict__ db_part,
+                                                    int splits, int M, int N, float* __restrict__ gW, float* __restrict__ gb) {
+    EQC_GRID_WAIT();
+    __shared__ double sh[8][32];
+    const int n = M * N, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    double s = 0.0;
+    if (i < n) {   // error-free in FP32: FP64 adds and conversions would take the longer part of the launch
+        float hi = 0.f, lo = 0.f;
+#pragma unroll 8
+        for (int z = w; z < splits; z += 8) {
+            float t, e;
+            two_sum(hi, part[(int64_t)z * n + i], t, e);
+            hi = t;
+            lo += e;
         }
+        s = (double)hi + (double)lo;
+    } else if (i < n + M) {
+        for (int z = w; z < splits; z += 8) s += db_part[(int64_t)z * M + i - n];
+    }
+    sh[w][lane] = s;
+    __syncthreads();
+    if (w != 0 || i >= n + M) return;
+#pragma unroll
+    for (int q = 1; q < 8; ++q) s += sh[q][lane];
+    if (i < n) gW[i] = (float)s;
+    else gb[i - n] = (float)s;
 }
 
-template <class TA, class TB>
-static void gemm(int M, int N, int K, const TA* A, int64_t sam, int64_t sak, const TB* B, int64_t sbk, int64_t sbn,
-                 float* C, int64_t ldc, const float* bias, float* Cg, cudaStream_t s) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    k_gemm<TA, TB><<<grid, 256, 0, s>>>(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, bias, Cg);
+// Convolution operands (kernel 5, stride 2, padding 2).  The layer's input at output position (b, t) and tap
+// (ci, k): in[b][ci][2t + k - 2], the positions along mn (forward) or along k (weight gradient).
+__device__ __forceinline__ uint32_t raw(float v) { return __float_as_uint(v); }
+__device__ __forceinline__ uint32_t raw(__nv_bfloat16 v) { return (uint32_t)__bfloat16_as_ushort(v) << 16; }
+template <bool KF>
+struct OpGather {
+    static constexpr bool K_FAST = KF, VEC = false;
+    __device__ static float value(const uint32_t (&v)[8], int i) { return __uint_as_float(v[i]); }
+};
+template <bool POS_K>
+struct OpConvIn : OpGather<POS_K> {
+    const float* in;
+    int Cin, Tin, Tout;
+    __device__ TilePtr<float> ptr(int n) const { return {in + (int64_t)(n / Tout) * Cin * Tin, 2 * (n % Tout) - 2}; }
+    __device__ TileOff off(int k) const { return {k / GN_K * Tin, k % GN_K}; }
+    __device__ uint32_t get(TilePtr<float> a, TileOff b, bool& ok) const {
+        const int s = a.s + b.s;
+        ok = s >= 0 && s < Tin;
+        return raw(a.q[b.off + min(max(s, 0), Tin - 1)]);
+    }
+};
+struct OpConvW : OpGather<true> {   // W[co][ci][k], m = co, k = (ci, k)
+    const __nv_bfloat16* W;
+    int ld;
+    __device__ TilePtr<__nv_bfloat16> ptr(int k) const { return {W + k, 0}; }
+    __device__ TileOff off(int m) const { return {m * ld, 0}; }
+    __device__ uint32_t get(TilePtr<__nv_bfloat16> a, TileOff b, bool&) const { return raw(a.q[b.off]); }
+};
+struct OpConvGz : OpGather<true> {   // g_z[b][co][t], m = co, k = (b, t)
+    const float* gz;
+    int T;
+    __device__ TilePtr<float> ptr(int k) const { return {gz + (int64_t)(k / T) * GN_C * T + k % T, 0}; }
+    __device__ TileOff off(int m) const { return {m * T, 0}; }
+    __device__ uint32_t get(TilePtr<float> a, TileOff b, bool&) const { return raw(a.q[b.off]); }
+};
+// The input's gradient at s = 2u + par: taps par + 2j, j < J = 3 - par, from the output positions u + 1 - j.
+template <int J>
+struct OpTapsW : OpGather<false> {   // W[co][m][par + 2j], k = (co, j)
+    const __nv_bfloat16* W;
+    __device__ TilePtr<__nv_bfloat16> ptr(int m) const { return {W + m * GN_K + 3 - J, 0}; }
+    __device__ TileOff off(int k) const { return {k / J * (GN_C * GN_K) + 2 * (k % J), 0}; }
+    __device__ uint32_t get(TilePtr<__nv_bfloat16> a, TileOff b, bool&) const { return raw(a.q[b.off]); }
+};
+template <int J>
+struct OpTapsGz : OpGather<false> {   // g_z[b][co][u + 1 - j], n = (b, u)
+    const float* gz;
+    int T, U;
+    __device__ TilePtr<float> ptr(int n) const { return {gz + (int64_t)(n / U) * GN_C * T, n % U + 1}; }
+    __device__ TileOff off(int k) const { return {k / J * T, -(k % J)}; }
+    __device__ uint32_t get(TilePtr<float> a, TileOff b, bool& ok) const {
+        const int t = a.s + b.s;
+        ok = t >= 0 && t < T;
+        return raw(a.q[b.off + min(max(t, 0), T - 1)]);
+    }
+};
+
+template <int S, class OA, class OB, class EP>
+static void tile_launch(const OA& A, const OB& B, const EP& E, int M, int N, int K, dim3 g, cudaStream_t s) {
+    if constexpr (S == 1) {
+        k_tile<OA, OB, EP, 1><<<g, GT_THREADS, 0, s>>>(A, B, E, M, N, K, K);
+    } else {
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3(g.x, g.y, S);
+        c.blockDim = dim3(GT_THREADS);
+        c.stream = s;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1;
+        at.val.clusterDim.y = 1;
+        at.val.clusterDim.z = S;
+        c.attrs = &at;
+        c.numAttrs = 1;
+        const int chunk = ((K + S - 1) / S + GT_K - 1) / GT_K * GT_K;
+        EQC_CUDA(cudaLaunchKernelEx(&c, k_tile<OA, OB, EP, S>, A, B, E, M, N, K, chunk));
+    }
     EQC_CHECK_LAUNCH();
     count_launch();
+}
+// K is split over a cluster where the tiles alone leave SMs idle: up to two CTAs for each SM and 64 of K and
+// more to each CTA.  SPLIT: not with row sums, which are of a CTA's K.
+template <bool SPLIT = true, class OA, class OB, class EP>
+static void tile(const OA& A, const OB& B, const EP& E, int M, int N, int K, cudaStream_t s) {
+    if (N == 0) return;   // the odd positions of a layer with one
+    const dim3 g((N + GT_N - 1) / GT_N, (M + GT_N - 1) / GT_N);
+    const int tiles = (int)(g.x * g.y);
+    if constexpr (SPLIT) {
+        if (tiles * 8 <= 2 * 152 && K >= 8 * 64) return tile_launch<8>(A, B, E, M, N, K, g, s);
+        if (tiles * 4 <= 2 * 152 && K >= 4 * 64) return tile_launch<4>(A, B, E, M, N, K, g, s);
+    }
+    tile_launch<1>(A, B, E, M, N, K, g, s);
 }
 
 // ---- GEMV for small batches (inference): y[b][o] = sum_i x[b][i] W[o][i] + bias[o]; one warp
@@ -136,7 +262,7 @@ static void linear(int B, int N, int K, const float* x, const __nv_bfloat16* W, 
         EQC_CHECK_LAUNCH();
         count_launch();
     } else {
-        gemm(B, N, K, x, (int64_t)K, (int64_t)1, W, (int64_t)1, (int64_t)K, y, (int64_t)N, bias, yg, s);
+        tile(OpRows<float, true>{x, K}, OpRows<__nv_bfloat16, true>{W, K}, EpLinear{{}, y, N, bias, yg}, B, N, K, s);
     }
 }
 
@@ -166,89 +292,22 @@ __global__ void k_conv_fwd(const float* __restrict__ in, int Cin, int Tin, const
     }
 }
 
-// g_in[b][ci][s] = sum_{co,k : 2t+k-2 = s} W[co][ci][k] g_z[b][co][t]
-__global__ void k_conv_dgrad(const float* __restrict__ gz, int Tout, const __nv_bfloat16* __restrict__ W, int Cin,
-                             float* __restrict__ gin, int Tin, int B) {
-    EQC_GRID_WAIT();
-    const int64_t n = (int64_t)B * Cin * Tin;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {
-        const int s = (int)(idx % Tin);
-        const int ci = (int)((idx / Tin) % Cin);
-        const int b = (int)(idx / ((int64_t)Tin * Cin));
-        float acc = 0.f;
-        const float* gb = gz + (int64_t)b * GN_C * Tout;
-        for (int co = 0; co < GN_C; ++co) {
-#pragma unroll
-            for (int k = 0; k < GN_K; ++k) {
-                const int u = s + 2 - k;
-                if (u >= 0 && (u & 1) == 0 && (u >> 1) < Tout)
-                    acc = fmaf(__bfloat162float(W[((int64_t)co * Cin + ci) * GN_K + k]), gb[(int64_t)co * Tout + (u >> 1)], acc);
-            }
-        }
-        gin[idx] = acc;
-    }
-}
-
-// gW[co][ci][k] = sum_{b,t} g_z[b][co][t] in[b][ci][2t+k-2] ; one CTA per (co, ci)
-__global__ void __launch_bounds__(256) k_conv_wgrad(const float* __restrict__ gz, const float* __restrict__ in, int Cin,
-                                                    int Tin, int Tout, int B, float* __restrict__ gW) {
-    EQC_GRID_WAIT();
-    __shared__ double sh[32];
-    const int co = blockIdx.x / Cin, ci = blockIdx.x % Cin;
-    float acc[GN_K] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int64_t e = threadIdx.x; e < (int64_t)B * Tout; e += blockDim.x) {
-        const int b = (int)(e / Tout), t = (int)(e % Tout);
-        const float g = gz[((int64_t)b * GN_C + co) * Tout + t];
-        const float* ib = in + ((int64_t)b * Cin + ci) * Tin;
-#pragma unroll
-        for (int k = 0; k < GN_K; ++k) {
-            const int s = 2 * t + k - 2;
-            if (s >= 0 && s < Tin) acc[k] = fmaf(g, ib[s], acc[k]);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < GN_K; ++k) {
-        const double v = block_sum((double)acc[k], sh);
-        if (threadIdx.x == 0) gW[((int64_t)co * Cin + ci) * GN_K + k] = (float)v;
-    }
-}
-
-// out[c] = sum over rows r and positions t of g[r][c][t]   (bias gradients; T = 1 for fc)
-__global__ void __launch_bounds__(256) k_bias_grad(const float* __restrict__ g, int B, int Cn, int T, float* __restrict__ out) {
-    EQC_GRID_WAIT();
-    __shared__ double sh[32];
-    const int c = blockIdx.x;
-    double s = 0.0;
-    for (int64_t e = threadIdx.x; e < (int64_t)B * T; e += blockDim.x) {
-        const int b = (int)(e / T), t = (int)(e % T);
-        s += g[((int64_t)b * Cn + c) * T + t];
-    }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) out[c] = (float)s;
-}
-
-// g *= GELU'(z)
-__global__ void k_gelu_bwd(float* __restrict__ g, const float* __restrict__ z, int64_t n) {
-    EQC_GRID_WAIT();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        g[i] *= gelu_grad(z[i]);
-}
-
 // Mean squared error over B x nout: g = 2 (out - tgt) / (B nout); loss[b] = sum_j (out - tgt)^2
 __global__ void __launch_bounds__(256) k_mse(const float* __restrict__ out, const float* __restrict__ tgt, int nout, int B,
                                              float* __restrict__ g, double* __restrict__ loss) {
     EQC_GRID_WAIT();
-    __shared__ double sh[32];
     const int b = blockIdx.x;
     const float sc = 2.f / ((float)B * (float)nout);
-    double s = 0.0;
+    DotAcc<float> acc;   // an error-free product and sum to each entry, in FP32
+#pragma unroll 4
     for (int j = threadIdx.x; j < nout; j += blockDim.x) {
         const float e = out[(int64_t)b * nout + j] - tgt[(int64_t)b * nout + j];
-        g[(int64_t)b * nout + j] = sc * e;
-        s += (double)e * (double)e;
+        g[(int64_t)b * GN_LDOUT + j] = sc * e;
+        acc.add(e, e);
     }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) loss[b] = s;
+    if (threadIdx.x < GN_LDOUT - nout) g[(int64_t)b * GN_LDOUT + nout + threadIdx.x] = 0.f;   // the row's padding
+    block_sum(acc);
+    if (threadIdx.x == 0) loss[b] = acc.value();
 }
 
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -287,7 +346,7 @@ void gn_reserve(GuessNet& g, int batch) {
     g.af1.alloc((size_t)batch * GN_NH);
     g.g_af1.alloc((size_t)batch * GN_NH);
     g.out.alloc((size_t)batch * g.nout);
-    g.g_out.alloc((size_t)batch * g.nout);
+    g.g_out.alloc((size_t)batch * GN_LDOUT);
     g.loss.alloc(batch);
 }
 
@@ -350,10 +409,16 @@ void gn_forward(GuessNet& g, const float* x0, int B, cudaStream_t s) {
     int cin = 2;
     for (int l = 0; l < GN_LAYERS; ++l) {
         const int64_t n = (int64_t)B * GN_C * g.T[l + 1];
-        k_conv_fwd<<<nblk(n), 256, 0, s>>>(in, cin, g.T[l], g.wbf.p + g.off_cw[l], g.master.p + g.off_cb[l], g.z[l].p,
-                                           g.a[l].p, g.T[l + 1], B);
-        EQC_CHECK_LAUNCH();
-        count_launch();
+        const __nv_bfloat16* W = g.wbf.p + g.off_cw[l];
+        const float* bias = g.master.p + g.off_cb[l];
+        if (B <= 4) {
+            k_conv_fwd<<<nblk(n), 256, 0, s>>>(in, cin, g.T[l], W, bias, g.z[l].p, g.a[l].p, g.T[l + 1], B);
+            EQC_CHECK_LAUNCH();
+            count_launch();
+        } else {
+            tile(OpConvW{{}, W, cin * GN_K}, OpConvIn<false>{{}, in, cin, g.T[l], g.T[l + 1]},
+                 EpConv{{}, g.z[l].p, g.a[l].p, bias, g.T[l + 1]}, GN_C, B * g.T[l + 1], cin * GN_K, s);
+        }
         in = g.a[l].p;
         cin = GN_C;
     }
@@ -364,41 +429,45 @@ void gn_forward(GuessNet& g, const float* x0, int B, cudaStream_t s) {
 
 // Gradient of the mean squared error of g.out (after gn_forward on x0) against tgt.
 void gn_backward(GuessNet& g, const float* x0, const float* tgt, int B, cudaStream_t s) {
+    if (!g.w_part.p) {
+        g.w_part.alloc((size_t)GN_WSPLIT * GN_C * GT_N);
+        g.b_part.alloc((size_t)GN_WSPLIT * GN_C);
+    }
     k_mse<<<B, 256, 0, s>>>(g.out.p, tgt, g.nout, B, g.g_out.p, g.loss.p);
     count_launch();
-    // fc2
-    gemm(g.nout, GN_NH, B, g.g_out.p, 1, g.nout, g.af1.p, GN_NH, 1, g.grad.p + g.off_f2w, GN_NH, (const float*)nullptr,
-         (float*)nullptr, s);
-    k_bias_grad<<<g.nout, 256, 0, s>>>(g.g_out.p, B, g.nout, 1, g.grad.p + g.off_f2b);
-    count_launch();
-    gemm(B, GN_NH, g.nout, g.g_out.p, g.nout, 1, g.wbf.p + g.off_f2w, GN_NH, 1, g.g_af1.p, GN_NH,
-         (const float*)nullptr, (float*)nullptr, s);
-    k_gelu_bwd<<<nblk((int64_t)B * GN_NH), 256, 0, s>>>(g.g_af1.p, g.zf1.p, (int64_t)B * GN_NH);
-    count_launch();
-    // fc1
-    const float* a3 = g.a[GN_LAYERS - 1].p;
-    gemm(GN_NH, g.flat, B, g.g_af1.p, 1, GN_NH, a3, g.flat, 1, g.grad.p + g.off_f1w, g.flat, (const float*)nullptr,
-         (float*)nullptr, s);
-    k_bias_grad<<<GN_NH, 256, 0, s>>>(g.g_af1.p, B, GN_NH, 1, g.grad.p + g.off_f1b);
-    count_launch();
-    gemm(B, g.flat, GN_NH, g.g_af1.p, GN_NH, 1, g.wbf.p + g.off_f1w, g.flat, 1, g.g_a[GN_LAYERS - 1].p, g.flat,
-         (const float*)nullptr, (float*)nullptr, s);
-    // convolutions, last to first
-    for (int l = GN_LAYERS - 1; l >= 0; --l) {
-        const int cin = l == 0 ? 2 : GN_C;
-        const int64_t n = (int64_t)B * GN_C * g.T[l + 1];
-        k_gelu_bwd<<<nblk(n), 256, 0, s>>>(g.g_a[l].p, g.z[l].p, n);
+    // fc2: weight and bias, then g_z of fc1
+    tile<false>(OpRows<float, false>{g.g_out.p, GN_LDOUT}, OpRows<float, false>{g.af1.p, GN_NH},
+         EpWeight<false, false>{g.grad.p + g.off_f2w, g.grad.p + g.off_f2b, nullptr, g.nout, GN_NH, {}}, g.nout, GN_NH, B, s);
+    tile(OpRows<float, true>{g.g_out.p, GN_LDOUT}, OpRows<__nv_bfloat16, false>{g.wbf.p + g.off_f2w, GN_NH},
+         EpGeluGrad{{}, g.g_af1.p, g.zf1.p, GN_NH}, B, GN_NH, g.nout, s);
+    // fc1: weight and bias, then g_z of the last convolution
+    constexpr int last = GN_LAYERS - 1;
+    tile<false>(OpRows<float, false>{g.g_af1.p, GN_NH}, OpRows<float, false>{g.a[last].p, g.flat},
+         EpWeight<false, false>{g.grad.p + g.off_f1w, g.grad.p + g.off_f1b, nullptr, GN_NH, g.flat, {}}, GN_NH, g.flat, B, s);
+    tile(OpRows<float, true>{g.g_af1.p, GN_NH}, OpRows<__nv_bfloat16, false>{g.wbf.p + g.off_f1w, g.flat},
+         EpGeluGrad{{}, g.g_a[last].p, g.z[last].p, g.flat}, B, g.flat, GN_NH, s);
+    // convolutions, last to first: weight and bias, then g_z of the layer below
+    for (int l = last; l >= 0; --l) {
+        const int cin = l == 0 ? 2 : GN_C, T = g.T[l + 1], N = cin * GN_K, K = B * T;
         const float* in = l == 0 ? x0 : g.a[l - 1].p;
-        k_conv_wgrad<<<GN_C * cin, 256, 0, s>>>(g.g_a[l].p, in, cin, g.T[l], g.T[l + 1], B, g.grad.p + g.off_cw[l]);
-        k_bias_grad<<<GN_C, 256, 0, s>>>(g.g_a[l].p, B, GN_C, g.T[l + 1], g.grad.p + g.off_cb[l]);
-        count_launch(3);
-        if (l > 0) {
-            const int64_t ni = (int64_t)B * GN_C * g.T[l];
-            k_conv_dgrad<<<nblk(ni), 256, 0, s>>>(g.g_a[l].p, g.T[l + 1], g.wbf.p + g.off_cw[l], GN_C, g.g_a[l - 1].p,
-                                                  g.T[l], B);
-            count_launch();
-        }
+        const int tiles = (N + GT_N - 1) / GT_N;
+        const int chunk = std::max(256, (K / (GN_WSPLIT / tiles) + GT_K) / GT_K * GT_K);
+        const dim3 grid(tiles, 1, (K + chunk - 1) / chunk);
+        const EpWeight<true, true> ep{g.w_part.p, nullptr, g.b_part.p, GN_C, N, {}};
+        k_tile<OpConvGz, OpConvIn<true>, EpWeight<true, true>, 1><<<grid, GT_THREADS, 0, s>>>(
+            OpConvGz{{}, g.g_a[l].p, T}, OpConvIn<true>{{}, in, cin, g.T[l], T}, ep, GN_C, N, K, chunk);
+        k_weight_sum<<<(GN_C * N + GN_C + 31) / 32, 256, 0, s>>>(g.w_part.p, g.b_part.p, grid.z, GN_C, N, g.grad.p + g.off_cw[l],
+                                                           g.grad.p + g.off_cb[l]);
         EQC_CHECK_LAUNCH();
+        count_launch(2);
+        if (l > 0) {
+            const __nv_bfloat16* W = g.wbf.p + g.off_cw[l];
+            const int Ti = g.T[l], U0 = (Ti + 1) / 2, U1 = Ti / 2;
+            tile(OpTapsW<3>{{}, W}, OpTapsGz<3>{{}, g.g_a[l].p, T, U0}, EpConvGrad{{}, g.g_a[l - 1].p, g.z[l - 1].p, Ti, U0, 0}, GN_C,
+                 B * U0, GN_C * 3, s);
+            tile(OpTapsW<2>{{}, W}, OpTapsGz<2>{{}, g.g_a[l].p, T, U1}, EpConvGrad{{}, g.g_a[l - 1].p, g.z[l - 1].p, Ti, U1, 1}, GN_C,
+                 B * U1, GN_C * 2, s);
+        }
     }
 }
 
@@ -566,11 +635,10 @@ __global__ void k_gather_batch(const float* __restrict__ pin, const float* __res
 }
 __global__ void k_sum_loss(const double* __restrict__ loss, int B, double* acc) {
     EQC_GRID_WAIT();
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < B; ++b) s += loss[b];
-        *acc += s;
-    }
+    double s = 0.0;
+    for (int b = threadIdx.x; b < B; b += 32) s += loss[b];
+    s = warp_sum(s);
+    if (threadIdx.x == 0) *acc += s;
 }
 
 struct TrainBufs {
@@ -603,7 +671,7 @@ static void gn_train(Handle& h, int64_t n, int epochs, double lr, int batch, uin
             count_launch();
             gn_forward(g, g.x0.p, batch, s);
             gn_backward(g, g.x0.p, tb.tgt.p, batch, s);
-            k_sum_loss<<<1, 1, 0, s>>>(g.loss.p, batch, tb.acc.p);
+            k_sum_loss<<<1, 32, 0, s>>>(g.loss.p, batch, tb.acc.p);
             count_launch();
             gn_adam(g, lr, s);
         }
@@ -638,7 +706,7 @@ static double gn_eval(Handle& h, int64_t n, float* out_host) {
                                                                        g.x0.p, tb.tgt.p);
         gn_forward(g, g.x0.p, B, s);
         k_mse<<<B, 256, 0, s>>>(g.out.p, tb.tgt.p, nout, B, g.g_out.p, g.loss.p);
-        k_sum_loss<<<1, 1, 0, s>>>(g.loss.p, B, tb.acc.p);
+        k_sum_loss<<<1, 32, 0, s>>>(g.loss.p, B, tb.acc.p);
         count_launch(3);
         if (out_host) g.out.download(out_host + b0 * nout, (size_t)B * nout, s);
         EQC_CUDA(cudaStreamSynchronize(s));

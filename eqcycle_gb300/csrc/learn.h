@@ -14,7 +14,9 @@
 
 namespace eqc {
 
+constexpr int GN_WSPLIT = 4 * 152;   // CTAs of a convolution's weight gradient, at most
 constexpr int GN_C = 64, GN_K = 5, GN_LAYERS = 4, GN_NH = 512, GN_GX = 121, GN_GY = 61;
+constexpr int GN_LDOUT = (GN_GX * GN_GY + 3) / 4 * 4;   // row pitch of g_out
 
 struct GuessNet {
     int Nf = 0;
@@ -29,6 +31,8 @@ struct GuessNet {
     // activations for a batch of up to cap samples
     int cap = 0;
     DBuf<float> x0, z[GN_LAYERS], a[GN_LAYERS], zf1, af1, out, g_out, g_af1, g_a[GN_LAYERS], g_x;
+    DBuf<float> w_part;    // a convolution's weight gradient by split of the batch's positions
+    DBuf<double> b_part;
     // training pairs resident on the device
     DBuf<float> pin, ptgt;
     int64_t npairs = 0;
