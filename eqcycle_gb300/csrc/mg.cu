@@ -176,17 +176,29 @@ __global__ void k_sub(const T* __restrict__ b, const T* t, T* r, int64_t n) {
 }
 // x[cx + k] = sum_j Cinv[k][j] b[cx + j]  (one warp per row).  Accumulates in T: FP32 for the
 // FP32 cycle (a preconditioner; GB300's FP64 rate would make this the slowest kernel of it).
-// The right-hand side is staged in shared memory (DNC entries at a time, zero beyond n); each warp reads
-// its row in 16-byte loads, eight in flight.
-constexpr int DNC = 2048, DN_WARPS = 8;
+// The right-hand side is staged in shared memory (DNC entries at a time, zero beyond n); each warp reads its row
+// in 16-byte loads, asked for before the wait for the kernel that writes b.  FP32: 14 MB at 1,864 unknowns
+// from L2, bound by latency, so 16 loads in flight and four rows to a CTA (5.7 us; eight and eight: 7.3).  FP64:
+// bound by its arithmetic, eight and eight (13.1 us; sixteen and four with two warps to a row: 15.8).
+constexpr int DNC = 2048;
+template <class T> constexpr int DN_WARPS = sizeof(T) == 4 ? 4 : 8;
 template <class T>
-__global__ void __launch_bounds__(32 * DN_WARPS) k_dense_mv(const T* __restrict__ Cinv, const T* __restrict__ b,
-                                                            T* __restrict__ x, int n, int pitch, int off) {
+__global__ void __launch_bounds__(32 * DN_WARPS<T>) k_dense_mv(const T* __restrict__ Cinv, const T* __restrict__ b,
+                                                               T* __restrict__ x, int n, int pitch, int off) {
     __shared__ __align__(16) T bs[DNC];
-    constexpr int V = 16 / (int)sizeof(T), U = 8;
+    constexpr int V = 16 / (int)sizeof(T), U = sizeof(T) == 4 ? 16 : 8;
     struct alignas(16) Vec { T v[V]; };
-    const int lane = threadIdx.x & 31, row = blockIdx.x * DN_WARPS + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, row = blockIdx.x * DN_WARPS<T> + (threadIdx.x >> 5);
     const T* rw = Cinv + (int64_t)min(row, n - 1) * pitch;
+    Vec c[U];
+    auto load = [&](int c0) {
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int j = c0 + (q * 32 + lane) * V;
+            c[q] = j < pitch ? *reinterpret_cast<const Vec*>(rw + j) : Vec{};
+        }
+    };
+    load(0);
     EQC_GRID_WAIT();
     T s[V];
 #pragma unroll
@@ -194,15 +206,10 @@ __global__ void __launch_bounds__(32 * DN_WARPS) k_dense_mv(const T* __restrict_
     for (int c0 = 0; c0 < n; c0 += DNC) {
         const int m = min(DNC, pitch - c0);
         if (c0) __syncthreads();
-        for (int k = threadIdx.x; k < m; k += 32 * DN_WARPS) bs[k] = c0 + k < n ? b[off + c0 + k] : T(0);
+        for (int k = threadIdx.x; k < m; k += 32 * DN_WARPS<T>) bs[k] = c0 + k < n ? b[off + c0 + k] : T(0);
         __syncthreads();
         for (int j0 = 0; j0 < m; j0 += 32 * V * U) {
-            Vec c[U];
-#pragma unroll
-            for (int q = 0; q < U; ++q) {
-                const int j = j0 + (q * 32 + lane) * V;
-                c[q] = j < m ? *reinterpret_cast<const Vec*>(rw + c0 + j) : Vec{};
-            }
+            if (c0 + j0) load(c0 + j0);
 #pragma unroll
             for (int q = 0; q < U; ++q) {
                 const int j = j0 + (q * 32 + lane) * V;
@@ -392,7 +399,7 @@ static void vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) 
     cudaStream_t s = h.stream;
     if (l == L) {  // coarsest: dense solve on rows >= 1 (row 0 of its vectors stays 0)
         StencilLevel& c = m.lev[L - 1];
-        k_dense_mv<T><<<(m.nc + DN_WARPS - 1) / DN_WARPS, 32 * DN_WARPS, 0, s>>>(Sel<T>::C(m), b, x, m.nc, m.nc_pitch, c.cx);
+        k_dense_mv<T><<<(m.nc + DN_WARPS<T> - 1) / DN_WARPS<T>, 32 * DN_WARPS<T>, 0, s>>>(Sel<T>::C(m), b, x, m.nc, m.nc_pitch, c.cx);
         EQC_CHECK_LAUNCH();
         count_launch();
         return;
