@@ -114,11 +114,11 @@ int64_t make_programmatic(cudaGraph_t g) {
     return changed;
 }
 
-void cond_end(Handle& h) {
+void cond_end(Handle& h, bool programmatic) {
     if (h.stream_stack.empty()) throw Error(EQC_E_STATE, "cond_end without cond_begin");
     cudaGraph_t g = nullptr;
     EQC_CUDA(cudaStreamEndCapture(h.stream, &g));
-    if (!h.pdl_off) h.pdl_edges += make_programmatic(g);
+    if (programmatic && !h.pdl_off) h.pdl_edges += make_programmatic(g);
     h.stream = h.stream_stack.back();
     h.stream_stack.pop_back();
 }

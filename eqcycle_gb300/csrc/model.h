@@ -296,9 +296,13 @@ void check_apply_err(Handle& h);
 // unless a kernel upstream of the node sets it).
 cudaGraphConditionalHandle cond_handle(Handle& h, unsigned dflt = 0);
 // Conditional node with handle c on the stream h.stream is capturing; until cond_end,
-// h.stream is the capture stream of the node's body.
+// h.stream is the capture stream of the node's body.  programmatic: its kernels' edges as make_programmatic has
+// them; the CG loop's bodies keep ordinary ones (ms per quasi-static step with and without: 48 x 48 elements
+// 1.50 and 1.40, 120 x 240 1.87 and 1.79, 240 x 480 2.76 and 2.69, 480 x 960 7.36 and 7.22, plain FP64 120 x 240
+// 5.38 and 5.29: the solver's kernels are short, and a waiting one holds the SMs of the one before).  The plain
+// dynamic step gains from them: 73 us against 76 on 61 x 95 elements.
 void cond_begin(Handle& h, cudaGraphConditionalNodeType type, cudaGraphConditionalHandle c);
-void cond_end(Handle& h);
+void cond_end(Handle& h, bool programmatic = true);
 // Ends every capture in progress on the handle's streams and restores h.stream.
 void abort_capture(Handle& h);
 // Turns the edges of graph g between two of this library's kernels, where the second has no

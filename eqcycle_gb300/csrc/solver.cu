@@ -582,11 +582,11 @@ void enqueue_solve(Handle& h, double tol, int maxit, bool graph, bool carry, con
             const int64_t t0 = capture_tally();
             cond_begin(h, cudaGraphCondTypeIf, hc);
             setup_residual_carry(h, guess);
-            cond_end(h);
+            cond_end(h, false);
             const int64_t t1 = capture_tally();
             cond_begin(h, cudaGraphCondTypeIf, hf);
             setup_residual_full(h, mixed);
-            cond_end(h);
+            cond_end(h, false);
             if (h.capturing) {
                 h.capturing->k_carry = t1 - t0;
                 h.capturing->k_full = capture_tally() - t1;
@@ -624,7 +624,7 @@ void enqueue_solve(Handle& h, double tol, int maxit, bool graph, bool carry, con
             const int64_t t1 = capture_tally();
             cond_begin(h, cudaGraphCondTypeIf, hi);
             update_mixed(h, hw, 1);
-            cond_end(h);
+            cond_end(h, false);
             if (h.capturing) {
                 h.capturing->k_update = capture_tally() - t1;
                 h.capturing->k_iter = t1 - t0;
@@ -637,7 +637,7 @@ void enqueue_solve(Handle& h, double tol, int maxit, bool graph, bool carry, con
                 h.capturing->k_bodies += capture_tally() - t0;
             }
         }
-        cond_end(h);
+        cond_end(h, false);
     } else {
         k_cg_init<<<1, 1, 0, h.stream>>>(S, tol, maxit, h.opt.tol_rule, incr_updates(h, mixed), 0, 0);
         count_launch();
