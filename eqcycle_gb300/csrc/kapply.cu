@@ -656,17 +656,24 @@ static_assert(UniTile::OY * UniTile::EX == UNT && UniTile::EY * UniTile::OX <= U
 // Back to back on the damage-zone models, before (both contractions, 8 x 7 tiles) and now: 61 x 95
 // elements 19.4 and 10.4 us, 120 x 240 37.1 and 21.9, 240 x 480 134.2 and 68.6 (122.8 and 60.8 where
 // one x and y stay in L2), 480 x 960 496 and 248: 48 us of the 60.8 are the pipe's.
-// RES: the mixed solver's residual r64 = -K_II x with ResidualOut's work (sign -1, zero_row0).
-template <bool RES>
+// TAIL: NoTail; ResidualOut, the mixed solver's residual r64 = -K_II x with its work (sign -1, zero_row0);
+// DotOut, the CG's x . K x (a launch of its own took 9 us on 120 x 240 elements, the sum here 4).
+struct NoTail {};
+template <class TAIL>
 __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUtensorMap umap,
                                                      const __grid_constant__ CUtensorMap mmap, double* __restrict__ y,
                                                      ApplyArgs<double> A, double sign, int zero_row0, int ntx, int ntiles,
-                                                     OpEpi<double> E, ResidualOut R) {
+                                                     OpEpi<double> E, TAIL R) {
     EQC_GRID_WAIT();
     if (A.gate && *A.gate != A.gate_val) return;
-    const double sg = RES ? R.S->sigma : 0.0;
-    const int es = RES ? R.S->sigma_exp : 0;
-    DotAcc<float> acc;
+    constexpr bool RES = std::is_same_v<TAIL, ResidualOut>, DOT = std::is_same_v<TAIL, DotOut>;
+    double sg = 0.0;
+    int es = 0;
+    if constexpr (RES) {
+        sg = R.S->sigma;
+        es = R.S->sigma_exp;
+    }
+    DotAcc<std::conditional_t<RES, float, double>> acc;
     using UT = UniTile;
     const Layout& L = A.L;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -781,10 +788,14 @@ __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUt
         const bool mine = has_y && er > 0 && ix < L.nx;
         const int64_t o0 = (int64_t)iy0 * L.ld + ix;
         EpiIn<double> in[4];
+        double xin[4];
         if (mine && !RES) {
 #pragma unroll
             for (int l = 0; l < 4; ++l)
-                if (iy0 + l < L.ny) in[l] = epi_load1(E, o0 + (int64_t)l * L.ld);
+                if (iy0 + l < L.ny) {
+                    if constexpr (DOT) xin[l] = E.x[o0 + (int64_t)l * L.ld];
+                    else in[l] = epi_load1(E, o0 + (int64_t)l * L.ld);
+                }
         }
         __syncthreads();   // cy written; every read of this stage and of ys done
         if (threadIdx.x == 0) {
@@ -798,7 +809,10 @@ __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUt
                 if (iy0 + l < L.ny) {
                     const int64_t o = o0 + (int64_t)l * L.ld;
                     const double t = (zero_row0 && iy0 + l == 0) ? 0.0 : v[l];
-                    if constexpr (RES) {
+                    if constexpr (DOT) {
+                        y[o] = t;
+                        acc.add(t, xin[l]);
+                    } else if constexpr (RES) {
                         R.r64[o] = t;
                         R.r32[o] = residual32(t, es, sg, acc);
                     } else {
@@ -808,6 +822,7 @@ __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUt
         }
     }
     if constexpr (RES) residual_done(R, acc);
+    if constexpr (DOT) grid_sum(acc, R.part, R.count, [&](double t) { cg_take_dot(R.S, t, true); });
 }
 
 // ---- element-per-lane version (FP32) --------------------------------------------------------
@@ -1356,29 +1371,33 @@ static int resident_blocks(K kernel, int threads, int bytes) {
 }
 
 // Launch shape of k_apply_uni64: g_uni_sms SMs, at most g_uni_per_sm CTAs on each.
-static int g_uni_sms = 0, g_uni_per_sm[2] = {0, 0};   // [RES]
+static int g_uni_sms = 0;
+template <class TAIL> static int g_uni_per_sm = 0;
 constexpr int UNI_SMEM = 120 * 1024;   // the most a CTA asks for: then one fits an SM
 static void uni_setup() {
     int dev = 0;
     EQC_CUDA(cudaGetDevice(&dev));
     EQC_CUDA(cudaDeviceGetAttribute(&g_uni_sms, cudaDevAttrMultiProcessorCount, dev));
-    g_uni_per_sm[0] = resident_blocks(k_apply_uni64<false>, UNT, UniTile::BYTES) / g_uni_sms;
-    g_uni_per_sm[1] = resident_blocks(k_apply_uni64<true>, UNT, UniTile::BYTES) / g_uni_sms;
-    EQC_CUDA(cudaFuncSetAttribute(k_apply_uni64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, UNI_SMEM));
-    EQC_CUDA(cudaFuncSetAttribute(k_apply_uni64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, UNI_SMEM));
+    auto one = [](auto kernel, int& per_sm) {
+        per_sm = resident_blocks(kernel, UNT, UniTile::BYTES) / g_uni_sms;
+        EQC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, UNI_SMEM));
+    };
+    one(k_apply_uni64<NoTail>, g_uni_per_sm<NoTail>);
+    one(k_apply_uni64<ResidualOut>, g_uni_per_sm<ResidualOut>);
+    one(k_apply_uni64<DotOut>, g_uni_per_sm<DotOut>);
 }
 // The FP64 pipe of each SM bounds the kernel, so its CTAs have to be spread evenly: per SM no more than
 // an even spread of the tiles needs, kept to that by the shared memory that a CTA asks for.  (A
 // programmatic launch otherwise fills the SMs that its predecessor leaves empty with several CTAs
 // each: 26 us instead of 16 back to back on 61 x 95 elements.)
+template <class TAIL = NoTail>
 static void launch_uni64(const CUtensorMap& um, double* y, const ApplyArgs<double>& A, double sign, int zr,
-                         cudaStream_t s, const OpEpi<double>& E = OpEpi<double>(), const ResidualOut* R = nullptr) {
+                         cudaStream_t s, const OpEpi<double>& E = OpEpi<double>(), const TAIL& R = TAIL()) {
     const int ntx = A.L.NelX / UEX + 1, ntiles = ntx * (A.L.NelY / UEY + 1);
-    const int per_sm = std::min(g_uni_per_sm[R != nullptr], (ntiles + g_uni_sms - 1) / g_uni_sms);
+    const int per_sm = std::min(g_uni_per_sm<TAIL>, (ntiles + g_uni_sms - 1) / g_uni_sms);
     const int smem = std::max(UniTile::BYTES, std::min(UNI_SMEM, 228 * 1024 / (per_sm + 1) / 128 * 128 + 128));
     const int grid = std::min(ntiles, per_sm * g_uni_sms);
-    if (R) k_apply_uni64<true><<<grid, UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles, E, *R);
-    else k_apply_uni64<false><<<grid, UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles, E, ResidualOut());
+    k_apply_uni64<TAIL><<<grid, UNT, smem, s>>>(um, A.tma->mu, y, A, sign, zr, ntx, ntiles, E, R);
     EQC_CHECK_LAUNCH();
     count_launch();
 }
@@ -1580,11 +1599,21 @@ bool apply_K_epi(const double* x, const ApplyArgs<double>& A, int mode, const Op
     return true;
 }
 
+bool apply_K_dot(const double* x, double* y, const ApplyArgs<double>& A, const DotOut& dot, cudaStream_t s) {
+    if (!A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
+    const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
+    if (!uu) return false;
+    OpEpi<double> E;
+    E.x = x;
+    launch_uni64(*uu, y, A, 1.0, 1, s, E, dot);
+    return true;
+}
+
 bool apply_K_residual(const double* x, const ApplyArgs<double>& A, const ResidualOut& R, cudaStream_t s) {
     if (!A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
     const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
     if (!uu) return false;
-    launch_uni64(*uu, nullptr, A, -1.0, 1, s, OpEpi<double>(), &R);
+    launch_uni64(*uu, nullptr, A, -1.0, 1, s, OpEpi<double>(), R);
     return true;
 }
 

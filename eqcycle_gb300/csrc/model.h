@@ -262,6 +262,12 @@ inline bool df_pays(const Layout& L) { return (int64_t)L.NelX * L.NelY >= 32000;
 // straight into the residual (y and sign unused).  False when unavailable.
 bool apply_K_df(Handle& h, const double* x, double* y, double sign, int mode, cudaStream_t s,
                 const int* gate = nullptr, int gate_val = 0, const ResidualOut* R = nullptr);
+// Where an FP64 apply's launch leaves x . K x for the CG (cg_take_dot).
+struct DotOut {
+    double* part = nullptr;
+    unsigned* count = nullptr;
+    CGState* S = nullptr;
+};
 // r64 = -K_II x in FP64 with ResidualOut's work in the launch; false when the FP64 apply in use has none.
 bool apply_K_residual(const double* x, const ApplyArgs<double>& A, const ResidualOut& R, cudaStream_t s);
 void tma_init_for(TmaCache& c, const Layout& L, const float* W32p, const double* W64p, const double* mu);
@@ -269,6 +275,8 @@ void tma_init_for(TmaCache& c, const Layout& L, const float* W32p, const double*
 // (residual or Chebyshev step) instead of stored; false when the selected kernel has none.
 bool apply_K_epi(const float* x, const ApplyArgs<float>& A, int mode, const OpEpi<float>& E, cudaStream_t s);
 bool apply_K_epi(const double* x, const ApplyArgs<double>& A, int mode, const OpEpi<double>& E, cudaStream_t s);
+// y = K_II x with DotOut's sum in the launch; false when the FP64 apply in use has none.
+bool apply_K_dot(const double* x, double* y, const ApplyArgs<double>& A, const DotOut& dot, cudaStream_t s);
 // y = K x (FP32) on the node rows 0..3 of the fault's element row, by the element-per-lane
 // arithmetic of the full FP32 applies (variants 0 and 4-8): row 0 has the bits of their row 0.
 // False when the padded element data or 16-byte aligned vectors are missing.

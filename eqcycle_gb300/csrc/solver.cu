@@ -452,15 +452,22 @@ static void iter_fp64(Handle& h, cudaGraphConditionalHandle hw, int use_cond) {
     else jacobi(h, r, h.diag64.p, z, n);
     k_dot_cg<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(z, r, n, h.red_part.p, h.red_count.p, S, 0);
     k_pupdate<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(z, u, n, S);
-    apply_K<double>(h.p64.p, h.q64.p, args64(h), 1.0, 1, h.stream);
-    k_dot_cg<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(u, q, n, h.red_part.p, h.red_count.p, S, 1);
+    DotOut dot;   // u.q
+    dot.part = h.red_part.p;
+    dot.count = h.red_count.p;
+    dot.S = S;
+    if (!apply_K_dot(h.p64.p, h.q64.p, args64(h), dot, h.stream)) {
+        apply_K<double>(h.p64.p, h.q64.p, args64(h), 1.0, 1, h.stream);
+        k_dot_cg<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(u, q, n, h.red_part.p, h.red_count.p, S, 1);
+        count_launch();
+    }
     CheckA ck;
     ck.on = 2;
     ck.use_cond = use_cond;
     ck.hw = hw;
     k_xr_update<double><<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(x, r, u, nullptr, q, n, h.red_part.p, h.red_count.p, S, ck);
     EQC_CHECK_LAUNCH();
-    count_launch(4);
+    count_launch(3);
 }
 
 // Mixed precision: FP32 recurrences of one iteration, ending with the update decision (hi) and,
