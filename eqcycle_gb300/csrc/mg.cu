@@ -585,14 +585,13 @@ static double estimate_lmax(Handle& h, int l) {
         level_apply<double>(h, l, w.x64.p, w.t64.p);
         k_mul<double><<<vb(n), 256, 0, h.stream>>>(Dinv, w.t64.p, n);
         dot64(h, w.t64.p, w.t64.p, n, h.scal.p + 14);
-        dot64(h, w.x64.p, w.t64.p, n, h.scal.p + 13);
-        dot64(h, w.x64.p, w.x64.p, n, h.scal.p + 12);
-        double sc[3];
-        EQC_CUDA(cudaMemcpyAsync(sc, h.scal.p + 12, sizeof(double) * 3, cudaMemcpyDeviceToHost, h.stream));
+        dot64(h, w.x64.p, w.x64.p, n, h.scal.p + 13);
+        double sc[2];
+        EQC_CUDA(cudaMemcpyAsync(sc, h.scal.p + 13, sizeof(double) * 2, cudaMemcpyDeviceToHost, h.stream));
         EQC_CUDA(cudaStreamSynchronize(h.stream));
-        lam = std::sqrt(sc[2] / sc[0]);
+        lam = std::sqrt(sc[1] / sc[0]);
         EQC_CUDA(cudaMemcpyAsync(w.x64.p, w.t64.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, h.stream));
-        k_scale<double><<<vb(n), 256, 0, h.stream>>>(w.x64.p, n, 1.0 / std::sqrt(sc[2]));
+        k_scale<double><<<vb(n), 256, 0, h.stream>>>(w.x64.p, n, 1.0 / std::sqrt(sc[1]));
         count_launch(2);
     }
     EQC_CHECK_LAUNCH();
