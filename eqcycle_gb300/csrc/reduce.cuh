@@ -34,7 +34,7 @@ __device__ __forceinline__ void block_sum(Acc& acc) {
     if (w == 0) {
         acc = Acc();
         if (lane < nw) acc.merge(sh[lane]);
-        acc.warp_sum();
+        acc.warp_sum(nw);
     }
     __syncthreads();
 }

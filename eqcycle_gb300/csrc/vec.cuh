@@ -44,6 +44,7 @@ __device__ __forceinline__ void st4(double* p, const double (&a)[4]) {
 // FP64-class dot products of FP32 vectors without FP64 arithmetic before the total (an FP64
 // instruction holds an SM's FP64 pipe for 16 clocks per warp and its result comes late: with FP64 sums
 // of the warps, the CTA and the CTAs' partials a reduction's tail took 5 us of every launch).
+// warp_sum: into lane 0, of the first `lanes` lanes (the others hold zero).
 template <class T> struct DotAcc;
 template <> struct DotAcc<double> {
     using Part = double;   // what crosses warps and CTAs
@@ -52,9 +53,10 @@ template <> struct DotAcc<double> {
     __device__ __forceinline__ Part part() const { return s; }
     __device__ __forceinline__ void merge(Part p) { s += p; }
     __device__ __forceinline__ double value() const { return s; }
-    __device__ __forceinline__ void warp_sum() {
+    __device__ __forceinline__ void warp_sum(int lanes = 32) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        for (int o = 16; o > 0; o >>= 1)
+            if (o < lanes) s += __shfl_down_sync(0xffffffffu, s, o);
     }
 };
 template <> struct DotAcc<float> {
@@ -73,13 +75,14 @@ template <> struct DotAcc<float> {
         fast_two_sum(hi, e, s, lo);
         hi = s;
     }
-    __device__ __forceinline__ void warp_sum() {
+    __device__ __forceinline__ void warp_sum(int lanes = 32) {
         float s, e;
         two_sum(hi, lo, s, e);   // a proper pair first
         hi = s;
         lo = e;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
+            if (o >= lanes) continue;
             const float h = __shfl_down_sync(0xffffffffu, hi, o), l = __shfl_down_sync(0xffffffffu, lo, o);
             add_pair(h, l);
         }
