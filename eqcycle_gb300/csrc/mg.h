@@ -55,7 +55,6 @@ struct MGHier {
     int nc = 0, nc_pitch = 0;         // coarsest dense size, row pitch of its inverse
     DBuf<double> Cinv64;
     DBuf<float> Cinv32;
-    int64_t launches_per_vcycle = 0;
 };
 
 // host setup helpers (mg_setup.cpp)
