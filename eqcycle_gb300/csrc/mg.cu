@@ -57,25 +57,11 @@ __global__ void __launch_bounds__(VTX * VTY) k_stencil2(const T* __restrict__ A,
     out[i] = cheb_x_pt<T>(x1, xi, bi, t, di, c1b, c2b);
 }
 
-// bc = P^T r on coarse rows >= 1 (row 0 = 0), with the coarse level's first smoothing step, for a tile of
-// RCX x RCY coarse points.  One thread per fine point of the tile brings the residual r into shared
-// memory: stored by a separate launch (LdPlain), or formed here from the fine operator (LdResidual),
-// which saves that launch and r's store and load; the coarse points then sum their 3 x 3 fine points.
 constexpr int RCX = 15, RCY = 3, RFX = 2 * RCX + 1, RFY = 2 * RCY + 1;
-template <class T, class Ld>
-__global__ void __launch_bounds__(RFX * RFY) k_restrict(Ld rf, T* __restrict__ bc, Coarsen X, Coarsen Y, ChebFirst<T> F) {
-    EQC_GRID_WAIT();
-    __shared__ T rs[RFY][RFX];
-    const int tx = threadIdx.x % RFX, ty = threadIdx.x / RFX;
-    const int cx0 = blockIdx.x * RCX, cy0 = blockIdx.y * RCY;
-    const int fx = min(max(2 * cx0 - 1 + tx, 0), X.nf - 1), fy = min(max(2 * cy0 - 1 + ty, 0), Y.nf - 1);
-    const int cxi = cx0 + threadIdx.x % RCX, cyi = cy0 + threadIdx.x / RCX;
-    const bool mine = threadIdx.x < RCX * RCY && cxi < X.nc && cyi < Y.nc;
-    const int64_t o = (int64_t)cyi * X.nc + cxi;
-    const T di = mine && F.dinv ? F.dinv[o] : T(0);
-    rs[ty][tx] = rf(fx, fy);
-    __syncthreads();
-    if (!mine) return;
+// The sum over a coarse point's 3 x 3 fine points (rs: the tile's residual, RFX x RFY from (2 cx0 - 1, 2 cy0 - 1)).
+template <class T>
+__device__ __forceinline__ T restrict_tile(const T (&rs)[RFY][RFX], const Coarsen& X, const Coarsen& Y, int cxi, int cyi,
+                                           int cx0, int cy0) {
     T s = T(0);
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -90,8 +76,80 @@ __global__ void __launch_bounds__(RFX * RFY) k_restrict(Ld rf, T* __restrict__ b
         }
         s = fma_rn<T>(gy == 0 || cyi == 0 ? T(0) : w, sx, s);
     }
+    return s;
+}
+
+// bc = P^T r on coarse rows >= 1 (row 0 = 0), with the coarse level's first smoothing step, for a tile of
+// RCX x RCY coarse points.  One thread per fine point of the tile brings the residual r into shared
+// memory: stored by a separate launch (LdPlain), or formed here from the fine operator (LdResidual),
+// which saves that launch and r's store and load; the coarse points then sum their 3 x 3 fine points.
+template <class T, class Ld>
+__global__ void __launch_bounds__(RFX * RFY) k_restrict(Ld rf, T* __restrict__ bc, Coarsen X, Coarsen Y, ChebFirst<T> F) {
+    EQC_GRID_WAIT();
+    __shared__ T rs[RFY][RFX];
+    const int tx = threadIdx.x % RFX, ty = threadIdx.x / RFX;
+    const int cx0 = blockIdx.x * RCX, cy0 = blockIdx.y * RCY;
+    const int fx = min(max(2 * cx0 - 1 + tx, 0), X.nf - 1), fy = min(max(2 * cy0 - 1 + ty, 0), Y.nf - 1);
+    const int cxi = cx0 + threadIdx.x % RCX, cyi = cy0 + threadIdx.x / RCX;
+    const bool mine = threadIdx.x < RCX * RCY && cxi < X.nc && cyi < Y.nc;
+    const int64_t o = (int64_t)cyi * X.nc + cxi;
+    const T di = mine && F.dinv ? F.dinv[o] : T(0);
+    rs[ty][tx] = rf(fx, fy);
+    __syncthreads();
+    if (!mine) return;
+    const T s = restrict_tile<T>(rs, X, Y, cxi, cyi, cx0, cy0);
     bc[o] = s;
     if (F.dinv) F.x[o] = cheb_first_pt<T>(di, s, F.inv_theta);
+}
+
+// Steps 1 and 2 of the pre-smoothing (k_stencil2 from x1 with the iterate before it 0), the residual of their
+// result x3 and its restriction (k_restrict) in one launch: each stage on a ring fewer of the tile's fine
+// points, in shared memory.  x3 is stored too, each point by one tile.  3.2 us on 49 x 49 points, where the two
+// launches take 2.7 and 2.9: a launch's latency is what a vertex level costs, not the ring's points done twice.
+constexpr int RPX = RFX + 4, RPY = RFY + 4;
+template <class T>
+__global__ void __launch_bounds__(RPX * RPY) k_smooth_restrict(const T* __restrict__ A, const T* __restrict__ b,
+                                                               const T* __restrict__ dinv, const T* __restrict__ x1,
+                                                               T* __restrict__ x3, T* __restrict__ bc, Coarsen X, Coarsen Y,
+                                                               T c1a, T c2a, T c1b, T c2b, ChebFirst<T> F) {
+    EQC_GRID_WAIT();
+    __shared__ T xs[2][RPY][RPX];
+    __shared__ T rs[RFY][RFX];
+    const int cx = X.nf, cy = Y.nf;
+    const int tx = threadIdx.x % RPX, ty = threadIdx.x / RPX;
+    const int cx0 = blockIdx.x * RCX, cy0 = blockIdx.y * RCY;
+    const int fx = 2 * cx0 - 3 + tx, fy = 2 * cy0 - 3 + ty;
+    const int ix = min(max(fx, 0), cx - 1), iy = min(max(fy, 0), cy - 1);
+    const int64_t i = (int64_t)iy * cx + ix;
+    const int cxi = cx0 + threadIdx.x % RCX, cyi = cy0 + threadIdx.x / RCX;
+    const bool coarse = threadIdx.x < RCX * RCY && cxi < X.nc && cyi < Y.nc;
+    const int64_t o = (int64_t)cyi * X.nc + cxi;
+    T a[9], v[9];
+    stencil_row<T>(A, cx, cy, ix, iy, a);
+    const LdPlain<T> ld{x1, cx};
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        v[k] = ld(min(max(ix + (k % 3) - 1, 0), cx - 1), min(max(iy + (k / 3) - 1, 1), cy - 1));
+    const T bi = b[i], di = dinv[i], xi = x1[i], dc = coarse && F.dinv ? F.dinv[o] : T(0);
+    const T x2 = cheb_x_pt<T>(xi, T(0), bi, stencil_sum<T>(a, iy, [&](int k) { return v[k]; }), di, c1a, c2a);
+    xs[0][ty][tx] = x2;
+    __syncthreads();
+    const bool in1 = tx >= 1 && tx < RPX - 1 && ty >= 1 && ty < RPY - 1, in2 = tx >= 2 && tx < RPX - 2 && ty >= 2 && ty < RPY - 2;
+    if (in1) {
+        const T t = stencil_sum<T>(a, iy, [&](int k) { return xs[0][ty + k / 3 - 1][tx + k % 3 - 1]; });
+        const T y = cheb_x_pt<T>(x2, xi, bi, t, di, c1b, c2b);
+        xs[1][ty][tx] = y;
+        if (fx >= 2 * cx0 && fx < 2 * (cx0 + RCX) && fx < cx && fy >= 2 * cy0 && fy < 2 * (cy0 + RCY) && fy < cy) x3[i] = y;
+    }
+    __syncthreads();
+    if (in2)
+        rs[ty - 2][tx - 2] =
+            sub_rn<T>(bi, stencil_sum<T>(a, iy, [&](int k) { return xs[1][ty + k / 3 - 1][tx + k % 3 - 1]; }));
+    __syncthreads();
+    if (!coarse) return;
+    const T s = restrict_tile<T>(rs, X, Y, cxi, cyi, cx0, cy0);
+    bc[o] = s;
+    if (F.dinv) F.x[o] = cheb_first_pt<T>(dc, s, F.inv_theta);
 }
 
 // xf = x + P xc on every row (row 0: x)
@@ -132,6 +190,36 @@ __global__ void __launch_bounds__(VTX * VTY) k_prolong_smooth(const T* __restric
     const T t = stencil_sum<T>(a, iy, [&](int k) { return xs[ty + k / 3 - 1][tx + k % 3 - 1]; });
     if (xf) xf[i] = xi;
     out[i] = cheb_x_pt<T>(xi, xi, bi, t, di, T(0), inv_theta);
+}
+
+// The prolongation and three post-smoothing steps in one launch (k_prolong_smooth, then k_stencil2 on its result):
+// each stage on a ring fewer of the tile's points, in shared memory.  2.9 us on 49 x 49 points, 2.7 and 2.7 apart.
+constexpr int PSX = 32, PSY = 16;
+template <class T>
+__global__ void __launch_bounds__(PSX * PSY) k_prolong_smooth3(const T* __restrict__ A, const T* __restrict__ b,
+                                                               const T* __restrict__ dinv, T* __restrict__ out,
+                                                               LdProlonged<T> P, T inv_theta, T c1a, T c2a, T c1b, T c2b) {
+    EQC_GRID_WAIT();
+    __shared__ T xs[2][PSY][PSX];
+    const int cx = P.X.nf, cy = P.Y.nf;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int fx = blockIdx.x * (PSX - 6) - 3 + tx, fy = blockIdx.y * (PSY - 6) - 3 + ty;
+    const int ix = min(max(fx, 0), cx - 1), iy = min(max(fy, 0), cy - 1);
+    const int64_t i = (int64_t)iy * cx + ix;
+    T a[9];
+    const T bi = b[i], di = dinv[i];
+    stencil_row<T>(A, cx, cy, ix, iy, a);
+    const int ring = min(min(tx, PSX - 1 - tx), min(ty, PSY - 1 - ty));
+    const T x0 = iy == 0 ? P.x[i] : P(ix, iy);
+    xs[0][ty][tx] = x0;
+    __syncthreads();
+    auto at = [&](int s) { return stencil_sum<T>(a, iy, [&](int k) { return xs[s][ty + k / 3 - 1][tx + k % 3 - 1]; }); };
+    T y1 = T(0), y2 = T(0);
+    if (ring >= 1) xs[1][ty][tx] = y1 = cheb_x_pt<T>(x0, x0, bi, at(0), di, T(0), inv_theta);
+    __syncthreads();
+    if (ring >= 2) xs[0][ty][tx] = y2 = cheb_x_pt<T>(y1, x0, bi, at(1), di, c1a, c2a);
+    __syncthreads();
+    if (ring >= 3 && fx < cx && fy < cy) out[i] = cheb_x_pt<T>(y2, y1, bi, at(0), di, c1b, c2b);
 }
 
 // ---- transfers between the spectral-element grid and the element-vertex grid ----------
@@ -467,10 +555,11 @@ static void vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) 
         count_launch();
     }
     const bool four = V.deg == 4;
-    if (V.pairs) {
-        cheb_pair<T>(h, l, V.post1, nullptr, four ? V.pre : nullptr, four ? V.post0 : V.pre, b, cc1.data(), cc2.data());
-        if (four) cheb_step<T>(h, l, V.post0, V.pre, false, V.pre, b, (T)cc1[3], (T)cc2[3]);
-    } else {
+    const bool three = V.pairs && V.deg == 3;
+    if (four && V.pairs) {
+        cheb_pair<T>(h, l, V.post1, nullptr, V.pre, V.post0, b, cc1.data(), cc2.data());
+        cheb_step<T>(h, l, V.post0, V.pre, false, V.pre, b, (T)cc1[3], (T)cc2[3]);
+    } else if (!three) {
         for (int k = 1; k < V.deg; ++k)
             cheb_step<T>(h, l, V.pre_iter(k), k > 1 ? V.pre_iter(k - 1) : nullptr, k == 1, V.pre_iter(k + 1), b, (T)cc1[k],
                          (T)cc2[k]);
@@ -491,7 +580,11 @@ static void vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) 
     }
     const dim3 cgrid((lc.cx + RCX - 1) / RCX, (lc.cy + RCY - 1) / RCY);
     const Coarsen X = {l > 0 ? m.lev[l - 1].cx : 0, lc.cx}, Y = {l > 0 ? m.lev[l - 1].cy : 0, lc.cy};   // vertex levels
-    if (l > 0 && h.fuse) {
+    if (three) {
+        StencilLevel& lev = m.lev[l - 1];
+        k_smooth_restrict<T><<<cgrid, RPX * RPY, 0, s>>>(Sel<T>::A(lev), b, Sel<T>::Di(lev), V.post1, V.pre, bc, X, Y, (T)cc1[1],
+                                                         (T)cc2[1], (T)cc1[2], (T)cc2[2], F);
+    } else if (l > 0 && h.fuse) {
         StencilLevel& lev = m.lev[l - 1];
         k_restrict<T><<<cgrid, RFX * RFY, 0, s>>>(LdResidual<T>{Sel<T>::A(lev), V.pre, b, lev.cx, lev.cy}, bc, X, Y, F);
     } else {
@@ -514,6 +607,15 @@ static void vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) 
     EQC_CHECK_LAUNCH();
     vcycle<T>(h, l + 1, xc, bc, l + 1 < L);
     // prolongation and post-smoothing
+    if (three) {
+        StencilLevel& lev = m.lev[l - 1];
+        k_prolong_smooth3<T><<<dim3((lev.cx + PSX - 7) / (PSX - 6), (lev.cy + PSY - 7) / (PSY - 6)), dim3(PSX, PSY), 0, s>>>(
+            Sel<T>::A(lev), b, Sel<T>::Di(lev), x, LdProlonged<T>{V.pre, xc, X, Y}, inv_theta, (T)cc1[1], (T)cc2[1], (T)cc1[2],
+            (T)cc2[2]);
+        EQC_CHECK_LAUNCH();
+        count_launch();
+        return;
+    }
     if (l > 0 && h.fuse) {
         StencilLevel& lev = m.lev[l - 1];
         k_prolong_smooth<T><<<dim3((lev.cx + VTX - 3) / (VTX - 2), (lev.cy + VTY - 3) / (VTY - 2)), dim3(VTX, VTY), 0, s>>>(
@@ -531,9 +633,9 @@ static void vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) 
         cheb_step<T>(h, l, V.post0, nullptr, false, V.post1, b, T(0), inv_theta);
     }
     EQC_CHECK_LAUNCH();
-    if (V.pairs) {   // the first iterate is in r; the last goes to x, which is post0 for four steps and post1 for three
-        cheb_pair<T>(h, l, Sel<T>::r(w), V.post0, four ? V.post1 : nullptr, four ? V.pre : V.post1, b, cc1.data(), cc2.data());
-        if (four) cheb_step<T>(h, l, V.pre, V.post1, false, V.post0, b, (T)cc1[3], (T)cc2[3]);
+    if (V.pairs) {   // four steps: the first iterate is in r, the last goes to post0, which is x
+        cheb_pair<T>(h, l, Sel<T>::r(w), V.post0, V.post1, V.pre, b, cc1.data(), cc2.data());
+        cheb_step<T>(h, l, V.pre, V.post1, false, V.post0, b, (T)cc1[3], (T)cc2[3]);
         return;
     }
     for (int k = 1; k < V.deg; ++k) {   // iterate k in post1 (k odd) or post0, the one before it in the other
