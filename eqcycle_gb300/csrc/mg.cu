@@ -555,10 +555,13 @@ static void vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) 
         count_launch();
     }
     const bool four = V.deg == 4;
-    const bool three = V.pairs && V.deg == 3;
-    if (four && V.pairs) {
-        cheb_pair<T>(h, l, V.post1, nullptr, V.pre, V.post0, b, cc1.data(), cc2.data());
-        cheb_step<T>(h, l, V.post0, V.pre, false, V.pre, b, (T)cc1[3], (T)cc2[3]);
+    // three steps with the transfer in one launch; in FP64, whose operations on the rings cost more than a launch on
+    // large levels (ms per step of the plain method with them and without: 120 x 240 elements, levels up to
+    // 29,161 points, 5.05 and 5.08; 240 x 480, up to 116,161, 13.24 and 13.10; 480 x 960 31.4 and 31.0)
+    const bool three = V.pairs && V.deg == 3 && (sizeof(T) == 4 || n <= 40000);
+    if (V.pairs && !three) {
+        cheb_pair<T>(h, l, V.post1, nullptr, four ? V.pre : nullptr, four ? V.post0 : V.pre, b, cc1.data(), cc2.data());
+        if (four) cheb_step<T>(h, l, V.post0, V.pre, false, V.pre, b, (T)cc1[3], (T)cc2[3]);
     } else if (!three) {
         for (int k = 1; k < V.deg; ++k)
             cheb_step<T>(h, l, V.pre_iter(k), k > 1 ? V.pre_iter(k - 1) : nullptr, k == 1, V.pre_iter(k + 1), b, (T)cc1[k],
@@ -633,9 +636,9 @@ static void vcycle(Handle& h, int l, T* x, const T* b, bool first_done = false) 
         cheb_step<T>(h, l, V.post0, nullptr, false, V.post1, b, T(0), inv_theta);
     }
     EQC_CHECK_LAUNCH();
-    if (V.pairs) {   // four steps: the first iterate is in r, the last goes to post0, which is x
-        cheb_pair<T>(h, l, Sel<T>::r(w), V.post0, V.post1, V.pre, b, cc1.data(), cc2.data());
-        cheb_step<T>(h, l, V.pre, V.post1, false, V.post0, b, (T)cc1[3], (T)cc2[3]);
+    if (V.pairs) {   // the first iterate is in r; the last goes to x, which is post0 for four steps and post1 for three
+        cheb_pair<T>(h, l, Sel<T>::r(w), V.post0, four ? V.post1 : nullptr, four ? V.pre : V.post1, b, cc1.data(), cc2.data());
+        if (four) cheb_step<T>(h, l, V.pre, V.post1, false, V.post0, b, (T)cc1[3], (T)cc2[3]);
         return;
     }
     for (int k = 1; k < V.deg; ++k) {   // iterate k in post1 (k odd) or post0, the one before it in the other

@@ -1,6 +1,6 @@
 """Two smoothing steps of a vertex level in one launch (k_stencil2) against one launch each (EQC_NO_FUSE): the same
-bits, on vertex grids around the edges of its 30 x 6-point tiles, for three and four steps (one pair, and a pair and
-a single step) in both precisions."""
+bits, on vertex grids around the edges of its 30 x 6-point tiles, for three and four steps (three with the transfer in
+one launch, a pair and a single step) in both precisions; the last grid's 40,401 points take the pair in FP64."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision,variant", [(EQC_FP64, 0), (EQC_MIXED, 8)], ids=["fp64", "mixed"])
 @pytest.mark.parametrize("degc", [3, 4])
-@pytest.mark.parametrize("nelx,nely", [(29, 23), (30, 24), (31, 29), (59, 36)])
+@pytest.mark.parametrize("nelx,nely", [(29, 23), (30, 24), (31, 29), (59, 36), (200, 200)])
 def test_pairs_equal_single_steps(eqclib, monkeypatch, nelx, nely, degc, precision, variant):
     cfg = preset("dz480").replace(NelX=nelx, NelY=nely, LY=24e3 * nely / nelx)
     P = set_parameters(cfg)
