@@ -18,7 +18,7 @@
 //   k_apply_pipe   the same pipeline with both contractions of every line (variant 3, and the K d
 //                  refresh of the mixed method's dynamic steps);
 //                  k_apply_tma / k_apply_lines: one tile per CTA (1, 2);
-//   k_apply        the strip modes 2 and 3 (first element row only).
+//   k_strip        the strip modes 2 and 3 (first element row only).
 // The FP32 element kernels take an epilogue (epi.cuh) that finishes the V-cycle's residual or
 // Chebyshev step at each owned node.
 #include "model.h"
@@ -45,124 +45,73 @@ template <> __device__ __forceinline__ float Hc<float>(int i, int j) { return cH
 // mode 2: fault strip: only element row 0, x rows > 0 read as zero, rows 1..4 written
 //         (y_I = K_IF x_F, the right-hand side of the quasi-static solve)
 // mode 3: fault strip: only element row 0, row 0 written (fault traction (K d)[iFlt])
-template <class T, int TEX, int TEY>
-__global__ void __launch_bounds__(256) k_apply(const T* __restrict__ x, T* __restrict__ y, ApplyArgs<T> A,
-                                               T sign, int mode) {
+//
+// The strip modes: a thread forms one node column's share of one element (STX elements and the one left of
+// them, five columns each), then the columns' nodes sum their one or two elements.  Latency bounds it: every
+// thread's loads are independent and its two contractions one chain of FMAs, the x-line of row 0 formed
+// again by each of its nodes (mode 3).  240 element columns: 8.0 us as lines through shared
+// memory, now 4.2 (mode 2) and 5.6 (mode 3), with the same bits.
+constexpr int STX = 8, ST_THREADS = 64;
+template <class T, int MODE>
+__global__ void __launch_bounds__(ST_THREADS) k_strip(const T* __restrict__ x, T* __restrict__ y, ApplyArgs<T> A, T sign) {
     EQC_GRID_WAIT();
     if (A.gate && *A.gate != A.gate_val) return;
+    constexpr int ROWS = MODE == 2 ? 4 : 1, ROW0 = MODE == 2 ? 1 : 0;
+    __shared__ T part[ROWS][5 * (STX + 1)];
     const Layout L = A.L;
-    const bool strip = mode >= 2;
-    const int ex0 = blockIdx.x * TEX;
-    const int ey0 = strip ? 0 : blockIdx.y * TEY;
-    const int exs = max(ex0 - 1, 0), exe = min(ex0 + TEX, L.NelX);
-    const int eys = strip ? 0 : max(ey0 - 1, 0);
-    const int eye = strip ? 1 : min(ey0 + TEY, L.NelY);
-    const int nex = exe - exs, ney = eye - eys, nE = nex * ney;
-    const int tnx = 4 * nex + 1, tny = 4 * ney + 1;
-    const int ix0 = 4 * exs, iy0 = 4 * eys;
-
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* us = reinterpret_cast<T*>(smem_raw);
-    constexpr int USZ = (4 * (TEX + 1) + 1) * (4 * (TEY + 1) + 1);
-    constexpr int ESZ = (TEX + 1) * (TEY + 1) * 25;
-    T* Ws = us + USZ;
-    T* yl = Ws + ESZ;
-
-    for (int k = threadIdx.x; k < tnx * tny; k += blockDim.x) {
-        const int a = k % tnx, b = k / tnx;
-        T v = x[(int64_t)(iy0 + b) * L.ld + ix0 + a];
-        if (mode == 2 && (iy0 + b) > 0) v = T(0);
-        us[k] = v;
-    }
-    for (int k = threadIdx.x; k < nE * 25; k += blockDim.x) {
-        const int le = k / 25, q = k - 25 * le;
-        const int lex = le % nex, ley = le / nex;
-        Ws[k] = A.W[((int64_t)(eys + ley) * L.NelX + exs + lex) * 25 + q];
-    }
-    __syncthreads();
-
-    // x-lines: for element le and GLL row j, contract along xi.
-    for (int t = threadIdx.x; t < nE * 5; t += blockDim.x) {
-        const int le = t / 5, j = t - 5 * le;
-        const int lex = le % nex, ley = le / nex;
-        const T* ul = us + (4 * ley + j) * tnx + 4 * lex;
-        const T* w = Ws + le * 25;
-        T u[5], s[5];
+    const int ex0 = blockIdx.x * STX, t = threadIdx.x, ex = ex0 - 1 + t / 5, i = t % 5;
+    if (t < 5 * (STX + 1) && ex >= 0 && ex < L.NelX) {
+        const T* w = A.W + (int64_t)ex * 25;
+        const T* u = x + 4 * ex;
+        T v[5], wy[5], c[5], wx[5];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) u[k] = ul[k];
+        for (int l = 0; l < 5; ++l) {
+            v[l] = MODE == 3 || l == 0 ? u[(int64_t)l * L.ld + i] : T(0);
+            wy[l] = w[i + 5 * l];
+            if (MODE == 3) {
+                c[l] = u[l];
+                wx[l] = w[l];
+            }
+        }
+        T s[5];
 #pragma unroll
-        for (int p = 0; p < 5; ++p) {
+        for (int p = 0; p < 5; ++p) {   // y-line of column i
             T acc = T(0);
 #pragma unroll
-            for (int k = 0; k < 5; ++k) acc += Hc<T>(k, p) * u[k];
-            s[p] = w[p + 5 * j] * acc;
+            for (int l = 0; l < (MODE == 3 ? 5 : 1); ++l) acc = fma_rn<T>(v[l], Hc<T>(l, p), acc);
+            s[p] = mul_rn<T>(wy[p], acc);
+        }
+        T xl = T(0);
+        if (MODE == 3) {                // x-line of row 0, at column i
+#pragma unroll
+            for (int p = 0; p < 5; ++p) {
+                T acc = T(0);
+#pragma unroll
+                for (int k = 0; k < 5; ++k) acc = fma_rn<T>(Hc<T>(k, p), c[k], acc);
+                xl = fma_rn<T>(Hc<T>(i, p), mul_rn<T>(wx[p], acc), xl);
+            }
+            xl = mul_rn<T>((T)A.c1, xl);
         }
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
+        for (int r = 0; r < ROWS; ++r) {
             T acc = T(0);
 #pragma unroll
-            for (int p = 0; p < 5; ++p) acc += Hc<T>(i, p) * s[p];
-            yl[le * 25 + i + 5 * j] = A.c1 * acc;
+            for (int p = 0; p < 5; ++p) acc = fma_rn<T>(s[p], Hc<T>(ROW0 + r, p), acc);
+            part[r][t] = fma_rn<T>((T)A.c2, acc, xl);
         }
     }
     __syncthreads();
-    // y-lines: for element le and GLL column i, contract along eta.
-    for (int t = threadIdx.x; t < nE * 5; t += blockDim.x) {
-        const int le = t / 5, i = t - 5 * le;
-        const int lex = le % nex, ley = le / nex;
-        const T* ul = us + (4 * ley) * tnx + 4 * lex + i;
-        const T* w = Ws + le * 25;
-        T u[5], s[5];
-#pragma unroll
-        for (int l = 0; l < 5; ++l) u[l] = ul[l * tnx];
-#pragma unroll
-        for (int p = 0; p < 5; ++p) {
-            T acc = T(0);
-#pragma unroll
-            for (int l = 0; l < 5; ++l) acc += u[l] * Hc<T>(l, p);
-            s[p] = w[i + 5 * p] * acc;
-        }
-#pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            T acc = T(0);
-#pragma unroll
-            for (int p = 0; p < 5; ++p) acc += s[p] * Hc<T>(j, p);
-            yl[le * 25 + i + 5 * j] += A.c2 * acc;
-        }
-    }
-    __syncthreads();
-
-    // Gather for owned nodes.
-    const int ixb = 4 * ex0;
-    const int ixe = (ex0 + TEX >= L.NelX) ? L.nx : 4 * (ex0 + TEX);
-    int iyb, iye;
-    if (mode == 2) { iyb = 1; iye = 5; }
-    else if (mode == 3) { iyb = 0; iye = 1; }
-    else { iyb = 4 * ey0; iye = (ey0 + TEY >= L.NelY) ? L.ny : 4 * (ey0 + TEY); }
-    const int ownx = ixe - ixb, nown = ownx * (iye - iyb);
-    for (int k = threadIdx.x; k < nown; k += blockDim.x) {
-        const int ix = ixb + k % ownx, iy = iyb + k / ownx;
-        int exA, iA, exB = -1, iB = 0;
-        if (ix == 0) { exA = 0; iA = 0; }
-        else if (ix == L.nx - 1) { exA = L.NelX - 1; iA = 4; }
-        else if ((ix & 3) == 0) { exA = (ix >> 2) - 1; iA = 4; exB = ix >> 2; iB = 0; }
-        else { exA = ix >> 2; iA = ix & 3; }
-        int eyA, jA, eyB = -1, jB = 0;
-        if (iy == 0) { eyA = 0; jA = 0; }
-        else if (iy == L.ny - 1) { eyA = L.NelY - 1; jA = 4; }
-        else if ((iy & 3) == 0) { eyA = (iy >> 2) - 1; jA = 4; eyB = iy >> 2; jB = 0; }
-        else { eyA = iy >> 2; jA = iy & 3; }
-        if (strip && eyB >= 1) eyB = -1;   // strip modes: element row 0 only
+    const int nown = ex0 + STX >= L.NelX ? L.nx - 4 * ex0 : 4 * STX;
+    for (int k = t; k < nown * ROWS; k += ST_THREADS) {
+        const int q = k % nown, r = k / nown, ix = 4 * ex0 + q, e = q / 4 + 1;   // its element, and the one left of it
         T acc = T(0);
-        acc += yl[((eyA - eys) * nex + exA - exs) * 25 + iA + 5 * jA];
-        if (exB >= 0) acc += yl[((eyA - eys) * nex + exB - exs) * 25 + iB + 5 * jA];
-        if (eyB >= 0) {
-            acc += yl[((eyB - eys) * nex + exA - exs) * 25 + iA + 5 * jB];
-            if (exB >= 0) acc += yl[((eyB - eys) * nex + exB - exs) * 25 + iB + 5 * jB];
+        if ((q & 3) == 0) {
+            if (ix > 0) acc = add_rn<T>(acc, part[r][5 * (e - 1) + 4]);
+            if (ix < L.nx - 1) acc = add_rn<T>(acc, part[r][5 * e]);
+        } else {
+            acc = add_rn<T>(acc, part[r][5 * e + (q & 3)]);
         }
-        T out = sign * acc;
-        if (mode == 1 && iy == 0) out = T(0);
-        y[(int64_t)iy * L.ld + ix] = out;
+        y[(int64_t)(ROW0 + r) * L.ld + ix] = sign * acc;
     }
 }
 
@@ -1249,11 +1198,6 @@ static bool encode_w_walk(CUtensorMap* m, const float* base, int NelX, int NelY)
 
 constexpr int TEX = 8, TEY = 8;
 
-template <class T>
-static size_t apply_smem() {
-    return sizeof(T) * ((size_t)(4 * (TEX + 1) + 1) * (4 * (TEY + 1) + 1) + 2 * (size_t)(TEX + 1) * (TEY + 1) * 25);
-}
-
 constexpr int LTEX = 8, LTEY = 7, LNT = 256;
 
 template <class T> static CUtensorMap& wmap_ref(TmaCache& c);
@@ -1498,10 +1442,6 @@ bool set_H(const double* H, cudaStream_t s) {
     }
     EQC_CUDA(cudaStreamSynchronize(s));
     // kernel attributes are set here, at handle creation, never during a stream capture
-    EQC_CUDA(cudaFuncSetAttribute(k_apply<double, TEX, TEY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)apply_smem<double>()));
-    EQC_CUDA(cudaFuncSetAttribute(k_apply<float, TEX, TEY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)apply_smem<float>()));
     g_pipe_blocks[0] = resident_blocks(k_apply_pipe<float, LTEX, LTEY, LNT>, LNT, PipeLayout<float, LTEX, LTEY>::BYTES);
     g_pipe_blocks[1] = resident_blocks(k_apply_pipe<double, LTEX, LTEY, LNT>, LNT, PipeLayout<double, LTEX, LTEY>::BYTES);
     uni_setup();
@@ -1564,9 +1504,9 @@ void apply_K(const T* x, T* y, const ApplyArgs<T>& A, T sign, int mode, cudaStre
         count_launch();
         return;
     }
-    const size_t sm = apply_smem<T>();
-    dim3 grid((A.L.NelX + TEX - 1) / TEX, mode >= 2 ? 1 : (A.L.NelY + TEY - 1) / TEY);
-    k_apply<T, TEX, TEY><<<grid, 256, sm, s>>>(x, y, A, sign, mode);
+    const int grid = (A.L.NelX + STX - 1) / STX;
+    if (mode == 2) k_strip<T, 2><<<grid, ST_THREADS, 0, s>>>(x, y, A, sign);
+    else k_strip<T, 3><<<grid, ST_THREADS, 0, s>>>(x, y, A, sign);
     EQC_CHECK_LAUNCH();
     count_launch();
 }
