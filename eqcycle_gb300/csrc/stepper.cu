@@ -148,14 +148,18 @@ __global__ void k_zero_list(const int64_t* __restrict__ idx, int n, double* x, d
 }
 
 // ---------------------------------------------------------------- dynamic kernels
-// vPre on the fault; d += dt v + dt^2/2 a ; v += dt/2 a   (main.jl:299-306)
+// vPre on the fault; d += dt v + dt^2/2 a ; v += dt/2 a   (main.jl:299-306).  begin: with k_step_begin's work.
 __global__ void k_dyn_predict(double* __restrict__ d, double* __restrict__ v, const double* __restrict__ a,
-                              double* __restrict__ vPre_f, int Nf, int64_t n, Ctrl* C) {
+                              double* __restrict__ vPre_f, int Nf, int64_t n, Ctrl* C, int begin) {
     EQC_GRID_WAIT();
     const double dt = C->dt, hdt = C->half_dt, hdt2 = C->half_dt_sq;
     if (blockIdx.x == 0 && threadIdx.x == 0) {   // d changes: no carried residual, no QS history
         C->r_valid = 0;
         C->qs_prev = 0;
+        if (begin) {
+            C->it += 1;
+            C->t = C->t + dt;
+        }
     }
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double vi = v[i], ai = a[i];
@@ -335,39 +339,6 @@ __global__ void k_dyn_bc_nodes(double* __restrict__ a, const double* __restrict_
     }
 }
 
-// Fault boundary condition (main.jl:321-331): FltVfree, Vf, FBC! (two NR solves per node),
-// tau = tau2 - tauo, psi = psi2, a[iFlt] -= FltB tau.
-__global__ void __launch_bounds__(FNT) k_dyn_fault(double* __restrict__ a, const double* __restrict__ v, FaultArgs f, Ctrl* C) {
-    EQC_GRID_WAIT();
-    const double dt = C->dt, hdt = C->half_dt, Vpl = C->Vpl;
-    for (int k = threadIdx.x + blockIdx.x * blockDim.x; k < f.Nf; k += blockDim.x * gridDim.x) {
-        const double vfree = 2 * v[k] + 2 * hdt * a[k] / f.Mf[k];
-        f.FltVfree[k] = vfree;
-        const double vf = 2 * f.vPre[k] + Vpl;
-        f.Vf[k] = vf;
-        if (k >= f.NFBC0) {
-            const double p1 = dev_IDS(f.xLf[k], f.Vo[k], f.psi[k], dt, vf, 1e-5);
-            f.psi1[k] = p1;
-            double V1, T1;
-            dev_NR(f.fo[k], f.Vo[k], f.cca[k], f.ccb[k], f.Seff[k], 0.0, f.tauo[k], p1, f.FltZ[k], vfree, &V1, &T1);
-            f.Vf1[k] = V1;
-            f.tau1[k] = T1;
-            if (vf > 1e10 || isnan(vf) || isnan(T1)) atomicMin(&C->fail, k + 1);
-            const double p2 = dev_IDS2(f.xLf[k], f.Vo[k], f.psi[k], p1, dt, vf, V1);
-            f.psi2[k] = p2;
-            double V2, T2;
-            dev_NR(f.fo[k], f.Vo[k], f.cca[k], f.ccb[k], f.Seff[k], T1, f.tauo[k], p2, f.FltZ[k], vfree, &V2, &T2);
-            f.Vf2[k] = V2;
-            f.tau2[k] = T2;
-        }
-        double t = f.tau2[k] - f.tauo[k];
-        if (f.creep[k]) t = 0.;
-        f.tau[k] = t;
-        f.psi[k] = f.psi2[k];
-        a[k] = a[k] - f.FltB[k] * t;
-    }
-}
-
 // a = a / M ; v += dt/2 a   (main.jl:336-339), the plain method's rounding of the division
 __global__ void k_dyn_correct(double* __restrict__ a, double* __restrict__ v, const double* __restrict__ M,
                               const double* __restrict__ invM, int64_t n, const Ctrl* C) {
@@ -504,6 +475,54 @@ __global__ void __launch_bounds__(FNT) k_control(const double* __restrict__ v, F
     for (int k = threadIdx.x + blockIdx.x * blockDim.x; k < f.Nf; k += blockDim.x * gridDim.x)
         ctl_add(c, k, v[k], f.XiLf[k], f.NFBC0, Vpl);
     ctl_last(c, part, count, C);
+}
+
+// Fault boundary condition (main.jl:321-331): FltVfree, Vf, FBC! (two NR solves per node),
+// tau = tau2 - tauo, psi = psi2, a[iFlt] -= FltB tau.  With M (the plain method, the creeping nodes in the fault
+// row): also the row's end of step (main.jl:336-344: k_dyn_correct's arithmetic, creeping nodes a = v = 0) and the
+// control, which leaves five launches to a step instead of eight: 71.6 to 70.7 us on 61 x 95 elements, where the
+// searches are most of a step, 127.5 to 107 on 120 x 240, 257 to 232 on 240 x 480.
+__global__ void __launch_bounds__(FNT) k_dyn_fault(double* __restrict__ a, double* __restrict__ v, FaultArgs f, Ctrl* C,
+                                                   const double* __restrict__ M, const double* __restrict__ invM,
+                                                   CtlAcc* part, unsigned* count) {
+    EQC_GRID_WAIT();
+    const double dt = C->dt, hdt = C->half_dt, Vpl = C->Vpl;
+    CtlAcc acc = ctl_init();
+    for (int k = threadIdx.x + blockIdx.x * blockDim.x; k < f.Nf; k += blockDim.x * gridDim.x) {
+        const double vfree = 2 * v[k] + 2 * hdt * a[k] / f.Mf[k];
+        f.FltVfree[k] = vfree;
+        const double vf = 2 * f.vPre[k] + Vpl;
+        f.Vf[k] = vf;
+        if (k >= f.NFBC0) {
+            const double p1 = dev_IDS(f.xLf[k], f.Vo[k], f.psi[k], dt, vf, 1e-5);
+            f.psi1[k] = p1;
+            double V1, T1;
+            dev_NR(f.fo[k], f.Vo[k], f.cca[k], f.ccb[k], f.Seff[k], 0.0, f.tauo[k], p1, f.FltZ[k], vfree, &V1, &T1);
+            f.Vf1[k] = V1;
+            f.tau1[k] = T1;
+            if (vf > 1e10 || isnan(vf) || isnan(T1)) atomicMin(&C->fail, k + 1);
+            const double p2 = dev_IDS2(f.xLf[k], f.Vo[k], f.psi[k], p1, dt, vf, V1);
+            f.psi2[k] = p2;
+            double V2, T2;
+            dev_NR(f.fo[k], f.Vo[k], f.cca[k], f.ccb[k], f.Seff[k], T1, f.tauo[k], p2, f.FltZ[k], vfree, &V2, &T2);
+            f.Vf2[k] = V2;
+            f.tau2[k] = T2;
+        }
+        double t = f.tau2[k] - f.tauo[k];
+        if (f.creep[k]) t = 0.;
+        f.tau[k] = t;
+        f.psi[k] = f.psi2[k];
+        double ak = a[k] - f.FltB[k] * t;
+        if (M) {
+            ak = div_by(ak, M[k], invM[k]);
+            double vk = v[k] + hdt * ak;
+            if (f.creep[k]) ak = vk = 0.;
+            v[k] = vk;
+            ctl_add(acc, k, vk, f.XiLf[k], f.NFBC0, Vpl);
+        }
+        a[k] = ak;
+    }
+    if (M) ctl_last(acc, part, count, C);
 }
 
 // The fault row of the mixed method's dynamic step, from a = -(K d)[iFlt] (t0, the FP64 strip
@@ -982,10 +1001,14 @@ static void enqueue_dyn_mixed_fused(Handle& h) {
     launch_check();
 }
 
+// The plain method's dynamic step advances it and t in its predictor and ends in its fault kernel, control included.
+static bool plain_row_ends(const Handle& h) { return h.opt.precision == EQC_FP64 && h.creep_prefix; }
+
 static void enqueue_dyn(Handle& h, bool graph) {
     cudaStream_t s = h.stream;
     const int64_t n = h.L.size();
     FaultArgs f = fargs(h, h.bcflag.p);
+    const bool row_ends = plain_row_ends(h);
     if (h.opt.precision == EQC_MIXED && h.nm_fused) {
         enqueue_dyn_mixed_fused(h);
         return;
@@ -1024,7 +1047,7 @@ static void enqueue_dyn(Handle& h, bool graph) {
         k_dyn_force<<<vblocks4(n), 256, 0, s>>>(h.Kd.p, h.q32.p, h.a.p, n, h.ctrl.p);
         count_launch();
     } else {
-        k_dyn_predict<<<vblocks(n), 256, 0, s>>>(h.d.p, h.v.p, h.a.p, h.F.vPre.p, h.F.Nf, n, h.ctrl.p);
+        k_dyn_predict<<<vblocks(n), 256, 0, s>>>(h.d.p, h.v.p, h.a.p, h.F.vPre.p, h.F.Nf, n, h.ctrl.p, row_ends ? 1 : 0);
         count_launch();
         apply_K<double>(h.d.p, h.a.p, args64(h), -1.0, 0, s);
     }
@@ -1034,7 +1057,16 @@ static void enqueue_dyn(Handle& h, bool graph) {
     else
         k_dyn_bc<<<1, 1024, 0, s>>>(h.a.p, h.v.p, h.iCreep.p, h.nCreep, h.iBcL.p, h.BcLC.p, h.nBcL, h.iBcT.p, h.BcTC.p,
                                     h.nBcT);
-    k_dyn_fault<<<fblocks(h.F.Nf), FNT, 0, s>>>(h.a.p, h.v.p, f, h.ctrl.p);
+    CtlAcc* part = reinterpret_cast<CtlAcc*>(h.fault_part.p);
+    if (row_ends) {   // the rows off the fault end first, then the fault row and the control
+        const int64_t ld = h.L.ld;
+        k_dyn_correct<<<vblocks(n - ld), 256, 0, s>>>(h.a.p + ld, h.v.p + ld, h.M.p + ld, h.invM.p + ld, n - ld, h.ctrl.p);
+        k_dyn_fault<<<fblocks(h.F.Nf), FNT, 0, s>>>(h.a.p, h.v.p, f, h.ctrl.p, h.M.p, h.invM.p, part, h.fault_count.p);
+        count_launch(3);
+        launch_check();
+        return;
+    }
+    k_dyn_fault<<<fblocks(h.F.Nf), FNT, 0, s>>>(h.a.p, h.v.p, f, h.ctrl.p, nullptr, nullptr, part, h.fault_count.p);
     const bool mixed = h.opt.precision == EQC_MIXED;
     const bool zero_fused = mixed && h.creep_prefix;
     if (mixed) k_dyn_correct_inv<<<vblocks4(n), 256, 0, s>>>(h.a.p, h.v.p, h.invM.p, n, h.ctrl.p,
@@ -1059,9 +1091,8 @@ void materialize_dyn_state(Handle& h) {
 }
 
 void enqueue_step(Handle& h, int iso, bool graph) {
-    // the mixed method's dynamic step advances it and t in its predictor and runs the control in
-    // its fault kernel
-    const bool fused = iso == 2 && h.opt.precision == EQC_MIXED && h.nm_fused;
+    // dynamic steps that advance it and t in their predictor and run the control in their fault kernel
+    const bool fused = iso == 2 && ((h.opt.precision == EQC_MIXED && h.nm_fused) || plain_row_ends(h));
     if (!fused) {
         k_step_begin<<<1, 1, 0, h.stream>>>(h.ctrl.p);
         count_launch();
