@@ -4,8 +4,8 @@
 // layout index k).  The quasi-static branch (main.jl:226-295) runs two predictor-corrector
 // passes, each one CG solve (solver.cu) plus fault-row kernels; the dynamic branch
 // (main.jl:297-345) is an explicit Newmark step with the friction Newton solve per fault
-// node (K5).  After each step a single-CTA control kernel reduces the fault slip rate
-// (Vfmax, main.jl:348), switches regime (main.jl:439-443) and computes the next dt
+// node (K5).  At its end a step's control, in a kernel of its own or in the fault kernel's last
+// CTA, reduces the fault slip rate (Vfmax, main.jl:348), switches regime (main.jl:439-443) and computes the next dt
 // (dtevol!, src/dtevol.jl:5-44).  Output triggers (main.jl:361-436) are evaluated on the
 // host from the control block.
 #include "model.h"
