@@ -662,6 +662,7 @@ __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUt
         bool done = false;
         const int polls = i == 0 ? A.wait_polls : MBAR_SPIN_LIMIT;
         for (int it = 0; it < polls && !done; ++it) done = mbar_try_wait(&bar[st], parity);
+        done = __all_sync(0xffffffffu, done);   // lanes poll apart: the tile may land between their last polls
         const int ex0 = (t % ntx) * UEX, ey0 = (t / ntx) * UEY;
         const double* us = reinterpret_cast<const double*>(smem + st * UT::STAGE);
         const double* ms = reinterpret_cast<const double*>(smem + st * UT::STAGE + UT::M_OFF) + (ex0 & 1);

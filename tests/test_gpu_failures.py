@@ -166,6 +166,25 @@ def test_tma_wait_gives_up_and_the_handle_recovers(eqclib, small, variant):
         assert np.array_equal(s.apply_K(x), y0)
 
 
+@pytest.mark.parametrize("variant", [0, 1, 3], ids=["one-contraction", "one-tile", "pipelined"])
+def test_tma_wait_gives_up_part_way(eqclib, small, variant):
+    """A few polls for the first tile wait: some threads of a CTA may see the tile land and others not.  Each
+    call gives either EQC_E_TIMEOUT or the K x of the full bound, and the handle keeps working."""
+    cfg, P = small
+    x = np.random.default_rng(0).uniform(-1e-3, 1e-3, P.int_.nglob)
+    with Solver(P, precond=EQC_PC_JACOBI, apply_variant=variant) as s:
+        y0 = s.apply_K(x)
+        default = s.scalar("tma_wait_polls")
+        for polls in (1, 2, 3, 4, 6, 8, 12, 16, 32, 64):
+            s.set_scalar("tma_wait_polls", polls)
+            try:
+                assert np.array_equal(s.apply_K(x), y0)
+            except EqcError as e:
+                assert e.status == E_TIMEOUT
+        s.set_scalar("tma_wait_polls", default)
+        assert np.array_equal(s.apply_K(x), y0)
+
+
 def test_tma_wait_timeout_in_the_time_loop(eqclib, small):
     """The same give-up inside graph-replayed steps (FP64 apply and multigrid): eqc_run reports
     EQC_E_TIMEOUT; afterwards, with the bound restored and the state initialised again, the
