@@ -1305,9 +1305,11 @@ static int g_pipe_blocks[2] = {0, 0};
 template <class T>
 static int pipe_blocks() { return g_pipe_blocks[sizeof(T) == 8 ? 1 : 0]; }
 
+// CTAs that fit with `bytes` of shared memory each; `most`: the most that a launch asks for.  A kernel's limit is set
+// to one value only: another thread may be launching it while this one creates a handle.
 template <class K>
-static int resident_blocks(K kernel, int threads, int bytes) {
-    EQC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+static int resident_blocks(K kernel, int threads, int bytes, int most = 0) {
+    EQC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(bytes, most)));
     int per_sm = 0, dev = 0, nsm = 0;
     EQC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes));
     EQC_CUDA(cudaGetDevice(&dev));
@@ -1324,8 +1326,7 @@ static void uni_setup() {
     EQC_CUDA(cudaGetDevice(&dev));
     EQC_CUDA(cudaDeviceGetAttribute(&g_uni_sms, cudaDevAttrMultiProcessorCount, dev));
     auto one = [](auto kernel, int& per_sm) {
-        per_sm = resident_blocks(kernel, UNT, UniTile::BYTES) / g_uni_sms;
-        EQC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, UNI_SMEM));
+        per_sm = resident_blocks(kernel, UNT, UniTile::BYTES, UNI_SMEM) / g_uni_sms;
     };
     one(k_apply_uni64<NoTail>, g_uni_per_sm<NoTail>);
     one(k_apply_uni64<ResidualOut>, g_uni_per_sm<ResidualOut>);
