@@ -858,6 +858,13 @@ void mg_build(Handle& h) {
     // the V-cycle recursion below the coarsest smoothed level uses lev[L-1] as the dense level
 }
 
+void mg_clear_work(Handle& h) {
+    for (MGWork& w : h.mg->work) {
+        for (DBuf<double>* b : {&w.x64, &w.b64, &w.r64, &w.d64, &w.t64}) b->zero(h.stream);
+        for (DBuf<float>* b : {&w.x32, &w.b32, &w.r32, &w.d32, &w.t32}) b->zero(h.stream);
+    }
+}
+
 void mg_destroy(Handle& h) {
     delete h.mg;
     h.mg = nullptr;

@@ -296,6 +296,8 @@ void enqueue_solve(Handle& h, double tol, int maxit, bool graph, bool carry = fa
 // Marks the carried residual stale (after the state was changed from outside the loop).
 void invalidate_residual(Handle& h);
 int qs_solve_device(Handle& h, double tol, int maxit, double* relres);
+// Zeroes what a solve that broke down (EQC_E_NAN) leaves in the work vectors and in the rows' padding.
+void clear_after_breakdown(Handle& h);
 // Throws EQC_E_TIMEOUT (and clears the device flag) when a TMA apply gave up a bounded wait.
 void check_apply_err(Handle& h);
 
@@ -347,6 +349,7 @@ double fault_dtevol(Handle& h, double dt, double dtmin, const double* Vf, int is
 // mg_setup.cpp / mg.cu
 void mg_build(Handle& h);
 void mg_destroy(Handle& h);
+void mg_clear_work(Handle& h);   // zeroes the cycle's vectors on every level
 void mg_apply64(Handle& h, const double* r, double* z);
 // ... true when its last launch also left rho = z.r and beta in S
 bool mg_apply32(Handle& h, const float* r, float* z, CGState* S);

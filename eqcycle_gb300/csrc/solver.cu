@@ -672,10 +672,26 @@ void invalidate_residual(Handle& h) {
     if (h.h_ctrl) h.h_ctrl->r_valid = h.h_ctrl->qs_prev = h.h_ctrl->kd_valid = 0;
 }
 
+// After a solve that broke down: its work vectors hold values that are not finite, in the rows' padding too, which
+// the vector kernels and sums run over and the applies do not write.  Cleared, so that the next solve starts from
+// finite numbers everywhere (of the state only the padding: its nodes are the caller's to set again).
+void clear_after_breakdown(Handle& h) {
+    cudaStream_t s = h.stream;
+    for (DBuf<double>* b : {&h.r64, &h.z64, &h.p64, &h.q64, &h.dx64, &h.kdx64}) b->zero(s);
+    for (DBuf<float>* b : {&h.r32, &h.z32, &h.p32, &h.p32b, &h.q32, &h.x32, &h.g32}) b->zero(s);
+    if (h.mg) mg_clear_work(h);
+    const Layout& L = h.L;
+    for (DBuf<double>* b : {&h.d, &h.v, &h.a, &h.dPre})
+        EQC_CUDA(cudaMemset2DAsync(b->p + L.nx, L.ld * sizeof(double), 0, (L.ld - L.nx) * sizeof(double), L.ny, s));
+    invalidate_residual(h);
+    EQC_CUDA(cudaStreamSynchronize(s));
+}
+
 // Solves for d_I given d row 0 = F (eager); returns iterations (negative: maxit reached).
 int qs_solve_device(Handle& h, double tol, int maxit, double* relres) {
     enqueue_solve(h, tol, maxit, false);
     const CGState& S = read_cg(h);
+    if (S.done == 3) clear_after_breakdown(h);
     check_apply_err(h);
     if (S.done == 3) throw Error(EQC_E_NAN, "non-finite residual in CG");
     if (relres) *relres = S.nb > 0 ? S.res / S.nb : S.res;

@@ -1248,6 +1248,7 @@ void post_step(Handle& h, int iso, eqc_run_stats& stats, PostBufs& pb, bool logg
     if (!logged && (int64_t)h.res.time_.size() >= h.cap_time)
         throw Error(EQC_E_CAPACITY, "time_ capacity (" + std::to_string(h.cap_time) + ") exceeded");
     if (!logged) h.res.time_.push_back(tnow);
+    if (C.cg_fail & 2) clear_after_breakdown(h);
     if (C.fail != 0x7fffffff)
         throw Error(EQC_E_NR, "NR SEARCH FAILED at fault node " + std::to_string(C.fail));
     if (C.apply_err) check_apply_err(h);
