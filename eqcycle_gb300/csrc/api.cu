@@ -237,7 +237,7 @@ static void create(Handle& h, const eqc_model& m, const eqc_material* mat) {
                              &h.q64, &h.Kd})
         b->alloc(N);
     for (DBuf<float>* b : {&h.r32, &h.z32, &h.p32, &h.q32, &h.x32, &h.g32, &h.p32b}) b->alloc(N);
-    if (h.opt.precision == EQC_MIXED && h.df_ok && df_pays(L) && std::getenv("EQC_NO_DF_UPDATE") == nullptr) {
+    if (h.opt.precision == EQC_MIXED && h.df_ok && std::getenv("EQC_NO_DF_UPDATE") == nullptr) {
         h.dx64.alloc(N);    // the intermediate reliable updates' correction and its K dx
         h.kdx64.alloc(N);
     }

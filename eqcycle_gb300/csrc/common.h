@@ -135,6 +135,7 @@ struct ApplyArgs {
                       // give-up path (eqc_set_scalar "tma_wait_polls")
     const int* gate = nullptr;   // when set, the launch does nothing unless *gate (written by a
     int gate_val = 0;            // preceding kernel) equals gate_val
+    bool uni = false;            // FP64: the one-contraction apply is the faster one (classify_elements)
 };
 
 // Bound, in polls of mbarrier.try_wait, of every wait of the TMA-fed stiffness applies.

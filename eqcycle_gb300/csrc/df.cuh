@@ -72,11 +72,12 @@ EQC_HD df df_mul(df x, df y) {
 
 // FP64 -> double-float: hi carries the 24 leading significand bits (truncated), lo the next 24
 // (rounded); |x| outside [2^-90, 2^120] maps to hi = lo = 0 (far below or above any value the
-// stiffness apply sees: displacements, forces).  Integer operations only.
+// stiffness apply sees: displacements, forces).  Integer operations only.  Without branches, which would
+// serialise a caller's loads; df_from_double_skip has them, for a caller that converts each value as it comes.
 EQC_HD df df_from_double(double x) {
     const int64_t b = df_bits64(x);
     const int32_t e = (int32_t)((b >> 52) & 0x7ff);
-    const bool in = e >= 1023 - 90 && e <= 1023 + 120;   // selected at the end: branches would serialise a caller's loads
+    const bool in = e >= 1023 - 90 && e <= 1023 + 120;
     const int32_t sgn = (int32_t)((uint64_t)b >> 63) << 31;
     const int64_t m = b & 0xfffffffffffffLL;                 // 52 fraction bits
     const int32_t hi = sgn | (int32_t)((uint32_t)(e - 1023 + 127) << 23) | (int32_t)(m >> 29);
@@ -86,6 +87,20 @@ EQC_HD df df_from_double(double x) {
     const int32_t re = ((rb >> 23) & 0xff) + (e - 1023 - 52);  // biased exponent of lo
     const int32_t lo = sgn | (int32_t)((uint32_t)re << 23) | (rb & 0x7fffff);
     return df{df_from_bits32(in ? hi : 0), df_from_bits32(in && rem != 0 && re > 0 ? lo : 0)};
+}
+EQC_HD df df_from_double_skip(double x) {
+    const int64_t b = df_bits64(x);
+    const int32_t e = (int32_t)((b >> 52) & 0x7ff);
+    if (e < 1023 - 90 || e > 1023 + 120) return df{0.f, 0.f};
+    const int32_t sgn = (int32_t)((uint64_t)b >> 63) << 31;
+    const int64_t m = b & 0xfffffffffffffLL;
+    const float hi = df_from_bits32(sgn | (int32_t)((uint32_t)(e - 1023 + 127) << 23) | (int32_t)(m >> 29));
+    const int32_t rem = (int32_t)(m & 0x1fffffff);
+    if (rem == 0) return df{hi, 0.f};
+    const int32_t rb = df_bits32((float)rem);
+    const int32_t re = ((rb >> 23) & 0xff) + (e - 1023 - 52);
+    if (re <= 0) return df{hi, 0.f};
+    return df{hi, df_from_bits32(sgn | (int32_t)((uint32_t)re << 23) | (rb & 0x7fffff))};
 }
 
 // double-float -> FP64 (one FP64 add; the widenings are exact and use integer operations)

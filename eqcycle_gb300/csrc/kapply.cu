@@ -552,6 +552,20 @@ __global__ void k_classify(const double* __restrict__ W, double* __restrict__ mu
     }
 }
 
+// *count += the tiles of tx x ty owned elements (on the grid of the element vertices, one halo column and row below
+// and left) that hold an element of several rigidities.
+__global__ void k_classify_tiles(const double* __restrict__ mu, int pitch, int NelX, int NelY, int tx, int ty, int* count) {
+    EQC_GRID_WAIT();
+    const int ntx = NelX / tx + 1, ntiles = ntx * (NelY / ty + 1);
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
+        const int ex0 = (t % ntx) * tx, ey0 = (t / ntx) * ty;
+        bool several = false;
+        for (int ey = max(ey0 - 1, 0); ey < min(ey0 + ty, NelY); ++ey)
+            for (int ex = max(ex0 - 1, 0); ex < min(ex0 + tx, NelX); ++ex) several = several || mu[(int64_t)ey * pitch + ex + 1] < 0.0;
+        if (several) atomicAdd(count, 1);
+    }
+}
+
 // Two contractions with W between them: a line that meets an element of several rigidities.
 __device__ __forceinline__ void generic_line(const double (&u)[5], const double (&w)[5], double (&o)[5]) {
     double s[5];
@@ -1287,16 +1301,39 @@ void classify_elements(Handle& h) {
         w /= (32.0 / 45.0) * (32.0 / 45.0);
         h.mu_unit = w > 0.0 && std::isfinite(w) ? w : 1.0;
     }
-    DBuf<int> several;
-    several.alloc(1);
+    DBuf<int> several;   // elements, tiles of the FP64 apply and of the double-float one
+    several.alloc(3);
     k_classify<<<(int)std::min<int64_t>((Nel + 255) / 256, 4096), 256, 0, h.stream>>>(
         h.W64.p, h.mu64.p, h.mu32.p, several.p, L.NelX, L.NelY, mp, h.mu_unit, h.uni_ok ? 1 : 0);
+    const int64_t t64 = (int64_t)(L.NelX / UEX + 1) * (L.NelY / UEY + 1), tdf = (int64_t)(L.NelX / DF_COLS + 1) * (L.NelY / DF_ROWS + 1);
+    k_classify_tiles<<<(int)std::min<int64_t>((t64 + 255) / 256, 4096), 256, 0, h.stream>>>(h.mu64.p, mp, L.NelX, L.NelY, UEX, UEY,
+                                                                                         several.p + 1);
+    k_classify_tiles<<<(int)std::min<int64_t>((tdf + 255) / 256, 4096), 256, 0, h.stream>>>(h.mu64.p, mp, L.NelX, L.NelY, DF_COLS,
+                                                                                         DF_ROWS, several.p + 2);
     EQC_CHECK_LAUNCH();
-    count_launch();
-    int n = 0;
-    several.download(&n, 1, h.stream);
+    count_launch(3);
+    int n[3] = {0, 0, 0};
+    several.download(n, 3, h.stream);
     EQC_CUDA(cudaStreamSynchronize(h.stream));
-    h.sem_ok = h.uni_ok && (int64_t)n * 8 <= Nel && L.size() < (int64_t)1 << 29 &&   // 32-bit byte offsets
+    // The one-contraction FP64 apply against the pipeline with both contractions, by the share f of its tiles that hold
+    // an element of several rigidities (us a launch, x and y in L2, 240 x 480 elements; before the line 135 for any f):
+    // none 70 and 135; scattered, f = 0.5 94 and 135, 0.77 105, 0.9 113, 0.99 134, then up to 170; in a band 87 at
+    // f = 0.25, 98 at 0.45, 110 at 0.66.  On 120 x 240: none 22 and 39, f = 0.5 31 and 39, 0.89 36, 0.99 41, up to 50; a
+    // band 36 at f = 0.66 and 40 at 0.75.  So up to two thirds of the tiles.  With two tiles or fewer to an SM the
+    // slowest tile sets the time: 61 x 95 in bands of 3 % 14 and 15, of 6 % 16 and 15, of 25 % 19 and 15; one
+    // element in 32 is asked there too.
+    const int64_t several_el = n[0];
+    h.uni64_pays = h.uni_ok && 3 * (int64_t)n[1] <= 2 * t64 && (t64 > 2 * 152 || 32 * several_el <= Nel);
+    h.few_several = 128 * several_el <= Nel;   // for df_pays
+    // The double-float apply (240 x 480): none 37 us, scattered over 0.28 of the CTAs 59, 0.36 62, 0.5 68, and 67 with
+    // both contractions everywhere.
+    h.uni_df_pays = h.uni_ok && 5 * (int64_t)n[2] <= 2 * tdf;
+    // The operator of sem.cu against the row-tile apply with its vector kernels (ms per quasi-static step, elements of
+    // several rigidities scattered over the mesh, whose warps take both contractions): one in eight 3.16 on 240 x 480
+    // elements and 9.33 on 480 x 960; one in four 3.24 and 3.41, 9.38 and 10.96; all 1.21 and 1.37 on 48 x 48, 1.66
+    // and 1.83 on 120 x 240, 3.31 and 3.49, 9.39 and 10.97.  It was the faster one at every share: one in eight keeps
+    // models of mostly several rigidities on the apply that the Newmark steps use.
+    h.sem_ok = h.uni_ok && several_el * 8 <= Nel && L.size() < (int64_t)1 << 29 &&   // 32-bit byte offsets
                L.NelX < 31 * 4096;                                              // partials of a dot product's CTAs
 }
 
@@ -1486,7 +1523,7 @@ void apply_K(const T* x, T* y, const ApplyArgs<T>& A, T sign, int mode, cudaStre
             }
         }
         if constexpr (sizeof(T) == 8) {
-            const CUtensorMap* uu = (A.tma && (A.variant == 0 || A.variant > 3)) ? tma_umap_uni(*A.tma, x, A.L) : nullptr;
+            const CUtensorMap* uu = (A.uni && A.tma && (A.variant == 0 || A.variant > 3)) ? tma_umap_uni(*A.tma, x, A.L) : nullptr;
             if (uu) {
                 launch_uni64(*uu, y, A, sign, mode == 1 ? 1 : 0, s);
                 return;
@@ -1534,7 +1571,7 @@ bool apply_K_epi(const float* x, const ApplyArgs<float>& A, int mode, const OpEp
 }
 
 bool apply_K_epi(const double* x, const ApplyArgs<double>& A, int mode, const OpEpi<double>& E, cudaStream_t s) {
-    if (mode > 1 || !A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
+    if (mode > 1 || !A.uni || !A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
     const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
     if (!uu) return false;
     launch_uni64(*uu, nullptr, A, 1.0, mode, s, E);
@@ -1542,7 +1579,7 @@ bool apply_K_epi(const double* x, const ApplyArgs<double>& A, int mode, const Op
 }
 
 bool apply_K_dot(const double* x, double* y, const ApplyArgs<double>& A, const DotOut& dot, cudaStream_t s) {
-    if (!A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
+    if (!A.uni || !A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
     const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
     if (!uu) return false;
     OpEpi<double> E;
@@ -1552,7 +1589,7 @@ bool apply_K_dot(const double* x, double* y, const ApplyArgs<double>& A, const D
 }
 
 bool apply_K_residual(const double* x, const ApplyArgs<double>& A, const ResidualOut& R, cudaStream_t s) {
-    if (!A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
+    if (!A.uni || !A.tma || (A.variant >= 1 && A.variant <= 3)) return false;
     const CUtensorMap* uu = tma_umap_uni(*A.tma, x, A.L);
     if (!uu) return false;
     launch_uni64(*uu, nullptr, A, -1.0, 1, s, OpEpi<double>(), R);

@@ -64,7 +64,7 @@ __device__ __forceinline__ df shfl_up_df(df v) {
     return df{__shfl_up_sync(0xffffffffu, v.hi, 1), __shfl_up_sync(0xffffffffu, v.lo, 1)};
 }
 
-template <int ROWS, bool RES>
+template <int ROWS, bool RES, bool UNI>
 __global__ void __launch_bounds__(32 * (ROWS + 1), 2)
     k_apply_df(const double* __restrict__ x, double* __restrict__ y, const float* __restrict__ Whi,
                const float* __restrict__ Wlo, const double* __restrict__ mu64, int mu_pitch, Layout L, df c1, df c2,
@@ -82,12 +82,12 @@ __global__ void __launch_bounds__(32 * (ROWS + 1), 2)
     // node (4 ex + i, 4 ey + j) of the element, zero outside the grid
     auto node = [&](int i, int j) {
         const int ix = 4 * ex + i, iy = 4 * ey + j;
-        return (ix >= 0 && ix < L.nx && iy >= 0 && iy < L.ny) ? df_from_double(__ldg(x + (int64_t)iy * L.ld + ix))
-                                                             : df{0.f, 0.f};
+        return (ix >= 0 && ix < L.nx && iy >= 0 && iy < L.ny) ? df_from_double_skip(__ldg(x + (int64_t)iy * L.ld + ix))
+                                                                  : df{0.f, 0.f};
     };
-    const double mu = real ? __ldg(mu64 + (int64_t)ey * mu_pitch + ex + 1) : 0.0;
+    const double mu = UNI && real ? __ldg(mu64 + (int64_t)ey * mu_pitch + ex + 1) : 0.0;
     df out[4][4], R[4], T[5];
-    if (__all_sync(0xffffffffu, __double2hiint(mu) >= 0)) {
+    if (UNI && __all_sync(0xffffffffu, __double2hiint(mu) >= 0)) {
         const df m = df_from_double(mu);
         // every load before the first conversion; an element outside the mesh reads the nearest one (mu is 0)
         const double* xe = x + (int64_t)(4 * min(max(ey, 0), L.NelY - 1)) * L.ld + 4 * min(max(ex, 0), L.NelX - 1);
@@ -250,11 +250,11 @@ void set_H_df(const double* H, cudaStream_t s) {
 bool apply_K_df(Handle& h, const double* x, double* y, double sign, int mode, cudaStream_t s, const int* gate,
                 int gate_val, const ResidualOut* Ro) {
     if (!h.df_ok || mode > 1 || !h.W32lo.p || (reinterpret_cast<uintptr_t>(y) & 15)) return false;
-    if (!gate && !Ro && !df_pays(h.L) && h.uni_ok && h.opt.apply_variant == 0) {
+    if (!gate && !Ro && !df_pays(h) && h.opt.apply_variant == 0) {
         apply_K<double>(x, y, args64(h), sign, mode, s);
         return true;
     }
-    constexpr int R = 6;
+    constexpr int R = DF_ROWS;
     const Layout& L = h.L;
     UniDF U;   // S = D^T diag(w) D in its even-odd form
     const double gw[5] = {0.1, 49.0 / 90.0, 32.0 / 45.0, 49.0 / 90.0, 0.1};
@@ -279,8 +279,13 @@ bool apply_K_df(Handle& h, const double* x, double* y, double sign, int mode, cu
         kernel<<<g, 32 * (R + 1), 0, s>>>(x, y, h.W32p.p, h.W32lo.p, h.mu64.p, mu_pitch(L.NelX), L, host_df(h.c1),
                                           host_df(h.c2), U, sign, mode == 1 ? 1 : 0, gate, gate_val, Ro ? *Ro : ResidualOut());
     };
-    if (Ro) go(k_apply_df<R, true>);
-    else go(k_apply_df<R, false>);
+    if (h.uni_df_pays) {
+        if (Ro) go(k_apply_df<R, true, true>);
+        else go(k_apply_df<R, false, true>);
+    } else {
+        if (Ro) go(k_apply_df<R, true, false>);
+        else go(k_apply_df<R, false, false>);
+    }
     EQC_CHECK_LAUNCH();
     count_launch();
     return true;

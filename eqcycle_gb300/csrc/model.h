@@ -165,6 +165,9 @@ struct Handle {
     double sem_scale = 1.0;  // set_H_sem
     bool sem_ok = false; // the FP32 operator of sem.cu pays (classify_elements)
     bool uni_ok = false; // H admits the one-contraction lines of the FP64 apply
+    bool uni64_pays = false;   // few enough elements of several rigidities for it (classify_elements)
+    bool uni_df_pays = false;  // the same of the double-float apply
+    bool few_several = false;  // at most one element in 128 is of several rigidities
     DBuf<float> W32, W32p;
     DBuf<float> W32lo;   // W - W32p rounded to FP32 (padded like W32p): W as double-float
     bool df_ok = false;  // the double-float FP64-class apply is usable (EQC_NO_DF unset, H symmetric)
@@ -229,11 +232,13 @@ bool set_H(const double* H, cudaStream_t s);
 inline int mu_pitch(int NelX) { return (NelX + 3) & ~1; }   // row pitch of mu64
 // mu64 from W64 (after every change of W64)
 void classify_elements(Handle& h);
+constexpr int DF_COLS = 31, DF_ROWS = 6;   // elements that a CTA of the double-float apply owns
 template <class T>
 void apply_K(const T* x, T* y, const ApplyArgs<T>& A, T sign, int mode, cudaStream_t s);
 
 inline ApplyArgs<double> args64(Handle& h) {
-    return {h.W64.p, h.c1, h.c2, h.L, h.W64p.p, &h.ctrl.p->apply_err, &h.tma, h.opt.apply_variant, h.tma_wait_polls};
+    return {h.W64.p, h.c1, h.c2, h.L, h.W64p.p, &h.ctrl.p->apply_err, &h.tma, h.opt.apply_variant, h.tma_wait_polls,
+            nullptr, 0, h.uni64_pays};
 }
 inline ApplyArgs<float> args32(Handle& h) {
     return {h.W32.p, (float)h.c1, (float)h.c2, h.L, h.W32p.p, &h.ctrl.p->apply_err, &h.tma, h.opt.apply_variant,
@@ -256,8 +261,13 @@ struct ResidualOut {
 };
 // The double-float apply takes 27 us on any small mesh (one CTA's chain of instructions), the FP64 one
 // (kapply.cu's one-contraction lines) 14.6 us on 48 x 48 elements, 27 on 120 x 240 (double-float 29), 40 on
-// 180 x 300 (30), 71 on 240 x 480 (39), 250 on 480 x 960 (127): the line lies between the third and the fourth.
-inline bool df_pays(const Layout& L) { return (int64_t)L.NelX * L.NelY >= 32000; }
+// 180 x 300 (30), 71 on 240 x 480 (39), 250 on 480 x 960 (127): the line lies between the second and the third.
+// With more elements of several rigidities than one in 128 the FP64 apply costs up to half as much again (29 to 36 us on
+// 120 x 240 elements, the double-float one 27; 27 to 30 on 110 x 190, 22 on 90 x 160): from 20,000 elements on.
+// Where the FP64 apply takes both contractions of every line (uni64_pays false), on any mesh (39 on 120 x 240).
+inline bool df_pays(const Handle& h) {
+    return (int64_t)h.L.NelX * h.L.NelY >= (h.few_several ? 32000 : 20000) || !h.uni64_pays;
+}
 // y = sign K x (FP64 vectors, mode 0/1) in double-float arithmetic, or in FP64 where that is faster; with R, K_II x of the scaled change
 // straight into the residual (y and sign unused).  False when unavailable.
 bool apply_K_df(Handle& h, const double* x, double* y, double sign, int mode, cudaStream_t s,

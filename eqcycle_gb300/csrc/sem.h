@@ -41,8 +41,8 @@ struct SemOp {
     unsigned* count = nullptr;
 };
 
-// True when this handle's FP32 quasi-static operator runs here (apply_variant 0, elements mostly of one
-// rigidity).
+// True when this handle's FP32 quasi-static operator runs here (apply_variant 0, at most one element in eight of
+// several rigidities: classify_elements).
 bool sem_usable(const Handle& h);
 void sem_launch(Handle& h, SemLoad load, SemEpi epi, SemPrev prev, const SemOp& o);
 double set_H_sem(const double* H, cudaStream_t s);   // returns Handle::sem_scale

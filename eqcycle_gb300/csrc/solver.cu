@@ -411,6 +411,11 @@ static void setup_residual_full(Handle& h, bool mixed) {
     else dot64(h, h.r64.p + ld, h.r64.p + ld, n, &S->rr);
 }
 
+// The intermediate reliable updates apply K to x's change (update_mixed).
+static int incr_updates(const Handle& h, bool mixed) {
+    return (mixed && h.df_ok && df_pays(h) && h.dx64.p && h.kdx64.p) ? 1 : 0;
+}
+
 // Carried residual: r64 -= K_IF (F - Flast) on rows 1..4 (tmp64b row 0 holds F - Flast), then
 // r32 = sigma r64 for this solve's sigma; with a guess increment g in d: r32 -= sigma K_II g
 // (the first reliable update recomputes r64).
@@ -430,7 +435,7 @@ static void setup_residual_carry(Handle& h, const float* guess) {
                                                               h.r64.p + ld, n);
         EQC_CHECK_LAUNCH();
         count_launch(3);
-        if (h.dx64.p) {   // r64 is the residual without the kept increment
+        if (incr_updates(h, true)) {   // r64 is the residual without the kept increment
             k_dx_init<<<vgrid<double>(n), VEC_THREADS, 0, h.stream>>>(h.dx64.p + ld, guess + ld, h.cg.p, n);
             EQC_CHECK_LAUNCH();
             count_launch();
@@ -534,9 +539,6 @@ static void iter_mixed_a(Handle& h, double delta, cudaGraphConditionalHandle hi,
 // convergence recomputes b - K_II x with the FP64 apply: the full K x's double-float error would
 // floor the residual near 1e-5 of |b| late in a cycle (|K||x| / |b| large; measured).  Both
 // forms run as gated launches (ApplyArgs::gate on S->upd_incr).
-static int incr_updates(const Handle& h, bool mixed) {
-    return (mixed && h.df_ok && h.dx64.p && h.kdx64.p) ? 1 : 0;
-}
 static void update_mixed(Handle& h, cudaGraphConditionalHandle hw, int use_cond) {
     const Layout& L = h.L;
     const int64_t ld = L.ld, n = L.size() - ld;
