@@ -149,23 +149,26 @@ __constant__ int cEO_ok;   // H is centro-antisymmetric (else the full contracti
 
 // An element of one rigidity mu has W(p, j) = mu w_p w_j (w the GLL weights), so the two contractions
 // of a line and the multiplication between them are one 5 x 5 matrix: the line's share of K x is
-// c mu w_j S v with S = D^T diag(w) D.  S is symmetric and centrosymmetric and its rows sum to zero:
-// with o_m = v_m - v_(4-m) and e_m = v_m + v_(4-m) - 2 v_2,
+// c mu w_j S v with S = D^T diag(w) D.  S is symmetric and centrosymmetric: with o_m = v_m - v_(4-m) and
+// e_m = v_m + v_(4-m) - 2 v_2 + g_m v_2,
 //   s_p, s_(4-p) = Q +- P,  Q = sum_m b_pm e_m,  P = sum_m a_pm o_m  (p = 0, 1),  s_2 = sum_m d_m e_m,
-// 20 operations where the two even-odd contractions and W take 45.  Every entry is taken as a
+// 22 operations where the two even-odd contractions and W take 45.  Every entry is taken as a
 // difference first (e_m = o_m + 2 (v_(4-m) - v_2)): on a smooth field the differences are exact or
-// nearly so, and the rounding left is of the size of the field's variation over the element (2e-16
-// of the result where the two contractions leave 3e-15).  Constants give exactly zero; through a
-// rounded D, whose rows sum to 2e-15 instead, they give 1e-15 of the entries of K.
+// nearly so, and the rounding left is of the size of the field's variation over the element.
+// g (set_H) gives constants the row sums of S, 1e-15 of its entries, that the rounding of the caller's D leaves:
+// without it constants would give zero, but the operator would not be the one that the caller's H defines (distance
+// from H's operator in extended precision, of the largest |K x|, smooth x on 61 x 95 elements: 6e-15 with both
+// contractions, 1e-14 without g; random x 3e-16 any way).
 struct UniCoef {
-    double a[2][2], b[2][2], d[2];
+    double a[2][2], b[2][2], d[2], g[2];
     double w[5];
 };
 __constant__ UniCoef cUni;
 
 __device__ __forceinline__ void uni_line(const double (&v)[5], double (&s)[5]) {
     const double o0 = v[0] - v[4], o1 = v[1] - v[3];
-    const double e0 = fma(2.0, v[4] - v[2], o0), e1 = fma(2.0, v[3] - v[2], o1);
+    const double e0 = fma(cUni.g[0], v[2], fma(2.0, v[4] - v[2], o0));
+    const double e1 = fma(cUni.g[1], v[2], fma(2.0, v[3] - v[2], o1));
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
         const double P = fma(cUni.a[p][1], o1, cUni.a[p][0] * o0);
@@ -1472,6 +1475,12 @@ bool set_H(const double* H, cudaStream_t s) {
                 u.b[p][m] = (double)(0.5L * (S(p, m) + S(p, 4 - m)));
             }
             u.d[p] = (double)S(2, p);
+        }
+        {   // b g = the row sums of rows 0 and 1; row 2's follows, since they add up to (D 1)^T w (D 1), 1e-30
+            const double b00 = u.b[0][0], b01 = u.b[0][1], b10 = u.b[1][0], b11 = u.b[1][1], det = b00 * b11 - b01 * b10;
+            auto rho = [&](int p) { return (double)(S(p, 0) + S(p, 1) + S(p, 2) + S(p, 3) + S(p, 4)); };
+            u.g[0] = uni ? (b11 * rho(0) - b01 * rho(1)) / det : 0.0;
+            u.g[1] = uni ? (b00 * rho(1) - b10 * rho(0)) / det : 0.0;
         }
         for (int p = 0; p < 5; ++p) u.w[p] = gw[p];
         EQC_CUDA(cudaMemcpyToSymbolAsync(cUni, &u, sizeof(u), 0, cudaMemcpyHostToDevice, s));
