@@ -71,21 +71,6 @@ __device__ __forceinline__ T cheb_x_pt(T x, T xp, T b, T t, T dinv, T c1, T c2) 
     return fma_rn<T>(c2, g, fma_rn<T>(c1, sub_rn<T>(x, xp), x));
 }
 
-// FP32 -> FP64, exact, by integer operations on the bit patterns (GB300 converts to FP64 on its
-// FP64 unit, a small fraction of its integer and FP32 rate).  Zeros, subnormals, infinities
-// and NaNs included.
-__device__ __forceinline__ double f32_to_f64(float f) {
-    const uint32_t b = __float_as_uint(f);
-    const uint64_t sign = (uint64_t)(b >> 31) << 63;
-    const uint32_t e = (b >> 23) & 0xffu, m = b & 0x7fffffu;
-    if (e == 0xffu) return __longlong_as_double((long long)(sign | (0x7ffull << 52) | ((uint64_t)m << 29)));
-    if (e != 0) return __longlong_as_double((long long)(sign | ((uint64_t)(e + 896u) << 52) | ((uint64_t)m << 29)));
-    if (m == 0) return __longlong_as_double((long long)sign);
-    const int p = 31 - __clz((int)m);                 // leading one of a subnormal: m * 2^-149
-    const uint64_t frac = ((uint64_t)m - (1ull << p)) << (52 - p);
-    return __longlong_as_double((long long)(sign | ((uint64_t)(p + 874) << 52) | frac));
-}
-
 // The FP32 increment dt vh of a dynamic step from the half-step velocity vh: vh rounded to FP32
 // (integer operations), times dt given as hi + lo in FP32, so the product is rounded once
 // without the systematic error of a rounded dt, which K d would accumulate step after step.

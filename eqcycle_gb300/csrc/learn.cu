@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(256) k_mse(const float* __restrict__ out, cons
         acc.add(e, e);
     }
     if (threadIdx.x < GN_LDOUT - nout) g[(int64_t)b * GN_LDOUT + nout + threadIdx.x] = 0.f;   // the row's padding
-    block_sum(acc);
-    if (threadIdx.x == 0) loss[b] = acc.value();
+    const double s = cta_sum(acc.value());
+    if (threadIdx.x == 0) loss[b] = s;
 }
 
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,

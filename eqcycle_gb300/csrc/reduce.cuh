@@ -4,53 +4,45 @@
 
 namespace eqc {
 
+constexpr int SUM_THREADS = 256;   // the largest CTA that sums
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
 }
 
-// Sum over the CTA; result valid in thread 0.
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) sh[w] = v;
+// Sum of one number per thread over the CTA (whole warps, at most SUM_THREADS threads); valid in thread 0.
+// An FP64 instruction of a warp holds its SM's FP64 pipe for 16 clocks, so one warp adds what every thread
+// leaves in shared memory, 12 instructions to a CTA where sums of each warp first take 45.
+__device__ __forceinline__ double cta_sum(double v) {
+    __shared__ double sh[SUM_THREADS];
+    sh[threadIdx.x] = v;
     __syncthreads();
-    const int nw = (blockDim.x + 31) >> 5;
-    v = (threadIdx.x < nw) ? sh[threadIdx.x] : 0.0;
-    if (w == 0) v = warp_sum(v);
+    if (threadIdx.x < 32) {
+        double t[SUM_THREADS / 32];
+#pragma unroll
+        for (int q = 0; q < SUM_THREADS / 32; ++q) t[q] = 32 * q < blockDim.x ? sh[32 * q + threadIdx.x] : 0.0;
+#pragma unroll
+        for (int h = SUM_THREADS / 64; h > 0; h >>= 1)
+#pragma unroll
+            for (int q = 0; q < h; ++q) t[q] += t[q + h];
+        v = warp_sum(t[0]);
+    }
     __syncthreads();
     return v;
 }
 
-// Sum of a dot-product accumulator (DotAcc) over the CTA (up to 1,024 threads); valid in warp 0's lane 0.
-template <class Acc>
-__device__ __forceinline__ void block_sum(Acc& acc) {
-    __shared__ typename Acc::Part sh[32];
-    acc.warp_sum();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    if (lane == 0) sh[w] = acc.part();
-    __syncthreads();
-    if (w == 0) {
-        acc = Acc();
-        if (lane < nw) acc.merge(sh[lane]);
-        acc.warp_sum(nw);
-    }
-    __syncthreads();
-}
-
-// Finishes a reduction over the grid: every CTA stores its partial, the last one to do so (an atomic
+// Finishes a reduction (DotAcc) over the grid: every CTA stores its partial, the last one to do so (an atomic
 // ticket) sums them, one per thread where there are threads enough, in an order that depends on the
-// grid only, and calls fin(total) in thread 0.  part: 16 bytes per CTA.
+// grid only, and calls fin(total) in thread 0.  part: one entry per CTA.
 template <class Acc, class Fin>
-__device__ __forceinline__ void grid_sum(Acc acc, double* part, unsigned* count, Fin fin) {
+__device__ __forceinline__ void grid_sum(const Acc& acc, double* part, unsigned* count, Fin fin) {
     __shared__ bool last;
-    using Part = typename Acc::Part;
-    Part* p = reinterpret_cast<Part*>(part);
     const unsigned nblk = gridDim.x * gridDim.y;
-    block_sum(acc);
+    const double s = cta_sum(acc.value());
     if (threadIdx.x == 0) {
-        p[blockIdx.y * gridDim.x + blockIdx.x] = acc.part();
+        part[blockIdx.y * gridDim.x + blockIdx.x] = s;
         __threadfence();
         const unsigned prev = atomicAdd(count, 1u);
         last = (prev == nblk - 1);
@@ -58,11 +50,11 @@ __device__ __forceinline__ void grid_sum(Acc acc, double* part, unsigned* count,
     __syncthreads();
     if (!last) return;
     __threadfence();
-    acc = Acc();
-    for (unsigned k = threadIdx.x; k < nblk; k += blockDim.x) acc.merge(__ldcg(p + k));
-    block_sum(acc);
+    double t = 0.0;
+    for (unsigned k = threadIdx.x; k < nblk; k += blockDim.x) t += __ldcg(part + k);
+    t = cta_sum(t);
     if (threadIdx.x == 0) {
-        fin(acc.value());
+        fin(t);
         *count = 0u;
     }
 }

@@ -9,7 +9,7 @@
 // Plain FP64 path: FP64 apply, FP64 preconditioner, FP64 vectors.
 // Mixed path: CG with reliable updates (van der Vorst & Ye residual replacement): the
 // Krylov recurrences run on FP32 vectors with an FP32 apply and FP32 preconditioner
-// (dot products accumulated in pairs of FP32 numbers); the iterate is accumulated in FP64 and, whenever
+// (dot products accumulated in FP64); the iterate is accumulated in FP64 and, whenever
 // the recurrence residual has dropped by a factor `delta` since the last update, the
 // true residual b - K_II x is recomputed with the FP64 apply and replaces the FP32 one.
 // Convergence is always certified on an FP64 true residual.

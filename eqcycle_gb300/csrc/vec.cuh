@@ -5,7 +5,6 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
-#include "df.cuh"
 
 namespace eqc {
 
@@ -38,55 +37,34 @@ __device__ __forceinline__ void st4(double* p, const double (&a)[4]) {
     reinterpret_cast<double2*>(p)[1] = make_double2(a[2], a[3]);
 }
 
+// FP32 -> FP64, exact, by integer operations on the bit patterns (GB300 converts to FP64 on its
+// FP64 unit, a small fraction of its integer and FP32 rate).  Zeros, subnormals, infinities
+// and NaNs included.
+__device__ __forceinline__ double f32_to_f64(float f) {
+    const uint32_t b = __float_as_uint(f);
+    const uint64_t sign = (uint64_t)(b >> 31) << 63;
+    const uint32_t e = (b >> 23) & 0xffu, m = b & 0x7fffffu;
+    if (e == 0xffu) return __longlong_as_double((long long)(sign | (0x7ffull << 52) | ((uint64_t)m << 29)));
+    if (e != 0) return __longlong_as_double((long long)(sign | ((uint64_t)(e + 896u) << 52) | ((uint64_t)m << 29)));
+    if (m == 0) return __longlong_as_double((long long)sign);
+    const int p = 31 - __clz((int)m);                 // leading one of a subnormal: m * 2^-149
+    const uint64_t frac = ((uint64_t)m - (1ull << p)) << (52 - p);
+    return __longlong_as_double((long long)(sign | ((uint64_t)(p + 874) << 52) | frac));
+}
+
 // Dot-product accumulator.  FP64 vectors accumulate in FP64.  FP32 vectors accumulate the
 // exact products (a*b = p + e, e by FMA) in an unevaluated FP32 pair (hi + lo, Knuth's
-// TwoSum), about 44 significant bits, and are summed as pairs over threads and CTAs (reduce.cuh):
-// FP64-class dot products of FP32 vectors without FP64 arithmetic before the total (an FP64
-// instruction holds an SM's FP64 pipe for 16 clocks per warp and its result comes late: with FP64 sums
-// of the warps, the CTA and the CTAs' partials a reduction's tail took 5 us of every launch).
-// warp_sum: into lane 0, of the first `lanes` lanes (the others hold zero).
+// TwoSum), about 44 significant bits, then hand a double to the cross-thread reduction (reduce.cuh):
+// FP64-class dot products of FP32 vectors without FP64 arithmetic per element (GB300's FP64
+// and FP32<->FP64 conversion rates are a small fraction of its FP32 rate).
 template <class T> struct DotAcc;
 template <> struct DotAcc<double> {
-    using Part = double;   // what crosses warps and CTAs
     double s = 0.0;
     __device__ __forceinline__ void add(double a, double b) { s = fma(a, b, s); }
-    __device__ __forceinline__ Part part() const { return s; }
-    __device__ __forceinline__ void merge(Part p) { s += p; }
     __device__ __forceinline__ double value() const { return s; }
-    __device__ __forceinline__ void warp_sum(int lanes = 32) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            if (o < lanes) s += __shfl_down_sync(0xffffffffu, s, o);
-    }
 };
 template <> struct DotAcc<float> {
-    using Part = float2;
     float hi = 0.f, lo = 0.f;
-    __device__ __forceinline__ Part part() const { return make_float2(hi, lo); }
-    __device__ __forceinline__ void merge(Part p) { add_pair(p.x, p.y); }
-    // (hi, lo) += (h, l): the accurate double-float addition (relative error 3 x 2^-48)
-    __device__ __forceinline__ void add_pair(float h, float l) {
-        float s, e, t, f;
-        two_sum(hi, h, s, e);
-        two_sum(lo, l, t, f);
-        e = __fadd_rn(e, t);
-        fast_two_sum(s, e, hi, e);
-        e = __fadd_rn(e, f);
-        fast_two_sum(hi, e, s, lo);
-        hi = s;
-    }
-    __device__ __forceinline__ void warp_sum(int lanes = 32) {
-        float s, e;
-        two_sum(hi, lo, s, e);   // a proper pair first
-        hi = s;
-        lo = e;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            if (o >= lanes) continue;
-            const float h = __shfl_down_sync(0xffffffffu, hi, o), l = __shfl_down_sync(0xffffffffu, lo, o);
-            add_pair(h, l);
-        }
-    }
     __device__ __forceinline__ void add(float a, float b) {
         const float p = __fmul_rn(a, b);
         const float e = __fmaf_rn(a, b, -p);
@@ -96,7 +74,7 @@ template <> struct DotAcc<float> {
         hi = s;
         lo = __fadd_rn(lo, __fadd_rn(err, e));
     }
-    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+    __device__ __forceinline__ double value() const { return f32_to_f64(hi) + f32_to_f64(lo); }
 };
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
