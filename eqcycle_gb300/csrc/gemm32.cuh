@@ -17,7 +17,7 @@
 #include <cstdint>
 #include <type_traits>
 #include "common.h"
-#include "df.cuh"
+#include "vec.cuh"
 
 namespace eqc {
 
@@ -64,20 +64,15 @@ struct OpRows {
     }
 };
 
-// Sums over k of A's rows beside the product (a bias's gradient from a weight's): error-free sums in FP32, in
+// Sums over k of A's rows beside the product (a bias's gradient from a weight's): in FP64, in
 // the threads that load A; done calls f(m, sum).  For the two ways in which a weight gradient's A is loaded.
 template <bool KF>
 struct RowSum {
     static constexpr int R = KF ? 8 : 4;
-    float hi[R] = {}, lo[R] = {};
+    double s[R] = {};
     __device__ __forceinline__ void add(const float (&v)[8]) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            float t, e;
-            two_sum(hi[i % R], v[i], t, e);
-            hi[i % R] = t;
-            lo[i % R] += e;
-        }
+        for (int i = 0; i < 8; ++i) s[i % R] += f32_to_f64(v[i]);
     }
     template <class F>
     __device__ __forceinline__ void done(int m0, int M, F f) const {
@@ -85,7 +80,7 @@ struct RowSum {
         if constexpr (KF) {   // one by one: rows (tid >> 4) + 8 i, of 16 threads
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                double d = (double)hi[i] + (double)lo[i];
+                double d = s[i];
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o, 16);
                 const int m = m0 + (tid >> 4) + 8 * i;
@@ -94,7 +89,7 @@ struct RowSum {
         } else {              // four a load: rows 4 (tid & 15) + i, of 8 threads
             __shared__ double part[8][GT_N];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) part[tid >> 4][4 * (tid & 15) + i] = (double)hi[i] + (double)lo[i];
+            for (int i = 0; i < 4; ++i) part[tid >> 4][4 * (tid & 15) + i] = s[i];
             __syncthreads();
             if (tid < GT_N && m0 + tid < M) {
                 double d = 0.0;

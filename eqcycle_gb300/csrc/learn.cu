@@ -88,7 +88,7 @@ struct EpWeight {
     __device__ int64_t npos(int n) const { return (PART ? (int64_t)blockIdx.z * M * N : 0) + n; }
     __device__ void put(int m, int, int64_t np, float v) const { C[np + (int64_t)m * N] = v; }
 };
-// gW and gb from the splits' shares, to FP64's accuracy: 32 results a CTA, every eighth split a warp (481 splits of
+// gW and gb from the splits' shares, in FP64: 32 results a CTA, every eighth split a warp (481 splits of
 // conv1's 640 weights: 73 us with a thread to each result).
 __global__ void __launch_bounds__(256) k_weight_sum(const float* __restrict__ part, const double* __restrict__ db_part,
                                                     int splits, int M, int N, float* __restrict__ gW, float* __restrict__ gb) {
@@ -97,16 +97,9 @@ __global__ void __launch_bounds__(256) k_weight_sum(const float* __restrict__ pa
     const int n = M * N, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
     double s = 0.0;
-    if (i < n) {   // error-free in FP32: FP64 adds and conversions would take the longer part of the launch
-        float hi = 0.f, lo = 0.f;
+    if (i < n) {
 #pragma unroll 8
-        for (int z = w; z < splits; z += 8) {
-            float t, e;
-            two_sum(hi, part[(int64_t)z * n + i], t, e);
-            hi = t;
-            lo += e;
-        }
-        s = (double)hi + (double)lo;
+        for (int z = w; z < splits; z += 8) s += f32_to_f64(part[(int64_t)z * n + i]);
     } else if (i < n + M) {
         for (int z = w; z < splits; z += 8) s += db_part[(int64_t)z * M + i - n];
     }
@@ -298,15 +291,16 @@ __global__ void __launch_bounds__(256) k_mse(const float* __restrict__ out, cons
     EQC_GRID_WAIT();
     const int b = blockIdx.x;
     const float sc = 2.f / ((float)B * (float)nout);
-    DotAcc<float> acc;   // an error-free product and sum to each entry, in FP32
+    double s = 0.0;
 #pragma unroll 4
     for (int j = threadIdx.x; j < nout; j += blockDim.x) {
         const float e = out[(int64_t)b * nout + j] - tgt[(int64_t)b * nout + j];
         g[(int64_t)b * GN_LDOUT + j] = sc * e;
-        acc.add(e, e);
+        const double d = f32_to_f64(e);
+        s = fma(d, d, s);
     }
     if (threadIdx.x < GN_LDOUT - nout) g[(int64_t)b * GN_LDOUT + nout + threadIdx.x] = 0.f;   // the row's padding
-    const double s = cta_sum(acc.value());
+    s = cta_sum(s);
     if (threadIdx.x == 0) loss[b] = s;
 }
 
