@@ -382,6 +382,8 @@ void gn_init(Handle& h, uint64_t seed) {
     g.m1.alloc(o);
     g.m2.alloc(o);
     g.wbf.alloc(o);
+    g.w_part.alloc((size_t)GN_WSPLIT * GN_C * GT_N);
+    g.b_part.alloc((size_t)GN_WSPLIT * GN_C);
     g.adam_t = 0;
     g.trained = false;
     gn_refresh_bf16(g, s);
@@ -423,10 +425,6 @@ void gn_forward(GuessNet& g, const float* x0, int B, cudaStream_t s) {
 
 // Gradient of the mean squared error of g.out (after gn_forward on x0) against tgt.
 void gn_backward(GuessNet& g, const float* x0, const float* tgt, int B, cudaStream_t s) {
-    if (!g.w_part.p) {
-        g.w_part.alloc((size_t)GN_WSPLIT * GN_C * GT_N);
-        g.b_part.alloc((size_t)GN_WSPLIT * GN_C);
-    }
     k_mse<<<B, 256, 0, s>>>(g.out.p, tgt, g.nout, B, g.g_out.p, g.loss.p);
     count_launch();
     // fc2: weight and bias, then g_z of fc1

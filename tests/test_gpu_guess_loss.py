@@ -24,3 +24,19 @@ def test_loss_over_the_range_of_targets(eqclib, batch, scale):
         mse = s.guess_eval(x0, tgt)
     want = float(np.mean(tgt.astype(np.longdouble) ** 2))
     assert abs(loss - want) <= 1e-12 * want and abs(mse - want) <= 1e-12 * want
+
+
+def test_gradient_allocates_nothing_of_its_own(eqclib):
+    """After an evaluation of as many pairs the buffers of a batch are there: the first gradient takes no more
+    device memory."""
+    torch = pytest.importorskip("torch")
+    P = set_parameters(preset("homog48").replace(NelX=13, NelY=4, LX=6.5e3, LY=2e3, creep_depth=6.5e3))
+    rng = np.random.default_rng(1)
+    with Solver(P, precond=EQC_PC_JACOBI) as s:
+        nin, nout, _ = s.guess_shape()
+        x0 = rng.uniform(-1, 1, (65, nin)).astype(np.float32)
+        tgt = rng.uniform(-1, 1, (65, nout)).astype(np.float32)
+        s.guess_eval(x0, tgt)
+        free = torch.cuda.mem_get_info()[0]
+        s.guess_grad(x0, tgt)
+        assert torch.cuda.mem_get_info()[0] == free
