@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(GT_THREADS) k_tile(OA A, OB B, EP E, int M, in
             fa[i] = ina >> i & 1 ? A.value(va, i) : 0.f;
             fb[i] = inb >> i & 1 ? B.value(vb, i) : 0.f;
         }
-        E.sum(fa, n0);
+        E.sum(fa, t);
         store(A, fa, [&](int k, int m, float v) { as[k * GT_P + m] = v; });
         store(B, fb, [&](int k, int n, float v) { bs[k * GT_P + n] = v; });
         __syncthreads();   // the other buffer's readers are past it too: they stored to this one after reading

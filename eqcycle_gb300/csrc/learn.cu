@@ -24,7 +24,7 @@ __device__ __forceinline__ float gelu_grad(float x) {
 // ---- layers as tiled products (gemm32.cuh) ------------------------------------------------
 // What becomes of C(m, n).  sum, sum_done: the row sums of A, where the layer's bias needs them.
 struct EpNoSum {
-    __device__ void sum(const float (&)[8], int) {}
+    __device__ void sum(const float (&)[8], int) {}   // of slice t
     __device__ void sum_done(int, int, int) {}
 };
 struct EpLinear : EpNoSum {   // C = v + bias[n], and its GELU where the next layer takes that
@@ -67,41 +67,53 @@ struct EpConvGrad : EpNoSum {   // n = (b, u) for the positions 2 u + par: g = v
         g[i] = v * gelu_grad(z[i]);
     }
 };
-// Weight and bias gradients: whole sums (a fully connected layer's K is the batch) or a split's share.
+// Weight and bias gradients: whole sums (a fully connected layer's K is the batch) or a split's share.  The row
+// sums are the first column tile's work, or each column tile's on its slices: every CTA of a split is resident
+// at once, so that the longest sets the time (the four layers of 256 pairs: 241 us with all slices summed by one
+// tile, 220 now).
 template <bool KF, bool PART>
 struct EpWeight {
     float* C;
     float* db;         // !PART
-    double* db_part;   // PART: [split][M]
+    double* db_part;   // PART: [split][column tile][M]
     int M, N;
     RowSum<KF> rs;
-    __device__ void sum(const float (&v)[8], int n0) {
-        if (n0 == 0) rs.add(v);
+    __device__ void sum(const float (&v)[8], int t) {
+        if ((PART ? t % gridDim.x : 0) == blockIdx.x) rs.add(v);
     }
     __device__ void sum_done(int m0, int n0, int) {
-        if (n0 != 0) return;
+        if (!PART && n0 != 0) return;
         rs.done(m0, M, [&](int m, double d) {
-            if (PART) db_part[(int64_t)blockIdx.z * M + m] = d;
+            if (PART) db_part[((int64_t)blockIdx.z * gridDim.x + blockIdx.x) * M + m] = d;
             else db[m] = (float)d;
         });
     }
     __device__ int64_t npos(int n) const { return (PART ? (int64_t)blockIdx.z * M * N : 0) + n; }
     __device__ void put(int m, int, int64_t np, float v) const { C[np + (int64_t)m * N] = v; }
 };
-// gW and gb from the splits' shares, in FP64: 32 results a CTA, every eighth split a warp (481 splits of
+// gW and gb from the splits' shares: 32 results a CTA, every eighth split a warp (481 splits of
 // conv1's 640 weights: 73 us with a thread to each result).
 __global__ void __launch_bounds__(256) k_weight_sum(const float* __restrict__ part, const double* __restrict__ db_part,
-                                                    int splits, int M, int N, float* __restrict__ gW, float* __restrict__ gb) {
+                                                    int splits, int tiles, int M, int N, float* __restrict__ gW,
+                                                    float* __restrict__ gb) {
     EQC_GRID_WAIT();
     __shared__ double sh[8][32];
     const int n = M * N, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
     double s = 0.0;
-    if (i < n) {
+    if (i < n) {   // a thread's shares as an error-free pair in FP32: FP64 sums of them took 64 us for 38, with the same bits
+        float hi = 0.f, lo = 0.f;
 #pragma unroll 8
-        for (int z = w; z < splits; z += 8) s += f32_to_f64(part[(int64_t)z * n + i]);
+        for (int z = w; z < splits; z += 8) {
+            float t, e;
+            two_sum(hi, part[(int64_t)z * n + i], t, e);
+            hi = t;
+            lo += e;
+        }
+        s = (double)hi + (double)lo;
     } else if (i < n + M) {
-        for (int z = w; z < splits; z += 8) s += db_part[(int64_t)z * M + i - n];
+#pragma unroll 8
+        for (int z = w; z < splits * tiles; z += 8) s += db_part[(int64_t)z * M + i - n];
     }
     sh[w][lane] = s;
     __syncthreads();
@@ -448,7 +460,7 @@ void gn_backward(GuessNet& g, const float* x0, const float* tgt, int B, cudaStre
         const EpWeight<true, true> ep{g.w_part.p, nullptr, g.b_part.p, GN_C, N, {}};
         k_tile<OpConvGz, OpConvIn<true>, EpWeight<true, true>, 1><<<grid, GT_THREADS, 0, s>>>(
             OpConvGz{{}, g.g_a[l].p, T}, OpConvIn<true>{{}, in, cin, g.T[l], T}, ep, GN_C, N, K, chunk);
-        k_weight_sum<<<(GN_C * N + GN_C + 31) / 32, 256, 0, s>>>(g.w_part.p, g.b_part.p, grid.z, GN_C, N, g.grad.p + g.off_cw[l],
+        k_weight_sum<<<(GN_C * N + GN_C + 31) / 32, 256, 0, s>>>(g.w_part.p, g.b_part.p, grid.z, tiles, GN_C, N, g.grad.p + g.off_cw[l],
                                                            g.grad.p + g.off_cb[l]);
         EQC_CHECK_LAUNCH();
         count_launch(2);
