@@ -72,3 +72,49 @@ def test_residual_of_reliable_updates(eqclib, monkeypatch, nelx, nely, material)
         assert abs(np.linalg.norm(r) / np.linalg.norm(b) - rr) <= 1e-11
         its.append(it)
     assert abs(its[0] - its[1]) <= 1
+
+
+@pytest.mark.parametrize("nelx,nely,material", [(155, 216, "one"), (181, 179, "trapezoid"), (1070, 31, "rectangle"),
+                                                (37, 23, "per-node all")])
+def test_double_float_apply_smooth(eqclib, nelx, nely, material):
+    """A smooth field (K x small against |K| |x|, the cancellation that a residual has), on odd meshes that the
+    double-float kernel serves: 1e-12 of the random case's scale, as the 240 x 480 mesh of test_apply_variants.py."""
+    torch = pytest.importorskip("torch")
+    P = _params(nelx, nely, material.replace(" all", ""))
+    if material.endswith("all"):
+        P.mesh.W[:] *= np.random.default_rng(5).uniform(0.5, 2.0, P.mesh.W.shape)
+    with Solver(P, precond=EQC_PC_JACOBI) as s:
+        nx, ny, ld = s.layout()
+        x = torch.zeros(ny, ld, dtype=torch.float64)
+        x[:, :nx] = torch.as_tensor(np.random.default_rng(3).uniform(-0.5, 0.5, (ny, nx)))
+        scale = np.max(np.abs(_apply(s, torch, x.cuda(), 0)))
+        ix = torch.arange(nx, dtype=torch.float64)[None, :]
+        iy = torch.arange(ny, dtype=torch.float64)[:, None]
+        x[:, :nx] = 0.3 + 1e-3 * ix + 2e-3 * iy + 1e-4 * torch.sin(0.05 * ix) * torch.cos(0.03 * iy)
+        z64, zdf = _apply(s, torch, x.cuda(), 0), _apply(s, torch, x.cuda(), 2)
+    assert not np.array_equal(z64, zdf)          # not the FP64 apply
+    assert np.max(np.abs(zdf - z64)) <= 1e-12 * scale * float(x.abs().max()) / 0.5
+
+
+@pytest.mark.parametrize("nelx,nely,material", [(155, 216, "trapezoid"), (33, 29, "per-node all")])
+def test_intermediate_updates_through_steps(eqclib, monkeypatch, nelx, nely, material):
+    """Quasi-static steps with the intermediate updates in double-float arithmetic and with each in FP64
+    (EQC_NO_DF_UPDATE), on meshes where the two launch different kernels: iteration counts within one per solve,
+    displacement and state to the solver tolerance's scale (the bounds of test_apply_variants.py)."""
+    P = _params(nelx, nely, material.replace(" all", ""))
+    if material.endswith("all"):
+        P.mesh.W[:] *= np.random.default_rng(5).uniform(0.8, 1.25, P.mesh.W.shape)
+    out = []
+    for env in (None, "EQC_NO_DF_UPDATE"):
+        if env:
+            monkeypatch.setenv(env, "1")
+        with Solver(P, precision=EQC_MIXED, precond=EQC_PC_AMG, cg_tol=1e-8) as s:
+            s.init(P.cfg.V_init)
+            st = s.run(12)
+            assert st["qs_steps"] == 12
+            out.append((st["cg_iters"], st["qs_solves"], {k: s.state(k) for k in ("d", "psi", "tau")}))
+    (it_df, solves, a), (it_64, _, b) = out
+    assert abs(it_df - it_64) <= solves
+    assert not np.array_equal(a["d"], b["d"])    # other roundings: not the same kernels
+    for k in a:
+        assert np.max(np.abs(a[k] - b[k])) <= 1e-6 * np.max(np.abs(b[k])), k
