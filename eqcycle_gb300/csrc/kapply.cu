@@ -12,13 +12,15 @@
 //   k_apply_rows   FP32, one lane per element, one warp per element row, ROWS rows per CTA
 //                  plus a halo warp (variants 0, 4-7; the FP32 default);
 //   k_apply_walk   the same arithmetic fed by TMA, one wave of CTAs each walking up a strip
-//                  (variant 8; the autotuner's usual choice);
+//                  (variant 8);
 //   k_apply_uni64  FP64: persistent tiles with a TMA pipeline, node-line form, one contraction per
-//                  line where the elements have one rigidity (the FP64 default);
-//   k_apply_pipe   the same pipeline with both contractions of every line (variant 3, and the K d
-//                  refresh of the mixed method's dynamic steps);
+//                  line where the elements have one rigidity (the FP64 default for models of mostly
+//                  such elements, classify_elements);
+//   k_apply_pipe   the same pipeline with both contractions of every line (variant 3, the FP64 default for
+//                  the other models, and the K d refresh of the mixed method's dynamic steps);
 //                  k_apply_tma / k_apply_lines: one tile per CTA (1, 2);
 //   k_strip        the strip modes 2 and 3 (first element row only).
+// Quasi-static solves with variant 0 take their FP32 operator from sem.cu instead.
 // The FP32 element kernels take an epilogue (epi.cuh) that finishes the V-cycle's residual or
 // Chebyshev step at each owned node.
 #include "model.h"
@@ -1213,8 +1215,6 @@ static bool encode_w_walk(CUtensorMap* m, const float* base, int NelX, int NelY)
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-
-constexpr int TEX = 8, TEY = 8;
 
 constexpr int LTEX = 8, LTEY = 7, LNT = 256;
 
