@@ -620,12 +620,12 @@ static_assert(UniTile::OY * UniTile::EX == UNT && UniTile::EY * UniTile::OX <= U
 // Bound: GB300 issues two FP64 operations per SM and clock (every FP64 instruction of a warp holds
 // the pipe for 16 clocks, whatever its active lanes), so the lines, their scaling and the sums at
 // shared nodes are arranged in whole warps, the rigidities' signs are tested as integers, and a tile
-// takes about 430 warp instructions of the pipe: 7.7 per element, where both contractions took 15.
+// takes about 460 warp instructions of the pipe: 8.2 per element, where both contractions took 15.
 // Back to back on the damage-zone models, before (both contractions, 8 x 7 tiles) and now: 61 x 95
-// elements 19.4 and 10.4 us, 120 x 240 37.1 and 21.9, 240 x 480 134.2 and 68.6 (122.8 and 60.8 where
-// one x and y stay in L2), 480 x 960 496 and 248: 48 us of the 60.8 are the pipe's.
+// elements 19.2 and 10.8 us, 120 x 240 37.2 and 22.6, 240 x 480 134.3 and 71.5 (122.8 and 62.5 where
+// one x and y stay in L2), 480 x 960 496 and 261: 51 us of the 62.5 are the pipe's.
 // TAIL: NoTail; ResidualOut, the mixed solver's residual r64 = -K_II x with its work (sign -1, zero_row0);
-// DotOut, the CG's x . K x (a launch of its own took 9 us on 120 x 240 elements, the sum here 4).
+// DotOut, the CG's x . K x (a launch of its own took 9 us on 120 x 240 elements, the sum here 1).
 struct NoTail {};
 template <class TAIL>
 __global__ void __launch_bounds__(UNT) k_apply_uni64(const __grid_constant__ CUtensorMap umap,
@@ -1454,7 +1454,7 @@ bool set_H(const double* H, cudaStream_t s) {
         }
         const int ok = asym <= 1e-12 * hmax ? 1 : 0;
         // S = D^T diag(w) D of the one-contraction lines, w the GLL weights of 5 points; its rows
-        // sum to zero when constants have no derivative (sum_k H(k, p) = 0)
+        // sum to zero, but for what rounding leaves, when constants have no derivative (sum_k H(k, p) = 0)
         const double gw[5] = {0.1, 49.0 / 90.0, 32.0 / 45.0, 49.0 / 90.0, 0.1};
         double rows = 0.0;
         for (int p = 0; p < 5; ++p) {

@@ -260,8 +260,8 @@ struct ResidualOut {
     int use_cond = 0, check = 0;
 };
 // The double-float apply takes 27 us on any small mesh (one CTA's chain of instructions), the FP64 one
-// (kapply.cu's one-contraction lines) 14.6 us on 48 x 48 elements, 27 on 120 x 240 (double-float 29), 40 on
-// 180 x 300 (30), 71 on 240 x 480 (39), 250 on 480 x 960 (127): the line lies between the second and the third.
+// (kapply.cu's one-contraction lines) 14.6 us on 48 x 48 elements, 27 on 120 x 240 (double-float 29), 41 on
+// 180 x 300 (30), 76 on 240 x 480 (39), 267 on 480 x 960 (127): the line lies between the second and the third.
 // With more elements of several rigidities than one in 128 the FP64 apply costs up to half as much again (29 to 36 us on
 // 120 x 240 elements, the double-float one 27; 27 to 30 on 110 x 190, 22 on 90 x 160): from 20,000 elements on.
 // Where the FP64 apply takes both contractions of every line (uni64_pays false), on any mesh (39 on 120 x 240).

@@ -383,8 +383,8 @@ void sem_launch(Handle& h, SemLoad load, SemEpi epi, SemPrev prev, const SemOp& 
     // 480 x 960 elements 7.13, and 8.19, 7.78 and 7.59 with the rows for 8, 24 and 40)
     const int64_t warps = (int64_t)nsx * (L.NelY + 1), slots = 152 * 16;
     G.rows = (int)((warps + slots - 1) / slots);
-    // a sum's end is per CTA: eight warps to one (ms per step on 240 x 480 elements 2.77 with two, 2.68 with four,
-    // 2.66 with eight; sixteen are slower on small meshes, 1.44 against 1.41 on 48 x 48)
+    // a sum's end is per CTA: eight warps to one (ms per step on 240 x 480 elements 2.70 with four, 2.66 with eight, on
+    // 480 x 960 7.45 and 7.43, the same on 48 x 48)
     const int W = o.dot ? 8 : 1;
     const dim3 grid(nsx, (L.NelY + W * G.rows) / (W * G.rows));
     auto go = [&](auto kernel) { kernel<<<grid, 32 * W, 0, h.stream>>>(G, o); };

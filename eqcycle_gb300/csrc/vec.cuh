@@ -9,11 +9,9 @@
 namespace eqc {
 
 // One wave of CTAs of 256 threads, four per SM of a GB300 for FP32 vectors, three for FP64 ones, fewer where n
-// has fewer 4-wide chunks.  A thread's share of a reduction's end is a hundred instructions, as many as five
-// of its entries take, so fewer threads with more entries pay less for it than full SMs gain in loads in
-// flight: ms per quasi-static step with 1,024 threads (two and one per SM) and now, 48 x 48 elements 1.39
-// and 1.36, 240 x 480 2.71 and 2.67, 480 x 960 7.23 and 7.17; plain FP64 90 x 60 2.94 and 2.80, 120 x 240
-// 5.19 and 5.13.
+// has fewer 4-wide chunks.  More threads have more loads in flight, fewer pay less for the ends of their sums:
+// ms per quasi-static step with two CTAs per SM, with four and three, and with six and four, 480 x 960 elements 7.59,
+// 7.43 and 7.42, 240 x 480 2.68, 2.66 and 2.66, 120 x 240 1.524, 1.517 and 1.517, plain FP64 the same.
 constexpr int VEC_THREADS = 256;
 template <class T> constexpr int VEC_PER_SM = sizeof(T) == 4 ? 4 : 3;
 template <class T> inline int vec_blocks(int64_t n) {

@@ -89,14 +89,17 @@ typedef struct {
     double reliable_delta;  /* mixed precision: a reliable update whenever the recurrence
                                residual fell by this factor (default 1e-3): r -= K dx with
                                a double-float apply, b - K x in FP64 for the update that
-                               certifies convergence and below 32,000 elements         */
+                               certifies convergence and, where its apply is the faster
+                               one (mostly elements of one rigidity), below 32,000
+                               elements                                                */
     int32_t mg_degree;      /* Chebyshev smoothing steps on the spectral-element level, pre and
                                post (default 4)                                        */
     int32_t mg_coarse_max;  /* largest coarsest level, solved densely (default 2048 unknowns) */
     int32_t apply_variant;  /* stiffness apply kernel: 0 default (FP32: one element per lane,
                                6 element rows per CTA, in quasi-static solves one contraction
                                per line; FP64: persistent TMA pipeline, one contraction per
-                               line), 1 one tile per CTA by TMA, 2 plain tile loads, 3 persistent
+                               line; for models of mostly several rigidities per
+                               element both contractions, as variant 3), 1 one tile per CTA by TMA, 2 plain tile loads, 3 persistent
                                TMA pipeline, FP32 only: 4 / 5 / 6 / 7 one element per lane
                                with 4 / 8 / 12 / 6 (2 CTAs per SM) element rows per CTA,
                                8 one element per lane fed by TMA, one wave of CTAs each
@@ -318,7 +321,8 @@ eqc_status eqc_layout(eqc_handle* h, int64_t* nx, int64_t* ny, int64_t* ld);
 
 /* y = K x on device buffers in the internal layout, FP64 (dtype 0), FP32 (dtype 1, W held in
  * FP32) or FP64 vectors in double-float arithmetic (dtype 2: the mixed solver's
- * intermediate updates, ~1e-14 relative; in FP64 below 32,000 elements), on the handle's stream.  Asynchronous. */
+ * intermediate updates, ~1e-14 relative; in FP64 where that is faster: meshes below 32,000
+ * elements, mostly of one rigidity each), on the handle's stream.  Asynchronous. */
 eqc_status eqc_apply_K_device(eqc_handle* h, const void* x, void* y, int32_t dtype);
 
 /* Time nrep launches of the stiffness apply (dtype as for eqc_apply_K_device) with CUDA
