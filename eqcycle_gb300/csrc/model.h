@@ -264,9 +264,11 @@ struct ResidualOut {
 // 180 x 300 (30), 76 on 240 x 480 (39), 267 on 480 x 960 (127): the line lies between the second and the third.
 // With more elements of several rigidities than one in 128 the FP64 apply costs up to half as much again (29 to 36 us on
 // 120 x 240 elements, the double-float one 27; 27 to 30 on 110 x 190, 22 on 90 x 160): from 20,000 elements on.
-// Where the FP64 apply takes both contractions of every line (uni64_pays false), on any mesh (39 on 120 x 240).
+// Where the FP64 apply takes both contractions of every line (uni64_pays false, apply_variant 1 to 3), on any mesh
+// (39 to 41 on 120 x 240).
 inline bool df_pays(const Handle& h) {
-    return (int64_t)h.L.NelX * h.L.NelY >= (h.few_several ? 32000 : 20000) || !h.uni64_pays;
+    const bool uni64 = h.uni64_pays && !(h.opt.apply_variant >= 1 && h.opt.apply_variant <= 3);
+    return (int64_t)h.L.NelX * h.L.NelY >= (h.few_several ? 32000 : 20000) || !uni64;
 }
 // y = sign K x (FP64 vectors, mode 0/1) in double-float arithmetic, or in FP64 where that is faster; with R, K_II x of the scaled change
 // straight into the residual (y and sign unused).  False when unavailable.

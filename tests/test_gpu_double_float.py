@@ -96,8 +96,9 @@ def test_double_float_apply_smooth(eqclib, nelx, nely, material):
     assert np.max(np.abs(zdf - z64)) <= 1e-12 * scale * float(x.abs().max()) / 0.5
 
 
-@pytest.mark.parametrize("nelx,nely,material", [(155, 216, "trapezoid"), (33, 29, "per-node all")])
-def test_intermediate_updates_through_steps(eqclib, monkeypatch, nelx, nely, material):
+@pytest.mark.parametrize("nelx,nely,material,variant", [(155, 216, "trapezoid", 0), (33, 29, "per-node all", 0),
+                                                        (33, 29, "trapezoid", 3)])
+def test_intermediate_updates_through_steps(eqclib, monkeypatch, nelx, nely, material, variant):
     """Quasi-static steps with the intermediate updates in double-float arithmetic and with each in FP64
     (EQC_NO_DF_UPDATE), on meshes where the two launch different kernels: iteration counts within one per solve,
     displacement and state to the solver tolerance's scale (the bounds of test_apply_variants.py)."""
@@ -108,7 +109,7 @@ def test_intermediate_updates_through_steps(eqclib, monkeypatch, nelx, nely, mat
     for env in (None, "EQC_NO_DF_UPDATE"):
         if env:
             monkeypatch.setenv(env, "1")
-        with Solver(P, precision=EQC_MIXED, precond=EQC_PC_AMG, cg_tol=1e-8) as s:
+        with Solver(P, precision=EQC_MIXED, precond=EQC_PC_AMG, cg_tol=1e-8, apply_variant=variant) as s:
             s.init(P.cfg.V_init)
             st = s.run(12)
             assert st["qs_steps"] == 12
