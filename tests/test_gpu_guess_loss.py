@@ -27,15 +27,16 @@ def test_loss_over_the_range_of_targets(eqclib, batch, scale):
 
 
 def test_gradient_allocates_nothing_of_its_own(eqclib):
-    """After an evaluation of as many pairs the buffers of a batch are there: the first gradient takes no more
-    device memory."""
+    """After an evaluation of as many pairs the buffers of a batch are there: a handle's first gradient takes no more
+    device memory (its kernels loaded by another handle's)."""
     torch = pytest.importorskip("torch")
     P = set_parameters(preset("homog48").replace(NelX=13, NelY=4, LX=6.5e3, LY=2e3, creep_depth=6.5e3))
     rng = np.random.default_rng(1)
-    with Solver(P, precond=EQC_PC_JACOBI) as s:
+    with Solver(P, precond=EQC_PC_JACOBI) as other, Solver(P, precond=EQC_PC_JACOBI) as s:
         nin, nout, _ = s.guess_shape()
         x0 = rng.uniform(-1, 1, (65, nin)).astype(np.float32)
         tgt = rng.uniform(-1, 1, (65, nout)).astype(np.float32)
+        other.guess_grad(x0, tgt)
         s.guess_eval(x0, tgt)
         free = torch.cuda.mem_get_info()[0]
         s.guess_grad(x0, tgt)
